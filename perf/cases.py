@@ -140,7 +140,7 @@ def _grains(case, seed):
     rot = scenes._random_rotations(rng, clumps)
     for q in range(clumps):
         z, rest = divmod(q, cx * cy)
-        c = np.array([(rest % cx + 0.5) * pitch, (rest // cx + 0.5) * pitch, box[2] + a + 0.5e-3 + z * pitch])
+        c = np.array([(rest % cx + 0.5) * pitch, (rest // cx + 0.5) * pitch, box[2] + a + 1.05 * rp + z * pitch])
         peb = c + tet @ rot[q].T
         mass = 2500.0 * 4.0 / 3.0 * math.pi * rp ** 3 * 3.2
         pr = np.full(4, rp)
