@@ -91,97 +91,222 @@ __device__ __forceinline__ bool nextCandidate(LaneWalk& w, const int* __restrict
     return true;
 }
 
-// Next cell member in lane's share of a box of cells (x0..x1, y0..y1, z0..z1,
-// all inside the domain), cells taken round-robin by the lanes.  Cells whose
-// nearest point is beyond the reach (the box's corners and edges) are
-// skipped: no particle in them can be a candidate.
-struct LaneBox {
-    int u, p, pe, x0, y0, z0, nx, ny, nz, hx, hy, hz, hash;
-    int ix, iy, iz;  // box-local index of cell u, advanced without dividing
-    int4 c;        // the particle's cell
-    float4 h;      // and its offset in it
-    float reach2;  // squared reach, widened past the FP32 rounding of the cell gaps
+// ---- candidate rebuild: rows of cells ----
+// The cells within `reach` of a particle, as rows of cells along x: the cells
+// of one row are consecutive keys, so their members are ONE range of the sorted
+// order.  Rows and row ends beyond the reach (the corners and edges of the
+// box) are left out: no particle in them can be a candidate.
+struct RowBox {
+    int y, z, y0, y1, z1;  // the row taken last, and the box's bounds
+    int4 c;                // the particle's cell
+    float4 h;              // and its offset in it
+    float wide;            // reach, widened past the FP32 rounding of the cell gaps
+    float gz2;             // squared gap to the cells of plane z
+    float ry, rz;          // the particle's y and z from the row's cells' corner
 };
 __device__ __forceinline__ float cellGap(int k, int c, float h, float cs)
 {
     const float lo = (float)(k - c) * cs - h, hi = h - (float)(k - c + 1) * cs;
     return fmaxf(0.f, fmaxf(lo, hi));
 }
-template <int L>
-__device__ __forceinline__ bool nextBoxMember(LaneBox& b, const int* __restrict__ start, const GridDev& g, int& idx)
+// The cells from lo to hi (offsets from the corner of cell c), clamped to n.
+__device__ __forceinline__ void cellRange(int c, float lo, float hi, float cs, int n, int& first, int& last)
 {
-    while (b.p >= b.pe) {
-        b.u += L;
-        if (b.u >= b.nx * b.ny * b.nz) return false;
-        b.ix += L;
-        while (b.ix >= b.nx) {
-            b.ix -= b.nx;
-            ++b.iy;
-        }
-        while (b.iy >= b.ny) {
-            b.iy -= b.ny;
-            ++b.iz;
-        }
-        b.hx = b.x0 + b.ix;
-        b.hy = b.y0 + b.iy;
-        b.hz = b.z0 + b.iz;
-        const float gx = cellGap(b.hx, b.c.x, b.h.x, g.cs.x), gy = cellGap(b.hy, b.c.y, b.h.y, g.cs.y),
-                    gz = cellGap(b.hz, b.c.z, b.h.z, g.cs.z);
-        if (gx * gx + gy * gy + gz * gz > b.reach2) continue;
-        b.hash = (b.hz * g.gy + b.hy) * g.gx + b.hx;
-        b.p = start[b.hash];
-        b.pe = start[b.hash + 1];
-    }
-    idx = b.p++;
-    return true;
+    first = max(0, c + (int)floorf(lo / cs));
+    last = min(n - 1, c + (int)floorf(hi / cs));
 }
-
-// The cells within `reach` of a particle at cell c, offset h (clamped to the domain).
-__device__ __forceinline__ LaneBox boxAround(int lane, int L, int4 c, float4 h, float reach, const GridDev& g)
+__device__ __forceinline__ RowBox rowsAround(bool live, int4 c, float4 h, float reach, const GridDev& g)
 {
-    LaneBox b;
-    b.u = lane - L;
-    b.p = b.pe = 0;
-    b.x0 = max(0, c.x + (int)floorf((h.x - reach) / g.cs.x));
-    b.y0 = max(0, c.y + (int)floorf((h.y - reach) / g.cs.y));
-    b.z0 = max(0, c.z + (int)floorf((h.z - reach) / g.cs.z));
-    const int x1 = min(g.gx - 1, c.x + (int)floorf((h.x + reach) / g.cs.x));
-    const int y1 = min(g.gy - 1, c.y + (int)floorf((h.y + reach) / g.cs.y));
-    const int z1 = min(g.gz - 1, c.z + (int)floorf((h.z + reach) / g.cs.z));
-    b.nx = max(0, x1 - b.x0 + 1);
-    b.ny = max(0, y1 - b.y0 + 1);
-    b.nz = max(0, z1 - b.z0 + 1);
-    b.hx = b.hy = b.hz = b.hash = 0;
-    b.ix = lane - L;  // cell u = lane - L: one advance of L reaches the lane's first cell
-    b.iy = b.iz = 0;
+    RowBox b;
     b.c = c;
     b.h = h;
     // the candidate test keeps partners up to 1e-4 past the reach (squared);
     // the gaps carry a few FP32 roundings of the cell size
-    const float wide = reach * 1.001f + 1.e-5f * (g.cs.x + g.cs.y + g.cs.z);
-    b.reach2 = wide * wide;
+    b.wide = reach * 1.001f + 1.e-5f * (g.cs.x + g.cs.y + g.cs.z);
+    int z0;
+    cellRange(c.y, h.y - b.wide, h.y + b.wide, g.cs.y, g.gy, b.y0, b.y1);
+    cellRange(c.z, h.z - b.wide, h.z + b.wide, g.cs.z, g.gz, z0, b.z1);
+    if (!live) b.z1 = z0 - 1;
+    b.y = b.y1;  // one advance reaches the first row
+    b.z = z0 - 1;
+    b.gz2 = b.ry = b.rz = 0.f;
     return b;
 }
+// The next row that holds members: their range of the sorted order.
+__device__ __forceinline__ bool nextRow(RowBox& b, const int* __restrict__ start, const GridDev& g, int& p, int& e)
+{
+    while (true) {
+        if (++b.y > b.y1) {
+            if (++b.z > b.z1) return false;
+            b.y = b.y0;
+            if (b.y > b.y1) return false;
+            const float gz = cellGap(b.z, b.c.z, b.h.z, g.cs.z);
+            b.gz2 = gz * gz;
+            b.rz = b.h.z + (float)(b.c.z - b.z) * g.cs.z;
+        }
+        const float gy = cellGap(b.y, b.c.y, b.h.y, g.cs.y);
+        const float rest = b.wide * b.wide - gy * gy - b.gz2;
+        if (rest < 0.f) continue;
+        const float rx = sqrtf(rest);
+        int x0, x1;
+        cellRange(b.c.x, b.h.x - rx, b.h.x + rx, g.cs.x, g.gx, x0, x1);
+        if (x0 > x1) continue;
+        const int row = (b.z * g.gy + b.y) * g.gx;
+        p = start[row + x0];
+        e = start[row + x1 + 1];
+        b.ry = b.h.y + (float)(b.c.y - b.y) * g.cs.y;
+        if (p < e) return true;
+    }
+}
 
-// The walk writes either the lists themselves (BUILD_LISTS: the reference's
-// walk every fluid step) or Verlet candidates (within the cut + fskin) that
-// kFluidFilter turns into the lists on the following fluid steps.
-enum WalkMode { BUILD_LISTS = 0, BUILD_CANDIDATES = 1 };
+// Calls test(p, box, id) for the members p of the box's rows and emit(k, id)
+// for those taken, k counting them in sorted order; returns their number.  A
+// group of L lanes shares the members (L at a time; a ballot keeps the order),
+// a single lane reads BATCH members ahead of their tests through
+// load(p, box): the particles of a warp are neighbours in the sorted order, so
+// their reads fall into the same few lines.
+template <int L, class Load, class Test, class Emit>
+__device__ __forceinline__ int takeMembers(RowBox& box, const int* __restrict__ start, const GridDev& g, bool live,
+                                           int lane, Load load, Test test, Emit emit)
+{
+    int k = 0, p = 0, e = 0;
+    if constexpr (L == 1) {
+        constexpr int BATCH = 4;
+        while (live && nextRow(box, start, g, p, e)) {
+            for (; p < e; p += BATCH) {
+                decltype(load(0)) m[BATCH];
+#pragma unroll
+                for (int u = 0; u < BATCH; ++u) m[u] = load(min(p + u, e - 1));
+#pragma unroll
+                for (int u = 0; u < BATCH; ++u)
+                    if (p + u < e && test(m[u], box)) emit(k++, m[u]);
+            }
+        }
+    } else {
+        const int groupShift = (threadIdx.x & 31) & ~(L - 1);
+        const unsigned groupBits = (1u << L) - 1u, below = (1u << lane) - 1u;
+        bool more = live;
+        while (true) {
+            if (more && p >= e) more = nextRow(box, start, g, p, e);
+            if (!__any_sync(0xffffffffu, more)) break;
+            decltype(load(0)) m;
+            bool take = false;
+            if (more && p + lane < e) {
+                m = load(p + lane);
+                take = test(m, box);
+            }
+            const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
+            if (take) emit(k + __popc(mine & below), m);
+            k += __popc(mine);
+            p += L;
+        }
+    }
+    return k;
+}
 
-template <int L, int MODE>
-__device__ __forceinline__ void fluidWalk(const DeviceState& d, RunIf when)
+// Verlet candidates of the fluid lists, of one particle by a group of L lanes:
+// every fluid within the largest cut + fskin and every solid within 2 h +
+// fskin, in sorted order (all particles are inside the domain here: one
+// outside it sends the lists back to the walk).  P (cellPack): a fluid
+// partner's cell and offset are its filter record, one 16-byte read.
+//
+// What bounds it: instruction issue.  Walking the cells one by one (64 cells
+// of a box, 8 members each, every lane at its own cell) took 836M warp
+// instructions for 400k particles at one lane each, 1017 us; a row's members
+// are one loop: 303M, 438 us (48k particles, eight lanes: 158 to 120 us).
+template <int L, bool P>
+__device__ __forceinline__ void fluidCandidates(const DeviceState& d)
 {
     const int th = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((th & ~31) >= d.nf * L || *d.status || !when.active()) return;
+    if ((th & ~31) >= d.nf * L) return;
+    const int i = th / L, lane = th % L;
+    const bool live = i < d.nf;
+    const int n = d.nf;
+    int4 ci = make_int4(0, 0, 0, 0);
+    float4 hi = make_float4(0, 0, 0, 0);
+    if (live) {
+        ci = d.fcell[i];
+        hi = d.fph[0][i];
+    }
+    const float skin = d.fskin;
+    const float4* __restrict__ rec = d.fcp;
+    struct Member {
+        float4 h;
+        int x, id;
+    };
+    // squared cut of a pair, widened past the rounding of the estimate below
+    const auto cut2 = [&](float h) {
+        const float c = 2.f * h + skin;
+        return c * c * (1.f + 1.e-4f);
+    };
+    const float cut2U = cut2(hi.w);
+    const auto within = [&](const Member& m, const RowBox& b, float dc, float c2) {
+        const float rx = (hi.x - m.h.x) + dc * d.grid.cs.x, ry = b.ry - m.h.y, rz = b.rz - m.h.z;
+        return rx * rx + ry * ry + rz * rz <= c2;
+    };
+    RowBox boxF = rowsAround(live, ci, hi, 2.f * fmaxf(hi.w, d.fhmax) + skin, d.grid);
+    const int nff = takeMembers<L>(
+        boxF, d.fcellStart, d.grid, live, lane,
+        [&](int p) {
+            Member m;
+            m.id = p;
+            if constexpr (P) {
+                m.h = __ldg(rec + p);
+                m.x = (int)(__float_as_uint(m.h.w) & 2047u);
+            } else {
+                m.h = d.fph[0][p];
+                m.x = d.fcell[p].x;
+            }
+            return m;
+        },
+        [&](const Member& m, const RowBox& b) {
+            // a packed cell's x + 2^23 as a float: no integer conversion per member
+            const float dc = P ? ((float)ci.x + 8388608.f) - __uint_as_float(0x4b000000u | (unsigned)m.x)
+                               : (float)(ci.x - m.x);
+            return within(m, b, dc, P ? cut2U : cut2(fmaxf(hi.w, m.h.w))) && m.id != i;
+        },
+        [&](int k, const Member& m) {
+            if (k < d.kvf) d.fvc[(size_t)k * n + i] = (unsigned)m.id;
+        });
+    RowBox boxS = rowsAround(live, ci, hi, 2.f * hi.w + skin, d.grid);
+    const int nfs = takeMembers<L>(
+        boxS, d.scellStart, d.grid, live, lane,
+        [&](int p) {
+            Member m;
+            m.id = d.ssorted[p];
+            m.h = d.sph[m.id];
+            m.x = d.scell[m.id].x;
+            return m;
+        },
+        [&](const Member& m, const RowBox& b) { return within(m, b, (float)(ci.x - m.x), cut2U); },
+        [&](int k, const Member& m) {
+            if (k < d.kvs) d.fvsc[(size_t)k * n + i] = m.id;
+        });
+    if (!live || lane != 0) return;
+    d.fvcn[i] = nff;
+    d.fvsn[i] = nfs;
+    d.fvref[i] = make_float4((float)ci.x * d.grid.cs.x + hi.x, (float)ci.y * d.grid.cs.y + hi.y,
+                             (float)ci.z * d.grid.cs.z + hi.z, 0.f);
+    if (nff > d.kvf || nfs > d.kvs) {
+        atomicOr(d.status, ST_FVERLET_OVERFLOW);
+        atomicMax(&d.need[2], nff);
+        atomicMax(&d.need[3], nfs);
+    }
+}
+
+// The lists from the reference's 27-cell walk (every fluid step once a particle
+// has left the domain, or at initialisation).
+template <int L>
+__device__ __forceinline__ void fluidWalk(const DeviceState& d)
+{
+    const int th = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((th & ~31) >= d.nf * L) return;
     const int i = th / L, lane = th % L;
     const bool live = i < d.nf;
     const int groupShift = (threadIdx.x & 31) & ~(L - 1);
     const unsigned groupBits = L == 32 ? 0xffffffffu : ((1u << L) - 1u);
     const unsigned below = (1u << lane) - 1u;
     const int n = d.nf;
-    const float skin = MODE == BUILD_CANDIDATES ? d.fskin : 0.f;
-    const int capF = MODE == BUILD_CANDIDATES ? d.kvf : d.kff;
-    const int capS = MODE == BUILD_CANDIDATES ? d.kvs : d.kfs;
     int4 ci = make_int4(0, 0, 0, 0);
     float4 hi = make_float4(0, 0, 0, 0), li = hi;
     dfl hI = df_make(0.f), cutS = hI;
@@ -199,29 +324,13 @@ __device__ __forceinline__ void fluidWalk(const DeviceState& d, RunIf when)
     // a walk position gives the partner's cell offset from the particle's own
     // cell only when the walk is centred on that cell
     const bool centred = sx == ci.x && sy == ci.y && sz == ci.z;
-    // candidates: every cell within the largest cut + skin, all inside the
-    // domain (particles outside it send the lists back to the walk)
-    LaneBox boxF, boxS;
-    if (MODE == BUILD_CANDIDATES) {
-        boxF = boxAround(lane, L, ci, hi, 2.f * fmaxf(hi.w, d.fhmax) + skin, d.grid);
-        boxS = boxAround(lane, L, ci, hi, 2.f * hi.w + skin, d.grid);
-        if (!live) boxF.nx = boxS.nx = 0;
-    }
     // fluid partners
     int nff = 0;
     {
         LaneWalk w{lane - L, 0, 0, 0, 0, 0, 0, false};
         while (true) {
             int j = 0;
-            const bool has = live && (MODE == BUILD_CANDIDATES ? nextBoxMember<L>(boxF, d.fcellStart, d.grid, j)
-                                                               : nextCandidate<L>(w, d.fcellStart, sx, sy, sz, d.grid, j));
-            if (MODE == BUILD_CANDIDATES) {
-                w.regular = true;
-                w.hx = boxF.hx;
-                w.hy = boxF.hy;
-                w.hz = boxF.hz;
-                w.hash = boxF.hash;
-            }
+            const bool has = live && nextCandidate<L>(w, d.fcellStart, sx, sy, sz, d.grid, j);
             bool take = false;
             int4 cj = make_int4(0, 0, 0, 0);
             if (has && j != i) {
@@ -230,11 +339,9 @@ __device__ __forceinline__ void fluidWalk(const DeviceState& d, RunIf when)
                 // FP32 decision away from the cut (most candidates); the exact
                 // double-float test within 1e-5 of it
                 const float3 r = relF(ci, hi, cj, hj, d.grid);
-                const float c = 2.f * fmaxf(hi.w, hj.w) + skin;
+                const float c = 2.f * fmaxf(hi.w, hj.w);
                 const float d2 = dot3(r, r), c2 = c * c;
-                if (MODE == BUILD_CANDIDATES) {
-                    take = d2 <= c2 * (1.f + 1.e-4f);
-                } else if (d2 < c2 * (1.f - 1.e-5f)) {
+                if (d2 < c2 * (1.f - 1.e-5f)) {
                     take = true;
                 } else if (d2 <= c2 * (1.f + 1.e-5f)) {
                     const dfl hJ = df_make(hj.w, d.fpl[0][j].w);
@@ -245,10 +352,7 @@ __device__ __forceinline__ void fluidWalk(const DeviceState& d, RunIf when)
             const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
             if (take) {
                 const int slot = nff + __popc(mine & below);
-                if (slot < capF) {
-                    if (MODE == BUILD_CANDIDATES) d.fvc[(size_t)slot * n + i] = (unsigned)j;
-                    else d.ff[(size_t)slot * n + i] = ffEntry(j, w.t, w.regular && centred);
-                }
+                if (slot < d.kff) d.ff[(size_t)slot * n + i] = ffEntry(j, w.t, w.regular && centred);
             }
             nff += __popc(mine);
             if (!__any_sync(0xffffffffu, has)) break;
@@ -260,15 +364,7 @@ __device__ __forceinline__ void fluidWalk(const DeviceState& d, RunIf when)
         LaneWalk w{lane - L, 0, 0, 0, 0, 0, 0, false};
         while (true) {
             int p = 0;
-            const bool has = live && (MODE == BUILD_CANDIDATES ? nextBoxMember<L>(boxS, d.scellStart, d.grid, p)
-                                                               : nextCandidate<L>(w, d.scellStart, sx, sy, sz, d.grid, p));
-            if (MODE == BUILD_CANDIDATES) {
-                w.regular = true;
-                w.hx = boxS.hx;
-                w.hy = boxS.hy;
-                w.hz = boxS.hz;
-                w.hash = boxS.hash;
-            }
+            const bool has = live && nextCandidate<L>(w, d.scellStart, sx, sy, sz, d.grid, p);
             bool take = false;
             int a = 0;
             if (has) {
@@ -276,41 +372,25 @@ __device__ __forceinline__ void fluidWalk(const DeviceState& d, RunIf when)
                 const int4 ca = w.regular ? make_int4(w.hx, w.hy, w.hz, w.hash) : d.scell[a];
                 const float4 ha = d.sph[a];
                 const float3 r = relF(ci, hi, ca, ha, d.grid);
-                const float c = 2.f * hi.w + skin;
+                const float c = 2.f * hi.w;
                 const float d2 = dot3(r, r), c2 = c * c;
-                if (MODE == BUILD_CANDIDATES) take = d2 <= c2 * (1.f + 1.e-4f);
-                else if (d2 < c2 * (1.f - 1.e-5f)) take = true;
+                if (d2 < c2 * (1.f - 1.e-5f)) take = true;
                 else if (d2 <= c2 * (1.f + 1.e-5f)) take = withinCut(ci, hi, li, ca, ha, d.spl, a, cutS, d.grid);
             }
             const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
             if (take) {
                 const int slot = nfs + __popc(mine & below);
-                if (slot < capS) {
-                    if (MODE == BUILD_CANDIDATES) d.fvsc[(size_t)slot * n + i] = a;
-                    else d.fs[(size_t)slot * n + i] = fsEntry(a, w.t);
-                }
+                if (slot < d.kfs) d.fs[(size_t)slot * n + i] = fsEntry(a, w.t);
             }
             nfs += __popc(mine);
             if (!__any_sync(0xffffffffu, has)) break;
         }
     }
     if (!live || lane != 0) return;
-    if (MODE == BUILD_CANDIDATES) {
-        d.fvcn[i] = nff;
-        d.fvsn[i] = nfs;
-        d.fvref[i] = make_float4((float)ci.x * d.grid.cs.x + hi.x, (float)ci.y * d.grid.cs.y + hi.y,
-                                 (float)ci.z * d.grid.cs.z + hi.z, 0.f);
-        if (nff > capF || nfs > capS) {
-            atomicOr(d.status, ST_FVERLET_OVERFLOW);
-            atomicMax(&d.need[2], nff);
-            atomicMax(&d.need[3], nfs);
-        }
-    } else {
-        d.ffc[i] = nff;
-        d.fsc[i] = nfs;
-        if (nff > d.kff) atomicOr(d.status, ST_FF_OVERFLOW);
-        if (nfs > d.kfs) atomicOr(d.status, ST_FS_OVERFLOW);
-    }
+    d.ffc[i] = nff;
+    d.fsc[i] = nfs;
+    if (nff > d.kff) atomicOr(d.status, ST_FF_OVERFLOW);
+    if (nfs > d.kfs) atomicOr(d.status, ST_FS_OVERFLOW);
 }
 
 // Walk position (0..26) of cell cj in the 27-cell walk centred on ci, or -1.
@@ -819,16 +899,17 @@ __global__ void kSolidNormals(DeviceState d, double h)
 // domain), else the Verlet candidates when they are stale - with the contact
 // rows' positions at the rebuild (a solid moving half the fluid margin since
 // then makes the candidates stale) - else nothing.
-template <int L>
+template <int L, bool P>
 __global__ void __launch_bounds__(T) kFluidWalk(DeviceState d, RunIf lists, RunIf cands)
 {
     stepKernelBegin();
+    if (*d.status) return;
     if (lists.active()) {
-        fluidWalk<L, BUILD_LISTS>(d, lists);
+        fluidWalk<L>(d);
         return;
     }
     if (!cands.active()) return;
-    fluidWalk<L, BUILD_CANDIDATES>(d, cands);
+    fluidCandidates<L, P>(d);
     if (*d.status) return;
     const auto ref = [&](int a) {
         const int4 c = d.scell[a];
@@ -857,7 +938,8 @@ void launchFluidWalk(const DeviceState& d, bool walk, cudaStream_t s)
     cands.a = d.frebuild;
     cands.unless = d.fslowMode;
     cands.unless2 = d.slowMode;
-    LAUNCH_LANES(kFluidWalk, d.lanes, d.nf, T, s, d, lists, cands);
+    if (d.cellPack) LAUNCH_LANES_U(kFluidWalk, true, d.lanes, d.nf, T, s, d, lists, cands);
+    else LAUNCH_LANES_U(kFluidWalk, false, d.lanes, d.nf, T, s, d, lists, cands);
 }
 
 void launchFluidFilter(const DeviceState& d, cudaStream_t s)
