@@ -159,16 +159,16 @@ void allocFluidLists(demsph_engine* e)
 {
     DeviceState& d = e->d;
     // in tile mode the fluid list exists only for exports (made on demand)
-    if (!d.fluidTiles) d.ff = dalloc<unsigned>((size_t)d.kff * d.nf, e->owned, e->stream, false);
-    d.fs = dalloc<int>((size_t)d.kfs * d.nf, e->owned, e->stream, false);
+    if (!d.fluidTiles) d.ff = dalloc<unsigned>(listEntries(d.kff, d.nf), e->owned, e->stream, false);
+    d.fs = dalloc<int>(listEntries(d.kfs, d.nf), e->owned, e->stream, false);
     if (e->debug & 1) d.fsPairForce = dalloc<float4>((size_t)d.kfs * d.nf, e->owned, e->stream);
 }
 
 void allocFluidCandidates(demsph_engine* e)
 {
     DeviceState& d = e->d;
-    d.fvc = dalloc<unsigned>((size_t)d.kvf * d.nf, e->owned, e->stream, false);
-    d.fvsc = dalloc<int>((size_t)d.kvs * d.nf, e->owned, e->stream, false);
+    d.fvc = dalloc<unsigned>(listEntries(d.kvf, d.nf), e->owned, e->stream, false);
+    d.fvsc = dalloc<int>(listEntries(d.kvs, d.nf), e->owned, e->stream, false);
 }
 
 // Per-slot arrays of the contact rows (scap slots per row).
@@ -602,7 +602,7 @@ void grow(demsph_engine* e, int status)
         // a particle left the domain: the lists come from the reference's walk
         // (the list kernels) from now on
         d.fluidTiles = 0;
-        if (!d.ff) d.ff = dalloc<unsigned>((size_t)d.kff * d.nf, e->owned, e->stream, false);
+        if (!d.ff) d.ff = dalloc<unsigned>(listEntries(d.kff, d.nf), e->owned, e->stream, false);
         if (!d.fvc) allocFluidCandidates(e);
     }
     if (status & ST_MODE_CHANGE) {
@@ -794,7 +794,6 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
                 id[i] = i;
             }
             d.fcell = dalloc<int4>(nf, e->owned, e->stream);
-            d.fcp = dalloc<float4>(nf, e->owned, e->stream);
             for (int b = 0; b < 2; ++b) {
                 d.fph[b] = dalloc<float4>(nf, e->owned, e->stream);
                 d.fpl[b] = dalloc<float4>(nf, e->owned, e->stream);
@@ -802,7 +801,7 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
                 d.fvl[b] = dalloc<float4>(nf, e->owned, e->stream);
                 d.fdrho[b] = dalloc<float>(nf, e->owned, e->stream);
             }
-            for (int b = 0; b < 3; ++b) d.fpd[b] = dalloc<float4>(nf, e->owned, e->stream);
+            for (int b = 0; b < 3; ++b) d.frec[b] = dalloc<FluidRec>(nf, e->owned, e->stream);
             d.facc = dalloc<float4>(nf, e->owned, e->stream);
             d.fpar = dalloc<float4>(nf, e->owned, e->stream);
             d.fsumW0 = dalloc<float2>(nf, e->owned, e->stream);
@@ -1280,6 +1279,8 @@ int demsph_fluid_integrate(demsph_engine* e, double dt, int i_step, int gap)
     if (gap < 1) return DEMSPH_ERR_ARGUMENT;
     ENGINE_GUARD(e)
     REQUIRE_INIT(e);
+    // the state may have been set since the last search
+    launchFluidRecords(e->d, e->stream);
     stageFluid(e, dt, i_step, gap);
     CK(cudaGetLastError());
     return DEMSPH_OK;
@@ -1574,6 +1575,7 @@ int demsph_autotune(demsph_engine* e, int* lanes_out)
         CK(cudaEventCreate(&b));
         float best = 0.f;
         int bestL = d.lanes;
+        launchFluidRecords(d, e->stream);
         for (int L = 1; L <= 8; L *= 2) {
             d.lanes = L;
             launchContinuityPass(d, 0, 1.0e-9, e->stream);  // warm-up
@@ -1629,7 +1631,7 @@ long long demsph_estimate_bytes(const demsph_scene* sc, const demsph_options* op
     // solid: state, sort and wall springs; per contact row: its slots, two
     // list parities, springs in and out, candidates; per cell: counts and starts
     const long long kvf = kff + kff / 2, kvs = kfs + kfs / 2;
-    return nf * (380 + 4 * (kff + kfs) + 4 * (kvf + kvs)) + ns * (248 + 48LL * sc->n_wall) +
+    return nf * (444 + 4 * (kff + kfs) + 4 * (kvf + kvs) + 64) + ns * (248 + 48LL * sc->n_wall) +
            rows * (72 + slots * 184 + 2 * slots * 4) + (cells + 1) * 16 + (long long)sc->n_clump * 160 +
            std::min(64 * rows + 1024, std::max(1LL, kfs * nf)) * 4 + (1 << 20);
 }

@@ -662,12 +662,12 @@ int demsph_export_fluid_pairs(demsph_engine* e, int* prefix, int* pointed, int* 
             void* p = d.ff;
             freeOne(e, p);
             d.kff = std::max(d.kff, most);
-            d.ff = dalloc<unsigned>((size_t)d.kff * n, e->owned, e->stream, false);
+            d.ff = dalloc<unsigned>(listEntries(d.kff, n), e->owned, e->stream, false);
         }
         launchBitsToLists(d, e->stream);
         CK(cudaStreamSynchronize(e->stream));
     }
-    d2h(ff, d.ff, (size_t)d.kff * n);
+    d2h(ff, d.ff, listEntries(d.kff, n));
     d2h(ffc, d.ffc, n);
     d2h(id, d.fid, n);
     slot.resize(n);
@@ -681,7 +681,7 @@ int demsph_export_fluid_pairs(demsph_engine* e, int* prefix, int* pointed, int* 
         const int m = std::min(ffc[s], d.kff);
         order.clear();
         for (int k = 0; k < m; ++k) {
-            const unsigned v = ff[(size_t)k * n + s];
+            const unsigned v = ff[listAt(k, s, n)];
             order.push_back({(long long)entryWalk(v) * n + id[ffPartner(v)], ffPartner(v)});
         }
         std::sort(order.begin(), order.end());
@@ -712,7 +712,7 @@ int demsph_export_fluid_solid_pairs(demsph_engine* e, int* prefix, int* pointed,
     const int n = d.nf;
     std::vector<int> fs, fsc, id, slot;
     std::vector<float4> pf;
-    d2h(fs, d.fs, (size_t)d.kfs * n);
+    d2h(fs, d.fs, listEntries(d.kfs, n));
     d2h(fsc, d.fsc, n);
     d2h(id, d.fid, n);
     if (d.fsPairForce) d2h(pf, d.fsPairForce, (size_t)d.kfs * n);
@@ -725,7 +725,7 @@ int demsph_export_fluid_solid_pairs(demsph_engine* e, int* prefix, int* pointed,
         const int m = std::min(fsc[s], d.kfs);
         order.clear();
         for (int k = 0; k < m; ++k) {
-            const int v = fs[(size_t)k * n + s];
+            const int v = fs[listAt(k, s, n)];
             order.push_back({(long long)entryWalk((unsigned)v) * d.ns + fsPartner(v), k});
         }
         std::sort(order.begin(), order.end());  // walk position, then index
@@ -733,7 +733,7 @@ int demsph_export_fluid_solid_pairs(demsph_engine* e, int* prefix, int* pointed,
             const int k = o.second;
             if (w < cap) {
                 if (pointed) pointed[w] = i;
-                if (pointing) pointing[w] = fsPartner(fs[(size_t)k * n + s]);
+                if (pointing) pointing[w] = fsPartner(fs[listAt(k, s, n)]);
                 if (force) {
                     const float4 f = pf.empty() ? make_float4(0, 0, 0, 0) : pf[(size_t)k * n + s];
                     force[3 * w] = f.x;

@@ -46,7 +46,10 @@ __device__ __forceinline__ void fluidHashOne(const DeviceState& d, int i, const 
         d.fcell[i] = c;
         d.fph[0][i] = h;
         d.fpl[0][i] = l;
-        if (d.cellPack) d.fcp[i] = make_float4(h.x, h.y, h.z, packCell(c));
+        if (d.uniformFluid) {
+            const float4 v = d.fvh[0][i];
+            d.frec[0][i] = FluidRec{make_float4(h.x, h.y, h.z, packCell(c)), make_float4(v.x, v.y, v.z, d.fdrho[0][i])};
+        }
         return;
     }
     // copy the whole particle into the gather sources
@@ -106,11 +109,14 @@ __device__ __forceinline__ void fluidGatherOne(const DeviceState& d, int p)
     const float4 h = d.fph[1][e];
     d.fcell[q] = c;
     d.fph[0][q] = h;
-    if (d.cellPack) d.fcp[q] = make_float4(h.x, h.y, h.z, packCell(c));
     d.fpl[0][q] = d.fpl[1][e];
-    d.fvh[0][q] = d.fvh[1][e];
+    const float4 v = d.fvh[1][e];
+    const float dr = d.fdrho[1][e];
+    d.fvh[0][q] = v;
     d.fvl[0][q] = d.fvl[1][e];
-    d.fdrho[0][q] = d.fdrho[1][e];
+    d.fdrho[0][q] = dr;
+    if (d.uniformFluid)
+        d.frec[0][q] = FluidRec{make_float4(h.x, h.y, h.z, packCell(c)), make_float4(v.x, v.y, v.z, dr)};
     d.facc[q] = d.tacc[e];
     d.fpar[q] = d.tpar[e];
     d.fsumW0[q] = d.tsumW0[e];

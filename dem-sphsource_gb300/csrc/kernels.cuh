@@ -164,6 +164,13 @@ inline void launchStepSmem(void (*kernel)(KArgs...), unsigned grid, unsigned blo
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// A fluid partner in one sector: position offset and packed cell (packCell),
+// velocity and density difference.
+struct alignas(32) FluidRec {
+    float4 pc;   // offset xyz, cell bits w
+    float4 vd;   // velocity xyz, density - rest density w
+};
+
 struct DeviceState {
     GridDev grid;
     double minB[3], cs[3];   // FP64 grid, for import and export
@@ -182,21 +189,19 @@ struct DeviceState {
     float4 fparU;            // speed, viscosity, mass) and the same smoothing length
     float4 fconstU;          // with them: 4 h^2, 0.5 / h, KG / h^5, 1 / sound speed
     int4* fcell;
-    // filter records of uniform fluids on grids of at most 2048 x 2048 x 1024
-    // cells (cellPack): the position offset of fph[0] and the cell packed in w
-    // (packCell), as each fluid step's hash or reorder leaves them
-    float4* fcp;
-    int cellPack;
+    int cellPack;            // uniform fluids on a grid whose cells packCell holds (2048 x 2048 x 1024)
     float4* fph[2];
     float4* fpl[2];
     float4* fvh[2];
     float4* fvl[2];
     float* fdrho[2];
-    // partner records of the uniform-fluid pair loops (position offset xyz,
-    // density w: one 16-byte gather): [0] position 0 with density 0 (the
-    // first continuity pass), [1] position 1 with density 1 (momentum), [2]
-    // position 0 with density 1 (the second continuity pass)
-    float4* fpd[3];
+    // partner records of uniform fluids (FluidRec: all a pair term reads of its
+    // partner, one 32-byte sector): [0] position 0, density 0 and velocity 0 as
+    // each fluid step's hash or reorder leaves them (list candidates, filter,
+    // first continuity pass), [1] position 1, density 1 and velocity 0
+    // (momentum), [2] position 0, density 1 and velocity 1 (second continuity
+    // pass)
+    FluidRec* frec[3];
     float4* facc;
     float4* fpar;
     float2* fsumW0;          // Shepard reference sum / sigma(h), double-float
@@ -216,9 +221,9 @@ struct DeviceState {
     // Verlet candidates of the fluid lists (slots as of the last reorder):
     // partners within the list cut + fskin at the last rebuild
     int kvf, kvs;            // fluid / solid candidates per fluid particle
-    unsigned* fvc;           // [k * nf + i]
+    unsigned* fvc;           // entry k of slot i at listAt(k, i, nf)
     int* fvcn;
-    int* fvsc;               // [k * nf + i] solid indices
+    int* fvsc;               // the same, solid indices
     int* fvsn;
     float4* fvref;           // per fluid slot: position (from the grid origin) at the rebuild
     float4* svref;           // per solid (those with a contact row or moved): the same
@@ -234,8 +239,8 @@ struct DeviceState {
     unsigned* fbits;
     int* fwalk;              // candidates of each fluid slot's walk
     int kbits;
-    // lists (column-major, stride nf); with membership bits ff is made from
-    // the bits for exports only
+    // lists (entry k of slot i at listAt(k, i, nf)); with membership bits ff is
+    // made from the bits for exports only
     unsigned* ff;
     int* ffc;
     int* fs;
@@ -411,9 +416,11 @@ struct RunIf {
     }
 };
 
-// Lanes per fluid particle in the fluid pair loops and list builder: enough
-// threads for every SM (152 SMs x 2048) when the scene is small, one lane per
-// particle when it is large.
+// Lanes per fluid particle in the fluid pair loops: enough threads for every SM
+// (152 SMs x 2048) when the scene is small, two when it is large (they share a
+// list sector: a step of 400k particles takes 793 us with one lane, 688 with
+// two, 697 with four; of 1.0M 1756, 1578, 1628; of 120k 333, 253, 233 and 239
+// with eight).
 int fluidLanes(int nf);
 
 // Launches kernel<L> (L in 1, 2, 4, 8) over n items x L lanes.
@@ -496,6 +503,9 @@ void launchSolidNormals(const DeviceState& d, double h, cudaStream_t s);
 
 // sph.cu
 void launchDensityReinit(const DeviceState& d, int iStep, cudaStream_t s);
+// The first continuity pass's partner records from the state, for passes that no
+// neighbour search precedes (the search's hash leaves them otherwise).
+void launchFluidRecords(const DeviceState& d, cudaStream_t s);
 // which = 0: first half step (densities 0 -> 1, positions drift 0 -> 1);
 // which = 1: second half step (densities 1 -> 0, velocities 1 -> 0).
 // countStep: the pass counts the step in stepsDone (the last kernel of a step)

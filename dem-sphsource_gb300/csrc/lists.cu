@@ -10,15 +10,17 @@
 // Here the same walk, the same order and the same membership test (a FP32
 // distance with a 1e-5 margin, and a double-float distance inside the margin,
 // so decisions agree with the FP64 reference), but:
-//   * fluid lists are FULL lists (both directions) per fluid slot, column-major
-//     ([k * n + i]) so a warp reads one coalesced 128-byte line per entry, and
-//     each entry carries the cell delta of the pair so the SPH loops never
-//     load the partner's cell;
+//   * fluid lists are FULL lists (both directions) per fluid slot, in sectors
+//     of eight entries (listAt), and each entry carries the cell delta of the
+//     pair so the SPH loops never load the partner's cell;
 //   * solid contacts are a forward CSR (A < B, by original index - the
 //     reference's list exactly) plus a per-particle reverse CSR of the lower
 //     partners, both filled in walk order; spring history is remapped by
 //     looking the pair (A, B) up in A's previous forward segment, which holds
 //     the same springs the reference finds through B's reverse span.
+#include <algorithm>
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "contact_rows.cuh"
 
@@ -28,12 +30,6 @@ namespace {
 
 constexpr int T = 128;
 
-
-__device__ __forceinline__ unsigned deltaCode(int dx, int dy, int dz)
-{
-    if (dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1) return 27u;
-    return (unsigned)((dx + 1) + 3 * (dy + 1) + 9 * (dz + 1));
-}
 
 __device__ __forceinline__ dfl dfMax(dfl a, dfl b) { return (a.hi > b.hi || (a.hi == b.hi && a.lo >= b.lo)) ? a : b; }
 
@@ -92,18 +88,97 @@ __device__ __forceinline__ bool nextCandidate(LaneWalk& w, const int* __restrict
 }
 
 // ---- candidate rebuild: rows of cells ----
-// The cells within `reach` of a particle, as rows of cells along x: the cells
-// of one row are consecutive keys, so their members are ONE range of the sorted
-// order.  Rows and row ends beyond the reach (the corners and edges of the
-// box) are left out: no particle in them can be a candidate.
-struct RowBox {
-    int y, z, y0, y1, z1;  // the row taken last, and the box's bounds
-    int4 c;                // the particle's cell
-    float4 h;              // and its offset in it
-    float wide;            // reach, widened past the FP32 rounding of the cell gaps
-    float gz2;             // squared gap to the cells of plane z
-    float ry, rz;          // the particle's y and z from the row's cells' corner
+// Lanes of a particle in the list kernels of small scenes (walk, candidate
+// rebuild, filter), whatever the pair loops use: eight lanes read neighbouring
+// members or one sector of candidates, and write whole sectors of their list.
+constexpr int LIST_LANES = 8;
+
+// Appends entries to the list of a particle (row layout listAt) from its
+// LIST_LANES lanes: the lanes' entries are collected in shared memory and
+// written a full 32-byte sector at a time.  Called by whole warps; `ring` holds
+// two sectors per particle of the block.
+struct ListRing {
+    unsigned v[T / LIST_LANES][16];
 };
+struct ListWriter {
+    unsigned* ring;
+    unsigned* out;  // first sector of the particle's list
+    size_t stride;  // from one of its sectors to the next
+    int k, cap;
+    __device__ __forceinline__ ListWriter(ListRing& r, unsigned* list, int i, int n, int capacity)
+        : ring(r.v[threadIdx.x / LIST_LANES]), out(list + (size_t)i * 8), stride((size_t)n * 8), k(0), cap(capacity)
+    {
+    }
+    __device__ __forceinline__ void add(bool take, unsigned value)
+    {
+        const int lane = threadIdx.x & (LIST_LANES - 1), shift = (threadIdx.x & 31) & ~(LIST_LANES - 1);
+        const unsigned mine = (__ballot_sync(0xffffffffu, take) >> shift) & ((1u << LIST_LANES) - 1u);
+        if (take) ring[(k + __popc(mine & ((1u << lane) - 1u))) & 15] = value;
+        __syncwarp();
+        const int next = k + __popc(mine);
+        if ((next ^ k) & ~7) {  // a sector is full
+            const int sector = k >> 3;
+            if (sector * 8 < cap) out[sector * stride + lane] = ring[((sector & 1) << 3) + lane];
+        }
+        k = next;
+        __syncwarp();
+    }
+    // the last sector, part full; returns the number of entries
+    __device__ __forceinline__ int finish()
+    {
+        const int lane = threadIdx.x & (LIST_LANES - 1), sector = k >> 3;
+        if (lane < (k & 7) && sector * 8 < cap) out[sector * stride + lane] = ring[((sector & 1) << 3) + lane];
+        __syncwarp();
+        return k;
+    }
+};
+
+// The same for one lane per particle (large scenes): each thread collects its
+// entries in two sectors of its own in shared memory.  flush() is called at
+// least once per eight add().
+struct LaneRing {
+    unsigned v[16][T];
+};
+struct LaneWriter {
+    LaneRing& ring;
+    unsigned* out;
+    size_t stride;
+    int k, done, cap;  // entries, sectors written, capacity
+    __device__ __forceinline__ LaneWriter(LaneRing& r, unsigned* list, int i, int n, int capacity)
+        : ring(r), out(list + (size_t)i * 8), stride((size_t)n * 8), k(0), done(0), cap(capacity)
+    {
+    }
+    // without a branch: an entry not taken is overwritten by the next
+    __device__ __forceinline__ void add(bool take, unsigned value)
+    {
+        ring.v[k & 15][threadIdx.x] = value;
+        k += take ? 1 : 0;
+    }
+    __device__ __forceinline__ void flush()
+    {
+        if ((k >> 3) != done) sector();
+    }
+    __device__ __forceinline__ void sector()
+    {
+        if (done * 8 < cap) {
+            unsigned e[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) e[u] = ring.v[((done & 1) << 3) + u][threadIdx.x];
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out), "r"(e[0]), "r"(e[1]), "r"(e[2]),
+                         "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7])
+                         : "memory");
+        }
+        out += stride;
+        ++done;
+    }
+    __device__ __forceinline__ int finish()
+    {
+        flush();
+        if (k & 7) sector();  // the entries past the count are never read as partners
+        return k;
+    }
+};
+
 __device__ __forceinline__ float cellGap(int k, int c, float h, float cs)
 {
     const float lo = (float)(k - c) * cs - h, hi = h - (float)(k - c + 1) * cs;
@@ -115,112 +190,158 @@ __device__ __forceinline__ void cellRange(int c, float lo, float hi, float cs, i
     first = max(0, c + (int)floorf(lo / cs));
     last = min(n - 1, c + (int)floorf(hi / cs));
 }
-__device__ __forceinline__ RowBox rowsAround(bool live, int4 c, float4 h, float reach, const GridDev& g)
+
+// Lists (id(m) in `to`, in sorted order) the members m = load(p) of the cells
+// within `reach` of a particle (cell c, offset h) that pass test(m, y, z) (y, z:
+// the particle's offset from the corner of the member's cell along those axes);
+// returns their number.  The cells of one row along x are
+// consecutive keys, so their members are ONE range of the sorted order; rows
+// and row ends beyond the reach (the corners and edges of the box) are left
+// out.  The eight lanes of the particle first take a row each and find its
+// range, then read the rows' members eight at a time; the four particles of a
+// warp go on together, each at its own row.  Called by whole warps.
+template <class Load, class Test>
+__device__ __forceinline__ int takeMembers(bool live, int4 c, float4 h, float reach, const int* __restrict__ start,
+                                           const GridDev& g, ListWriter to, Load load, Test test)
 {
-    RowBox b;
-    b.c = c;
-    b.h = h;
-    // the candidate test keeps partners up to 1e-4 past the reach (squared);
-    // the gaps carry a few FP32 roundings of the cell size
-    b.wide = reach * 1.001f + 1.e-5f * (g.cs.x + g.cs.y + g.cs.z);
-    int z0;
-    cellRange(c.y, h.y - b.wide, h.y + b.wide, g.cs.y, g.gy, b.y0, b.y1);
-    cellRange(c.z, h.z - b.wide, h.z + b.wide, g.cs.z, g.gz, z0, b.z1);
-    if (!live) b.z1 = z0 - 1;
-    b.y = b.y1;  // one advance reaches the first row
-    b.z = z0 - 1;
-    b.gz2 = b.ry = b.rz = 0.f;
-    return b;
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int L = LIST_LANES;
+    const int lane = threadIdx.x & (L - 1), groupShift = (threadIdx.x & 31) & ~(L - 1);
+    const unsigned groupBits = (1u << L) - 1u;
+    // widened past the slack of the candidate test (1e-4, squared) and the few
+    // FP32 roundings of the cell gaps
+    const float wide = reach * 1.001f + 1.e-5f * (g.cs.x + g.cs.y + g.cs.z);
+    int y0, y1, z0, z1;
+    cellRange(c.y, h.y - wide, h.y + wide, g.cs.y, g.gy, y0, y1);
+    cellRange(c.z, h.z - wide, h.z + wide, g.cs.z, g.gz, z0, z1);
+    const int ny = max(1, y1 - y0 + 1);
+    const int rows = live && y0 <= y1 && z0 <= z1 ? ny * (z1 - z0 + 1) : 0;
+    for (int base = 0; __any_sync(FULL, base < rows); base += L) {
+        const int row = base + lane;
+        int p = 0, e = 0;
+        float ry = 0.f, rz = 0.f;
+        if (row < rows) {
+            const int dz = row / ny, z = z0 + dz, y = y0 + row - dz * ny;
+            const float gy = cellGap(y, c.y, h.y, g.cs.y), gz = cellGap(z, c.z, h.z, g.cs.z);
+            const float rest = wide * wide - gy * gy - gz * gz;
+            if (rest >= 0.f) {
+                const float rx = sqrtf(rest);
+                int x0, x1;
+                cellRange(c.x, h.x - rx, h.x + rx, g.cs.x, g.gx, x0, x1);
+                if (x0 <= x1) {
+                    const int first = (z * g.gy + y) * g.gx;
+                    p = start[first + x0];
+                    e = start[first + x1 + 1];
+                }
+            }
+            ry = h.y + (float)(c.y - y) * g.cs.y;
+            rz = h.z + (float)(c.z - z) * g.cs.z;
+        }
+        unsigned todo = (__ballot_sync(FULL, p < e) >> groupShift) & groupBits;  // the particle's rows not begun
+        int q = 0, qe = 0;
+        float y = 0.f, z = 0.f;
+        while (true) {
+            const bool next = q >= qe && todo != 0u;
+            if (__any_sync(FULL, next)) {
+                const int r = next ? __ffs(todo) - 1 : 0;
+                const int np = __shfl_sync(FULL, p, r, L), ne = __shfl_sync(FULL, e, r, L);
+                const float nyo = __shfl_sync(FULL, ry, r, L), nzo = __shfl_sync(FULL, rz, r, L);
+                if (next) {
+                    q = np;
+                    qe = ne;
+                    y = nyo;
+                    z = nzo;
+                    todo &= todo - 1u;
+                }
+            }
+            if (!__any_sync(FULL, q < qe)) break;
+            bool take = false;
+            unsigned id = 0;
+            if (q + lane < qe) {
+                const auto m = load(q + lane);
+                take = test(m, y, z);
+                id = (unsigned)m.id;
+            }
+            to.add(take, id);
+            q += L;
+        }
+    }
+    return to.finish();
 }
-// The next row that holds members: their range of the sorted order.
-__device__ __forceinline__ bool nextRow(RowBox& b, const int* __restrict__ start, const GridDev& g, int& p, int& e)
+
+// The same by one lane: it takes row after row, and reads BATCH members ahead of
+// their tests (the particles of a warp are neighbours in the sorted order, so
+// their reads fall into the same few lines).
+struct RowBox {
+    int y, z, y0, y1, z1;  // the row taken last, and the box's bounds
+    float gz2, ry, rz;     // squared gap to plane z; the particle's y and z from the row's cells' corner
+};
+__device__ __forceinline__ bool nextRow(RowBox& b, int4 c, float4 h, float wide, const int* __restrict__ start,
+                                        const GridDev& g, int& p, int& e)
 {
     while (true) {
         if (++b.y > b.y1) {
             if (++b.z > b.z1) return false;
             b.y = b.y0;
             if (b.y > b.y1) return false;
-            const float gz = cellGap(b.z, b.c.z, b.h.z, g.cs.z);
+            const float gz = cellGap(b.z, c.z, h.z, g.cs.z);
             b.gz2 = gz * gz;
-            b.rz = b.h.z + (float)(b.c.z - b.z) * g.cs.z;
+            b.rz = h.z + (float)(c.z - b.z) * g.cs.z;
         }
-        const float gy = cellGap(b.y, b.c.y, b.h.y, g.cs.y);
-        const float rest = b.wide * b.wide - gy * gy - b.gz2;
+        const float gy = cellGap(b.y, c.y, h.y, g.cs.y);
+        const float rest = wide * wide - gy * gy - b.gz2;
         if (rest < 0.f) continue;
         const float rx = sqrtf(rest);
         int x0, x1;
-        cellRange(b.c.x, b.h.x - rx, b.h.x + rx, g.cs.x, g.gx, x0, x1);
+        cellRange(c.x, h.x - rx, h.x + rx, g.cs.x, g.gx, x0, x1);
         if (x0 > x1) continue;
         const int row = (b.z * g.gy + b.y) * g.gx;
         p = start[row + x0];
         e = start[row + x1 + 1];
-        b.ry = b.h.y + (float)(b.c.y - b.y) * g.cs.y;
+        b.ry = h.y + (float)(c.y - b.y) * g.cs.y;
         if (p < e) return true;
     }
 }
-
-// Calls test(p, box, id) for the members p of the box's rows and emit(k, id)
-// for those taken, k counting them in sorted order; returns their number.  A
-// group of L lanes shares the members (L at a time; a ballot keeps the order),
-// a single lane reads BATCH members ahead of their tests through
-// load(p, box): the particles of a warp are neighbours in the sorted order, so
-// their reads fall into the same few lines.
-template <int L, class Load, class Test, class Emit>
-__device__ __forceinline__ int takeMembers(RowBox& box, const int* __restrict__ start, const GridDev& g, bool live,
-                                           int lane, Load load, Test test, Emit emit)
+template <class Load, class Test>
+__device__ __forceinline__ int takeMembers(bool live, int4 c, float4 h, float reach, const int* __restrict__ start,
+                                           const GridDev& g, LaneWriter to, Load load, Test test)
 {
-    int k = 0, p = 0, e = 0;
-    if constexpr (L == 1) {
-        constexpr int BATCH = 4;
-        while (live && nextRow(box, start, g, p, e)) {
-            for (; p < e; p += BATCH) {
-                decltype(load(0)) m[BATCH];
+    constexpr int BATCH = 4;
+    const float wide = reach * 1.001f + 1.e-5f * (g.cs.x + g.cs.y + g.cs.z);
+    RowBox b;
+    int z0, p = 0, e = 0;
+    cellRange(c.y, h.y - wide, h.y + wide, g.cs.y, g.gy, b.y0, b.y1);
+    cellRange(c.z, h.z - wide, h.z + wide, g.cs.z, g.gz, z0, b.z1);
+    b.y = b.y1;  // one advance reaches the first row
+    b.z = z0 - 1;
+    b.gz2 = b.ry = b.rz = 0.f;
+    while (live && nextRow(b, c, h, wide, start, g, p, e)) {
+        for (; p < e; p += BATCH) {
+            decltype(load(0)) m[BATCH];
 #pragma unroll
-                for (int u = 0; u < BATCH; ++u) m[u] = load(min(p + u, e - 1));
+            for (int u = 0; u < BATCH; ++u) m[u] = load(min(p + u, e - 1));
 #pragma unroll
-                for (int u = 0; u < BATCH; ++u)
-                    if (p + u < e && test(m[u], box)) emit(k++, m[u]);
-            }
-        }
-    } else {
-        const int groupShift = (threadIdx.x & 31) & ~(L - 1);
-        const unsigned groupBits = (1u << L) - 1u, below = (1u << lane) - 1u;
-        bool more = live;
-        while (true) {
-            if (more && p >= e) more = nextRow(box, start, g, p, e);
-            if (!__any_sync(0xffffffffu, more)) break;
-            decltype(load(0)) m;
-            bool take = false;
-            if (more && p + lane < e) {
-                m = load(p + lane);
-                take = test(m, box);
-            }
-            const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
-            if (take) emit(k + __popc(mine & below), m);
-            k += __popc(mine);
-            p += L;
+            for (int u = 0; u < BATCH; ++u) to.add(test(m[u], b.ry, b.rz) && p + u < e, (unsigned)m[u].id);
+            to.flush();
         }
     }
-    return k;
+    return to.finish();
 }
 
-// Verlet candidates of the fluid lists, of one particle by a group of L lanes:
-// every fluid within the largest cut + fskin and every solid within 2 h +
-// fskin, in sorted order (all particles are inside the domain here: one
-// outside it sends the lists back to the walk).  P (cellPack): a fluid
-// partner's cell and offset are its filter record, one 16-byte read.
+// Verlet candidates of the fluid lists, of particle i by its L lanes (1 or
+// LIST_LANES; whole warps; live false past the last particle): every fluid within the
+// largest cut + fskin and every solid within 2 h + fskin, in sorted order (all
+// particles are inside the domain here: one outside it sends the lists back to
+// the walk).  P (cellPack): a fluid partner's cell and offset are its partner
+// record, one 16-byte read.
 //
 // What bounds it: instruction issue.  Walking the cells one by one (64 cells
 // of a box, 8 members each, every lane at its own cell) took 836M warp
-// instructions for 400k particles at one lane each, 1017 us; a row's members
-// are one loop: 303M, 438 us (48k particles, eight lanes: 158 to 120 us).
-template <int L, bool P>
-__device__ __forceinline__ void fluidCandidates(const DeviceState& d)
+// instructions for 400k particles, 1017 us; over rows of cells 305M, 421 us.
+template <int L, bool P, class Ring>
+__device__ __forceinline__ void fluidCandidates(const DeviceState& d, Ring& ring, int i, bool live)
 {
-    const int th = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((th & ~31) >= d.nf * L) return;
-    const int i = th / L, lane = th % L;
-    const bool live = i < d.nf;
+    using Writer = std::conditional_t<L == 1, LaneWriter, ListWriter>;
     const int n = d.nf;
     int4 ci = make_int4(0, 0, 0, 0);
     float4 hi = make_float4(0, 0, 0, 0);
@@ -229,7 +350,7 @@ __device__ __forceinline__ void fluidCandidates(const DeviceState& d)
         hi = d.fph[0][i];
     }
     const float skin = d.fskin;
-    const float4* __restrict__ rec = d.fcp;
+    const FluidRec* __restrict__ rec = d.frec[0];
     struct Member {
         float4 h;
         int x, id;
@@ -240,37 +361,32 @@ __device__ __forceinline__ void fluidCandidates(const DeviceState& d)
         return c * c * (1.f + 1.e-4f);
     };
     const float cut2U = cut2(hi.w);
-    const auto within = [&](const Member& m, const RowBox& b, float dc, float c2) {
-        const float rx = (hi.x - m.h.x) + dc * d.grid.cs.x, ry = b.ry - m.h.y, rz = b.rz - m.h.z;
+    const auto within = [&](const Member& m, float dc, float y, float z, float c2) {
+        const float rx = (hi.x - m.h.x) + dc * d.grid.cs.x, ry = y - m.h.y, rz = z - m.h.z;
         return rx * rx + ry * ry + rz * rz <= c2;
     };
-    RowBox boxF = rowsAround(live, ci, hi, 2.f * fmaxf(hi.w, d.fhmax) + skin, d.grid);
-    const int nff = takeMembers<L>(
-        boxF, d.fcellStart, d.grid, live, lane,
+    const int nff = takeMembers(
+        live, ci, hi, 2.f * fmaxf(hi.w, d.fhmax) + skin, d.fcellStart, d.grid, Writer(ring, d.fvc, i, n, d.kvf),
         [&](int p) {
             Member m;
             m.id = p;
             if constexpr (P) {
-                m.h = __ldg(rec + p);
-                m.x = (int)(__float_as_uint(m.h.w) & 2047u);
+                m.h = __ldg(&rec[p].pc);
+                m.x = (int)__float_as_uint(m.h.w);
             } else {
                 m.h = d.fph[0][p];
                 m.x = d.fcell[p].x;
             }
             return m;
         },
-        [&](const Member& m, const RowBox& b) {
+        [&](const Member& m, float y, float z) {
             // a packed cell's x + 2^23 as a float: no integer conversion per member
-            const float dc = P ? ((float)ci.x + 8388608.f) - __uint_as_float(0x4b000000u | (unsigned)m.x)
+            const float dc = P ? ((float)ci.x + 8388608.f) - __uint_as_float(0x4b000000u | ((unsigned)m.x & 2047u))
                                : (float)(ci.x - m.x);
-            return within(m, b, dc, P ? cut2U : cut2(fmaxf(hi.w, m.h.w))) && m.id != i;
-        },
-        [&](int k, const Member& m) {
-            if (k < d.kvf) d.fvc[(size_t)k * n + i] = (unsigned)m.id;
+            return within(m, dc, y, z, P ? cut2U : cut2(fmaxf(hi.w, m.h.w))) && m.id != i;
         });
-    RowBox boxS = rowsAround(live, ci, hi, 2.f * hi.w + skin, d.grid);
-    const int nfs = takeMembers<L>(
-        boxS, d.scellStart, d.grid, live, lane,
+    const int nfs = takeMembers(
+        live, ci, hi, 2.f * hi.w + skin, d.scellStart, d.grid, Writer(ring, (unsigned*)d.fvsc, i, n, d.kvs),
         [&](int p) {
             Member m;
             m.id = d.ssorted[p];
@@ -278,11 +394,8 @@ __device__ __forceinline__ void fluidCandidates(const DeviceState& d)
             m.x = d.scell[m.id].x;
             return m;
         },
-        [&](const Member& m, const RowBox& b) { return within(m, b, (float)(ci.x - m.x), cut2U); },
-        [&](int k, const Member& m) {
-            if (k < d.kvs) d.fvsc[(size_t)k * n + i] = m.id;
-        });
-    if (!live || lane != 0) return;
+        [&](const Member& m, float y, float z) { return within(m, (float)(ci.x - m.x), y, z, cut2U); });
+    if (!live || (threadIdx.x & (L - 1)) != 0) return;
     d.fvcn[i] = nff;
     d.fvsn[i] = nfs;
     d.fvref[i] = make_float4((float)ci.x * d.grid.cs.x + hi.x, (float)ci.y * d.grid.cs.y + hi.y,
@@ -296,13 +409,10 @@ __device__ __forceinline__ void fluidCandidates(const DeviceState& d)
 
 // The lists from the reference's 27-cell walk (every fluid step once a particle
 // has left the domain, or at initialisation).
-template <int L>
-__device__ __forceinline__ void fluidWalk(const DeviceState& d)
+__device__ __forceinline__ void fluidWalk(const DeviceState& d, int i, bool live)
 {
-    const int th = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((th & ~31) >= d.nf * L) return;
-    const int i = th / L, lane = th % L;
-    const bool live = i < d.nf;
+    constexpr int L = LIST_LANES;
+    const int lane = threadIdx.x & (L - 1);
     const int groupShift = (threadIdx.x & 31) & ~(L - 1);
     const unsigned groupBits = L == 32 ? 0xffffffffu : ((1u << L) - 1u);
     const unsigned below = (1u << lane) - 1u;
@@ -352,7 +462,7 @@ __device__ __forceinline__ void fluidWalk(const DeviceState& d)
             const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
             if (take) {
                 const int slot = nff + __popc(mine & below);
-                if (slot < d.kff) d.ff[(size_t)slot * n + i] = ffEntry(j, w.t, w.regular && centred);
+                if (slot < d.kff) d.ff[listAt(slot, i, n)] = ffEntry(j, w.t, w.regular && centred);
             }
             nff += __popc(mine);
             if (!__any_sync(0xffffffffu, has)) break;
@@ -380,7 +490,7 @@ __device__ __forceinline__ void fluidWalk(const DeviceState& d)
             const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
             if (take) {
                 const int slot = nfs + __popc(mine & below);
-                if (slot < d.kfs) d.fs[(size_t)slot * n + i] = fsEntry(a, w.t);
+                if (slot < d.kfs) d.fs[listAt(slot, i, n)] = fsEntry(a, w.t);
             }
             nfs += __popc(mine);
             if (!__any_sync(0xffffffffu, has)) break;
@@ -408,141 +518,247 @@ __device__ __forceinline__ int walkPosition(int4 ci, int4 cj)
 // here, so those are the cells the reference walks).  The rebuild flag is
 // cleared: the last position update of the step raises it again.
 //
-// P (cellPack): a candidate's cell and position offset come from its filter
-// record (one 16-byte read); the smoothing length is every particle's.
-#ifndef DEMSPH_FILTER_UNROLL
-#define DEMSPH_FILTER_UNROLL 4  // rounds of candidate reads in flight with one lane per particle
-#endif
-template <int L, bool P>
-__device__ __forceinline__ void fluidFilter(const DeviceState& d)
+// P (cellPack): a candidate's cell and offset are its partner record (one
+// 16-byte read), the smoothing length is every particle's, and the test runs
+// on the packed cells (packedWalk): no unpacking, no integer conversions.
+//
+// What bounds it: latency of the candidate stream and the records, then the
+// list's bytes.  With one column per entry, every entry stored was a sector
+// write of its own: of 199 us for 400k particles, 120 were those stores, 60 the
+// candidate ids, 20 the records; in sectors it takes 140 us (1.0M: 350 to 316).
+
+// Packed cells (x | y << 11 | z << 22) and their place in the 27-cell walk:
+// with one added to each field (PACK_ONES), the difference of two neighbouring
+// cells has fields dx + 1, dy + 1, dz + 1 in 0..2; any other difference has a
+// field of 3 or bits outside the fields (a borrow sets all of them).
+constexpr unsigned PACK_ONES = 1u | 1u << 11 | 1u << 22;
+__device__ __forceinline__ bool packedNeighbour(unsigned diff)
 {
-    // one lane per particle walks a long candidate list: 4 rounds of reads in
-    // flight; with 4 or 8 lanes a round already covers many candidates
-    constexpr int FILTER_UNROLL = L == 1 ? DEMSPH_FILTER_UNROLL : (L == 2 ? 2 : 1);
-    stepKernelBegin();
-    const int th = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((th & ~31) >= d.nf * L || *d.status || *d.fslowMode || *d.slowMode) return;
-    if (th == 0) *(volatile int*)d.frebuild = 0;
-    const int i = th / L, lane = th % L;
-    const bool live = i < d.nf;
-    const int groupShift = (threadIdx.x & 31) & ~(L - 1);
-    const unsigned groupBits = L == 32 ? 0xffffffffu : ((1u << L) - 1u);
-    const unsigned below = (1u << lane) - 1u;
-    const int n = d.nf;
-    int4 ci = make_int4(0, 0, 0, 0);
-    float4 hi = make_float4(0, 0, 0, 0), li = hi;
-    dfl hI = df_make(0.f), cutS = hI;
-    int nc = 0, ns = 0;
-    if (live) {
-        ci = d.fcell[i];
-        hi = d.fph[0][i];
-        li = d.fpl[0][i];
-        hI = df_make(hi.w, li.w);
-        cutS = df_add(hI, hI);
-        nc = min(d.fvcn[i], d.kvf);
-        ns = min(d.fvsn[i], d.kvs);
-    }
-    // candidates are taken FILTER_UNROLL rounds of L at a time: the rounds'
-    // reads are issued together, their results compacted round by round (the
-    // list order of one round per iteration)
-    int nff = 0;
-    // the next rounds' candidate ids are read while this round's partners are
-    // gathered and tested
-    int jn[FILTER_UNROLL];
+    return ((diff & ~(3u * PACK_ONES)) | (diff & (diff >> 1) & PACK_ONES)) == 0u;
+}
+// (dx + 1) + 3 (dy + 1) + 9 (dz + 1): the product puts the three terms at bit
+// 22, the smaller cross terms below it (they never carry) and the others past
+// bit 31.
+__device__ __forceinline__ unsigned packedWalk(unsigned diff) { return (diff * ((1u << 22) + (3u << 11) + 9u)) >> 22; }
+
+#ifndef DEMSPH_FILTER_UNROLL
+#define DEMSPH_FILTER_UNROLL 2  // sectors of candidates in flight
+#endif
+
+// The fluid part of the filter from the partner records; tab: the offsets of
+// the 27 walk cells, one array per axis.  Returns the number of partners.
+__device__ __forceinline__ int filterRecords(const DeviceState& d, const float (*tab)[32], ListWriter to, int i, int lane,
+                                             int nc, int4 ci, float4 hi, float4 li)
+{
+    constexpr int U = DEMSPH_FILTER_UNROLL;
+    const FluidRec* __restrict__ rec = d.frec[0];
+    const size_t stride = (size_t)d.nf * 8;
+    const unsigned* cand = d.fvc + (size_t)i * 8 + lane;
+    const unsigned mine0 = __float_as_uint(packCell(ci)) - PACK_ONES;
+    const float c = 2.f * hi.w, c2 = c * c, c2lo = c2 * (1.f - 1.e-5f), c2hi = c2 * (1.f + 1.e-5f);
+    int jn[U];
 #pragma unroll
-    for (int u = 0; u < FILTER_UNROLL; ++u) {
-        const int k = u * L + lane;
-        jn[u] = k < nc ? (int)d.fvc[(size_t)k * n + i] : -1;
-    }
-    for (int base = 0; __any_sync(0xffffffffu, base < nc); base += FILTER_UNROLL * L) {
-        int j[FILTER_UNROLL];
-        int4 cj[FILTER_UNROLL];
-        float4 hj[FILTER_UNROLL];
+    for (int u = 0; u < U; ++u, cand += stride) jn[u] = u * LIST_LANES + lane < nc ? (int)__ldcs(cand) : i;
+    for (int k = lane; __any_sync(0xffffffffu, k - lane < nc); k += U * LIST_LANES) {
+        int j[U];
+        float4 r[U];
 #pragma unroll
-        for (int u = 0; u < FILTER_UNROLL; ++u) {
+        for (int u = 0; u < U; ++u) {
             j[u] = jn[u];
-            const int k = base + (FILTER_UNROLL + u) * L + lane;
-            jn[u] = k < nc ? (int)d.fvc[(size_t)k * n + i] : -1;
+            r[u] = __ldg(&rec[j[u]].pc);
         }
 #pragma unroll
-        for (int u = 0; u < FILTER_UNROLL; ++u) {
-            if (j[u] >= 0) {
-                if constexpr (P) {
-                    const float4 r = __ldg(d.fcp + j[u]);
-                    cj[u] = unpackCell(r.w);
-                    hj[u] = make_float4(r.x, r.y, r.z, hi.w);
-                } else {
-                    cj[u] = d.fcell[j[u]];
-                    hj[u] = d.fph[0][j[u]];
-                }
+        for (int u = 0; u < U; ++u, cand += stride) jn[u] = k + (U + u) * LIST_LANES < nc ? (int)__ldcs(cand) : i;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned diff = __float_as_uint(r[u].w) - mine0;
+            const unsigned t = packedWalk(diff) & 31u;  // some word of the table where it is no neighbour
+            const float x = (hi.x - r[u].x) - tab[0][t], y = (hi.y - r[u].y) - tab[1][t], z = (hi.z - r[u].z) - tab[2][t];
+            const float d2 = x * x + y * y + z * z;
+            bool take = d2 <= c2hi && packedNeighbour(diff) && k + u * LIST_LANES < nc;
+            if (take && d2 >= c2lo) {  // within the rounding of the cut: decided in double-float
+                const dfl hI = df_make(hi.w, li.w);
+                take = withinCut(ci, hi, li, unpackCell(r[u].w), r[u], d.fpl[0], j[u], df_add(hI, hI), d.grid);
             }
+            to.add(take, ffEntry(j[u], (int)t, true));
+        }
+    }
+    return to.finish();
+}
+
+// The same from cells and positions of their own (fluids whose parameters
+// differ, grids too large for packed cells).
+__device__ __forceinline__ int filterCells(const DeviceState& d, ListWriter to, int i, int lane, int nc, int4 ci, float4 hi,
+                                           float4 li)
+{
+    const dfl hI = df_make(hi.w, li.w);
+    const size_t stride = (size_t)d.nf * 8;
+    const unsigned* cand = d.fvc + (size_t)i * 8 + lane;
+    int jn = lane < nc ? (int)__ldcs(cand) : i;
+    for (int k = lane; __any_sync(0xffffffffu, k - lane < nc); k += LIST_LANES) {
+        const int j = jn;
+        const int4 cj = d.fcell[j];
+        const float4 hj = d.fph[0][j];
+        cand += stride;
+        jn = k + LIST_LANES < nc ? (int)__ldcs(cand) : i;
+        const int t = walkPosition(ci, cj);
+        const float3 r = relF(ci, hi, cj, hj, d.grid);
+        const float c = 2.f * fmaxf(hi.w, hj.w);
+        const float d2 = dot3(r, r), c2 = c * c;
+        bool take = k < nc && t >= 0 && d2 <= c2 * (1.f + 1.e-5f);
+        if (take && d2 >= c2 * (1.f - 1.e-5f)) {
+            const dfl rad = dfMax(hI, df_make(hj.w, d.fpl[0][j].w));
+            take = withinCut(ci, hi, li, cj, hj, d.fpl[0], j, df_add(rad, rad), d.grid);
+        }
+        to.add(take, ffEntry(j, t & 31, true));
+    }
+    return to.finish();
+}
+
+// The reference's test for solid a of a fluid particle; t: the walk position of
+// its cell.
+__device__ __forceinline__ bool solidPartnerOf(const DeviceState& d, int4 ci, float4 hi, float4 li, int a, int4 ca,
+                                               float4 ha, int& t)
+{
+    t = walkPosition(ci, ca);
+    const float3 r = relF(ci, hi, ca, ha, d.grid);
+    const float d2 = dot3(r, r), c2 = 4.f * hi.w * hi.w;
+    if (t < 0 || d2 > c2 * (1.f + 1.e-5f)) return false;
+    if (d2 < c2 * (1.f - 1.e-5f)) return true;
+    const dfl hI = df_make(hi.w, li.w);
+    return withinCut(ci, hi, li, ca, ha, d.spl, a, df_add(hI, hI), d.grid);
+}
+
+// filterRecords by one lane per particle: a sector of candidates in one load,
+// four records in flight.
+__device__ __forceinline__ int filterRecordsLane(const DeviceState& d, const float (*tab)[32], LaneWriter to, int i, int nc,
+                                                 int4 ci, float4 hi, float4 li)
+{
+    constexpr int B = 4;
+    const FluidRec* __restrict__ rec = d.frec[0];
+    const size_t stride = (size_t)d.nf * 8;
+    const uint4* cand = reinterpret_cast<const uint4*>(d.fvc + (size_t)i * 8);
+    const unsigned mine0 = __float_as_uint(packCell(ci)) - PACK_ONES;
+    const float c = 2.f * hi.w, c2 = c * c, c2lo = c2 * (1.f - 1.e-5f), c2hi = c2 * (1.f + 1.e-5f);
+    uint4 a = make_uint4(i, i, i, i);
+    if (nc > 0) a = __ldcs(cand);
+    for (int k = 0; k < nc; k += B) {
+        const unsigned j[B] = {a.x, k + 1 < nc ? a.y : (unsigned)i, k + 2 < nc ? a.z : (unsigned)i,
+                               k + 3 < nc ? a.w : (unsigned)i};
+        float4 r[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) r[u] = __ldg(&rec[j[u]].pc);
+        // candidates k + 4 .. k + 7: the sector's other half, or the next sector
+        cand = (k & 4) ? reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned*>(cand) - 4 + stride) : cand + 1;
+        if (k + B < nc) a = __ldcs(cand);
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const unsigned diff = __float_as_uint(r[u].w) - mine0;
+            const unsigned t = packedWalk(diff) & 31u;
+            const float x = (hi.x - r[u].x) - tab[0][t], y = (hi.y - r[u].y) - tab[1][t], z = (hi.z - r[u].z) - tab[2][t];
+            const float d2 = x * x + y * y + z * z;
+            bool take = d2 <= c2hi && packedNeighbour(diff) && k + u < nc;
+            if (take && d2 >= c2lo) {
+                const dfl hI = df_make(hi.w, li.w);
+                take = withinCut(ci, hi, li, unpackCell(r[u].w), r[u], d.fpl[0], (int)j[u], df_add(hI, hI), d.grid);
+            }
+            to.add(take, ffEntry((int)j[u], (int)t, true));
+        }
+        to.flush();
+    }
+    return to.finish();
+}
+
+// One lane per particle (packed cells only).
+__global__ void __launch_bounds__(T) kFluidFilterLane(DeviceState d)
+{
+    stepKernelBegin();
+    __shared__ LaneRing ring;
+    __shared__ float tab[3][32];
+    if (threadIdx.x < 27) {
+        tab[0][threadIdx.x] = (float)((int)(threadIdx.x % 3) - 1) * d.grid.cs.x;
+        tab[1][threadIdx.x] = (float)((int)(threadIdx.x / 3 % 3) - 1) * d.grid.cs.y;
+        tab[2][threadIdx.x] = (float)((int)(threadIdx.x / 9) - 1) * d.grid.cs.z;
+    }
+    __syncthreads();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.nf || *d.status || *d.fslowMode || *d.slowMode) return;
+    if (i == 0) *(volatile int*)d.frebuild = 0;
+    const int n = d.nf;
+    const int4 ci = d.fcell[i];
+    const float4 hi = d.fph[0][i], li = d.fpl[0][i];
+    const int nc = min(d.fvcn[i], d.kvf), ns = min(d.fvsn[i], d.kvs);
+    const int nff = filterRecordsLane(d, tab, LaneWriter(ring, d.ff, i, n, d.kff), i, nc, ci, hi, li);
+    // few particles have solid candidates, but those many (a wall): four in flight
+    LaneWriter to(ring, (unsigned*)d.fs, i, n, d.kfs);
+    for (int k = 0; k < ns; k += 4) {
+        const int4 v = __ldcs(reinterpret_cast<const int4*>(d.fvsc + listAt(k, i, n)));
+        const int a[4] = {v.x, k + 1 < ns ? v.y : v.x, k + 2 < ns ? v.z : v.x, k + 3 < ns ? v.w : v.x};
+        int4 ca[4];
+        float4 ha[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            ca[u] = d.scell[a[u]];
+            ha[u] = d.sph[a[u]];
         }
 #pragma unroll
-        for (int u = 0; u < FILTER_UNROLL; ++u) {
-            bool take = false;
-            int t = -1;
-            if (j[u] >= 0) {
-                t = walkPosition(ci, cj[u]);
-                if (t >= 0) {
-                    const float3 r = relF(ci, hi, cj[u], hj[u], d.grid);
-                    const float c = 2.f * fmaxf(hi.w, hj[u].w);
-                    const float d2 = dot3(r, r), c2 = c * c;
-                    if (d2 < c2 * (1.f - 1.e-5f)) {
-                        take = true;
-                    } else if (d2 <= c2 * (1.f + 1.e-5f)) {
-                        const dfl hJ = P ? hI : df_make(hj[u].w, d.fpl[0][j[u]].w);
-                        const dfl rad = dfMax(hI, hJ);
-                        take = withinCut(ci, hi, li, cj[u], hj[u], d.fpl[0], j[u], df_add(rad, rad), d.grid);
-                    }
-                }
-            }
-            const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
-            if (take) {
-                const int slot = nff + __popc(mine & below);
-                if (slot < d.kff) d.ff[(size_t)slot * n + i] = ffEntry(j[u], t, true);
-            }
-            nff += __popc(mine);
+        for (int u = 0; u < 4; ++u) {
+            int t;
+            const bool take = solidPartnerOf(d, ci, hi, li, a[u], ca[u], ha[u], t) && k + u < ns;
+            to.add(take, (unsigned)fsEntry(a[u], t));
         }
+        to.flush();
     }
-    int nfs = 0;
-    for (int base = 0; __any_sync(0xffffffffu, base < ns); base += L) {
-        const int k = base + lane;
-        bool take = false;
-        int a = 0, t = -1;
-        if (k < ns) {
-            a = d.fvsc[(size_t)k * n + i];
-            const int4 ca = d.scell[a];
-            t = walkPosition(ci, ca);
-            if (t >= 0) {
-                const float4 ha = d.sph[a];
-                const float3 r = relF(ci, hi, ca, ha, d.grid);
-                const float d2 = dot3(r, r), c2 = 4.f * hi.w * hi.w;
-                if (d2 < c2 * (1.f - 1.e-5f)) take = true;
-                else if (d2 <= c2 * (1.f + 1.e-5f)) take = withinCut(ci, hi, li, ca, ha, d.spl, a, cutS, d.grid);
-            }
-        }
-        const unsigned mine = (__ballot_sync(0xffffffffu, take) >> groupShift) & groupBits;
-        if (take) {
-            const int slot = nfs + __popc(mine & below);
-            if (slot < d.kfs) d.fs[(size_t)slot * n + i] = fsEntry(a, t);
-        }
-        nfs += __popc(mine);
-    }
-    if (!live || lane != 0) return;
+    const int nfs = to.finish();
     d.ffc[i] = nff;
     d.fsc[i] = nfs;
     if (nff > d.kff) atomicOr(d.status, ST_FF_OVERFLOW);
     if (nfs > d.kfs) atomicOr(d.status, ST_FS_OVERFLOW);
 }
-template <int L>
+
+// One particle by its LIST_LANES lanes.
+template <bool P>
 __global__ void __launch_bounds__(T) kFluidFilter(DeviceState d)
 {
-    fluidFilter<L, false>(d);
-}
-template <int L>
-__global__ void __launch_bounds__(T) kFluidFilterPacked(DeviceState d)
-{
-    fluidFilter<L, true>(d);
+    stepKernelBegin();
+    __shared__ ListRing ring;
+    __shared__ float tab[3][32];
+    if (P) {
+        if (threadIdx.x < 27) {
+            tab[0][threadIdx.x] = (float)((int)(threadIdx.x % 3) - 1) * d.grid.cs.x;
+            tab[1][threadIdx.x] = (float)((int)(threadIdx.x / 3 % 3) - 1) * d.grid.cs.y;
+            tab[2][threadIdx.x] = (float)((int)(threadIdx.x / 9) - 1) * d.grid.cs.z;
+        }
+        __syncthreads();
+    }
+    const long long th = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(th / LIST_LANES), lane = threadIdx.x & (LIST_LANES - 1);
+    if ((th & ~31LL) >= (long long)d.nf * LIST_LANES || *d.status || *d.fslowMode || *d.slowMode) return;
+    if (th == 0) *(volatile int*)d.frebuild = 0;
+    const bool live = i < d.nf;
+    const int n = d.nf, self = live ? i : 0;
+    const int4 ci = d.fcell[self];
+    const float4 hi = d.fph[0][self], li = d.fpl[0][self];
+    const int nc = live ? min(d.fvcn[i], d.kvf) : 0, ns = live ? min(d.fvsn[i], d.kvs) : 0;
+    int nff;
+    if constexpr (P) nff = filterRecords(d, tab, ListWriter(ring, d.ff, self, n, d.kff), self, lane, nc, ci, hi, li);
+    else nff = filterCells(d, ListWriter(ring, d.ff, self, n, d.kff), self, lane, nc, ci, hi, li);
+    ListWriter to(ring, (unsigned*)d.fs, self, n, d.kfs);
+    for (int k = lane; __any_sync(0xffffffffu, k - lane < ns); k += LIST_LANES) {
+        bool take = false;
+        int a = 0, t = 0;
+        if (k < ns) {
+            a = d.fvsc[listAt(k, i, n)];
+            take = solidPartnerOf(d, ci, hi, li, a, d.scell[a], d.sph[a], t);
+        }
+        to.add(take, (unsigned)fsEntry(a, t));
+    }
+    const int nfs = to.finish();
+    if (!live || lane != 0) return;
+    d.ffc[i] = nff;
+    d.fsc[i] = nfs;
+    if (nff > d.kff) atomicOr(d.status, ST_FF_OVERFLOW);
+    if (nfs > d.kfs) atomicOr(d.status, ST_FS_OVERFLOW);
 }
 
 // ---- fluid partners of each massive solid (coupling force) ----
@@ -553,7 +769,7 @@ __global__ void kCoupCount(DeviceState d)
     if (i >= d.nf || *d.status) return;
     const int m = min(d.fsc[i], d.kfs);
     for (int k = 0; k < m; ++k) {
-        const int a = fsPartner(d.fs[(size_t)k * d.nf + i]);
+        const int a = fsPartner(d.fs[listAt(k, i, d.nf)]);
         if (d.sflags[a].w & F_HASMASS) atomicAdd(&d.coupCount[a], 1);
     }
 }
@@ -568,7 +784,7 @@ __global__ void kCoupFill(DeviceState d)
     }
     const int m = min(d.fsc[i], d.kfs);
     for (int k = 0; k < m; ++k) {
-        const int a = fsPartner(d.fs[(size_t)k * d.nf + i]);
+        const int a = fsPartner(d.fs[listAt(k, i, d.nf)]);
         if (d.sflags[a].w & F_HASMASS) d.coupList[d.coupStart[a] + atomicAdd(&d.coupCount[a], 1)] = i;
     }
 }
@@ -903,14 +1119,19 @@ template <int L, bool P>
 __global__ void __launch_bounds__(T) kFluidWalk(DeviceState d, RunIf lists, RunIf cands)
 {
     stepKernelBegin();
+    __shared__ std::conditional_t<L == 1, LaneRing, ListRing> ring;
     if (*d.status) return;
-    if (lists.active()) {
-        fluidWalk<L>(d);
-        return;
+    const bool walk = lists.active();
+    if (!walk && !cands.active()) return;
+    // whole warps: a warp takes 32 / lanes particles at a time
+    const int lanes = walk ? LIST_LANES : L;
+    const long long stride = (long long)gridDim.x * blockDim.x, total = (long long)d.nf * lanes;
+    for (long long th = (long long)blockIdx.x * blockDim.x + threadIdx.x; (th & ~31LL) < total; th += stride) {
+        const int i = (int)(th / lanes);
+        if (walk) fluidWalk(d, i, i < d.nf);
+        else fluidCandidates<L, P>(d, ring, i, i < d.nf);
     }
-    if (!cands.active()) return;
-    fluidCandidates<L, P>(d);
-    if (*d.status) return;
+    if (walk || *d.status) return;
     const auto ref = [&](int a) {
         const int4 c = d.scell[a];
         const float4 h = d.sph[a];
@@ -926,6 +1147,16 @@ __global__ void __launch_bounds__(T) kFluidWalk(DeviceState d, RunIf lists, RunI
         }
 }
 
+// One lane per particle in the list kernels of large scenes: fewer instructions
+// (no ballots), but eight times fewer threads.  Filter, eight lanes against
+// one: 12k particles 15 / 37 us, 48k 29 / 41, 80k 39 / 45, 120k 56 / 50, 400k
+// 166 / 140, 1.0M 397 / 316; the rebuild, averaged over the steps of a flowing
+// 400k dam break, 107 / 60.
+#ifndef DEMSPH_LANE_LISTS
+#define DEMSPH_LANE_LISTS 100000
+#endif
+static bool laneLists(int nf) { return nf >= DEMSPH_LANE_LISTS; }
+
 void launchFluidWalk(const DeviceState& d, bool walk, cudaStream_t s)
 {
     if (d.nf <= 0) return;
@@ -938,15 +1169,19 @@ void launchFluidWalk(const DeviceState& d, bool walk, cudaStream_t s)
     cands.a = d.frebuild;
     cands.unless = d.fslowMode;
     cands.unless2 = d.slowMode;
-    if (d.cellPack) LAUNCH_LANES_U(kFluidWalk, true, d.lanes, d.nf, T, s, d, lists, cands);
-    else LAUNCH_LANES_U(kFluidWalk, false, d.lanes, d.nf, T, s, d, lists, cands);
+    // the launch is idle on most steps: no more blocks than the GPU holds at
+    // once (eight per SM by registers)
+    const bool one = laneLists(d.nf);
+    const unsigned blocks = (unsigned)std::min(152LL * 8, ((long long)d.nf * (one ? 1 : LIST_LANES) + T - 1) / T);
+    if (one) launchStep(d.cellPack ? kFluidWalk<1, true> : kFluidWalk<1, false>, blocks, T, s, d, lists, cands);
+    else launchStep(d.cellPack ? kFluidWalk<LIST_LANES, true> : kFluidWalk<LIST_LANES, false>, blocks, T, s, d, lists, cands);
 }
 
 void launchFluidFilter(const DeviceState& d, cudaStream_t s)
 {
     if (d.nf <= 0) return;
-    if (d.cellPack) LAUNCH_LANES(kFluidFilterPacked, d.lanes, d.nf, T, s, d);
-    else LAUNCH_LANES(kFluidFilter, d.lanes, d.nf, T, s, d);
+    if (d.cellPack && laneLists(d.nf)) launchStep(kFluidFilterLane, blocksFor(d.nf, T), T, s, d);
+    else launchStep(d.cellPack ? kFluidFilter<true> : kFluidFilter<false>, blocksFor((long long)d.nf * LIST_LANES, T), T, s, d);
 }
 
 void launchCouplingLists(const DeviceState& d, cudaStream_t s)

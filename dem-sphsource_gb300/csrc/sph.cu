@@ -31,56 +31,44 @@ namespace {
 constexpr int T = 128;
 using namespace sph;
 
-#ifndef DEMSPH_WALK_TABLE
-#define DEMSPH_WALK_TABLE 1  // 1: the 27 cell offsets come from a table in shared memory
-#endif
-
-// Offset of walk cell `code` (dx, dy, dz in -1..1, code = (dz+1) 9 + (dy+1) 3 + dx+1)
-// times the cell size.
-__device__ __forceinline__ float4 walkOffsetOf(unsigned code, float3 cs)
+// The offsets of the 27 walk cells (code = (dz+1) 9 + (dy+1) 3 + dx+1), one
+// array per axis in a block's shared memory (filled before the block's first
+// early return): three 4-byte reads of 27 words each take a wavefront of the
+// L1 apiece, one 16-byte read took four to ten.
+struct WalkTable {
+    float o[3][32];
+};
+__device__ __forceinline__ void fillWalkTable(WalkTable& tab, float3 cs)
 {
-    const int dx = (int)(code % 3u) - 1, dy = (int)((code / 3u) % 3u) - 1, dz = (int)(code / 9u) - 1;
-    return make_float4((float)dx * cs.x, (float)dy * cs.y, (float)dz * cs.z, 0.f);
-}
-
-// The table of the 27 offsets in a block's shared memory (filled before the
-// block's first early return).
-__device__ __forceinline__ void fillWalkTable(float4* tab, float3 cs)
-{
-    if (DEMSPH_WALK_TABLE) {
-        if (threadIdx.x < 27) tab[threadIdx.x] = walkOffsetOf(threadIdx.x, cs);
-        __syncthreads();
+    const int code = threadIdx.x;
+    if (code < 27) {
+        tab.o[0][code] = (float)(code % 3 - 1) * cs.x;
+        tab.o[1][code] = (float)(code / 3 % 3 - 1) * cs.y;
+        tab.o[2][code] = (float)(code / 9 - 1) * cs.z;
     }
+    __syncthreads();
 }
 
-// Relative position of fluid partner entry e of slot i (tab: the offsets'
-// table; the products are exact, so the table changes no bit).
-__device__ __forceinline__ float3 fluidRel(const DeviceState& d, const float4* tab, int4 ci, float4 pi, unsigned e,
+// Relative position of fluid partner entry e of slot i (the products of the
+// table are exact, so it changes no bit).
+__device__ __forceinline__ float3 fluidRel(const DeviceState& d, const WalkTable& tab, int4 ci, float4 pi, unsigned e,
                                            int j, float4 pj)
 {
     if (ffRegular(e)) {
-        const float4 o = DEMSPH_WALK_TABLE ? tab[entryWalk(e)] : walkOffsetOf((unsigned)entryWalk(e), d.grid.cs);
-        return make_float3((pi.x - pj.x) - o.x, (pi.y - pj.y) - o.y, (pi.z - pj.z) - o.z);
+        const int t = entryWalk(e);
+        return make_float3((pi.x - pj.x) - tab.o[0][t], (pi.y - pj.y) - tab.o[1][t], (pi.z - pj.z) - tab.o[2][t]);
     }
     return relF(ci, pi, d.fcell[j], pj, d.grid);
 }
 
 // ---- batched partner loops ----
-// Entries per lane read before any of their partners is used: a lane reads
-// B list entries, then the B partners' state, then adds the B pair terms in
-// list order.  B gathers per lane are in flight instead of one (the loop is
-// bound by the latency of the list stream and the dependent gathers, not by
-// bandwidth), and every sum is that of the one-by-one loop, bit for bit.
-// Depths and block counts measured on GB300 (ms per fluid period of the 1.0M
-// coupled dam break, one lane per particle; depth 1 = the one-by-one loop):
-// depth 1 with 12 continuity blocks 3.889, depth 2 with 8 continuity and 6
-// momentum blocks 3.829, depth 4 3.89-4.15 (continuity spills at 8 blocks),
-// depth 8 4.43.  The 48k dam break (eight lanes) is flat within 3 %.
+// Partners whose state is gathered before any of them is used: B gathers per
+// lane are in flight instead of one.  Depths and block counts measured on GB300
+// (ms per fluid period of the 1.0M coupled dam break, one lane per particle):
+// the one-by-one loop 3.889, depth 2 with 8 continuity and 6 momentum blocks
+// 3.829, depth 4 3.89-4.15 (spills), depth 8 4.43.
 #ifndef DEMSPH_PAIR_BATCH
-#define DEMSPH_PAIR_BATCH 2       // entries per batch, one or two lanes per particle
-#endif
-#ifndef DEMSPH_PAIR_BATCH_WIDE
-#define DEMSPH_PAIR_BATCH_WIDE 2  // entries per batch, four or more lanes per particle
+#define DEMSPH_PAIR_BATCH 2
 #endif
 #ifndef DEMSPH_CONTINUITY_BLOCKS
 #define DEMSPH_CONTINUITY_BLOCKS 8  // resident blocks of T per SM the registers allow
@@ -88,73 +76,153 @@ __device__ __forceinline__ float3 fluidRel(const DeviceState& d, const float4* t
 #ifndef DEMSPH_MOMENTUM_BLOCKS
 #define DEMSPH_MOMENTUM_BLOCKS 6
 #endif
-#ifndef DEMSPH_PAIR_AHEAD
-#define DEMSPH_PAIR_AHEAD 1  // 1: the next batch's entries are read while this batch computes
-#endif
-#ifndef DEMSPH_PAIR_L2_AHEAD
-#define DEMSPH_PAIR_L2_AHEAD 0  // > 0: the list line that many batches ahead is prefetched into L2
-#endif
-template <int L>
-constexpr int batchDepth() { return L >= 4 ? DEMSPH_PAIR_BATCH_WIDE : DEMSPH_PAIR_BATCH; }
+constexpr int BATCH = DEMSPH_PAIR_BATCH;
 
-template <int L, int B, class Gather, class Term>
-__device__ __forceinline__ void forFluidPartners(const unsigned* __restrict__ ff, int n, int i, int lane, int m,
-                                                 Gather gather, Term term)
+// E consecutive list entries in one load (streamed: the list is read once a pass).
+template <int E>
+__device__ __forceinline__ void loadEntries(const unsigned* __restrict__ p, unsigned* e)
 {
-    const size_t stride = (size_t)L * n;  // from entry k of slot i to entry k + L
-    const unsigned* p = ff + (size_t)lane * n + i;
-    unsigned next[B];
-    if (DEMSPH_PAIR_AHEAD) {
-#pragma unroll
-        for (int u = 0; u < B; ++u) next[u] = lane + u * L < m ? __ldcs(p + u * stride) : 0u;
-    }
-    for (int k0 = lane; k0 < m; k0 += B * L) {
-        unsigned e[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u) e[u] = DEMSPH_PAIR_AHEAD ? next[u] : (k0 + u * L < m ? __ldcs(p + u * stride) : 0u);
-        p += B * stride;
-        if (DEMSPH_PAIR_AHEAD) {
-#pragma unroll
-            for (int u = 0; u < B; ++u) next[u] = k0 + (B + u) * L < m ? __ldcs(p + u * stride) : 0u;
-        }
-        if (DEMSPH_PAIR_L2_AHEAD > 0 && k0 + DEMSPH_PAIR_L2_AHEAD * B * L < m)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (size_t)(DEMSPH_PAIR_L2_AHEAD - 1) * B * stride));
-        decltype(gather(0u)) g[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (k0 + u * L < m) g[u] = gather(e[u]);
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (k0 + u * L < m) term(e[u], g[u]);
+    if constexpr (E == 8) {
+        asm("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(e[0]), "=r"(e[1]), "=r"(e[2]), "=r"(e[3]), "=r"(e[4]), "=r"(e[5]), "=r"(e[6]), "=r"(e[7])
+            : "l"(p));
+    } else if constexpr (E == 4) {
+        const uint4 v = __ldcs(reinterpret_cast<const uint4*>(p));
+        e[0] = v.x, e[1] = v.y, e[2] = v.z, e[3] = v.w;
+    } else if constexpr (E == 2) {
+        const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p));
+        e[0] = v.x, e[1] = v.y;
+    } else {
+        e[0] = __ldcs(p);
     }
 }
 
-// A fluid partner's state read by the continuity and momentum terms (the
-// buffers a pass reads are not written by it: read-only loads).  Uniform
-// fluids (U) read the position and density as one partner record (pd, the
-// pass's fpd); par only for scenes whose fluids differ (U false).
-template <bool U>
+// The loop over the m entries of particle i's list by one of its L lanes.  A
+// sector of eight entries (listAt) is shared by the lanes, 8 / L consecutive
+// entries each in one load; the next sector is read while this one is used.
+// gather(e) reads a partner's state, use(e, state, ok) takes B of them at a time
+// without a branch on the entry (ok false: past the list's end, where the entry
+// is the particle itself), so that the B terms' chains interleave.
+template <int L, int B, class Gather, class Use>
+__device__ __forceinline__ void forFluidPartners(const unsigned* __restrict__ ff, int n, int i, int lane, int m,
+                                                 Gather gather, Use use)
+{
+    constexpr int E = 8 / L, S = E < B ? B / E : 1, N = E * S;  // entries of a lane per sector, sectors and entries per round
+    const size_t stride = (size_t)n * 8;
+    const unsigned* p = ff + (size_t)i * 8 + lane * E;
+    const int sectors = (m + 7) >> 3;
+    const unsigned none = ffEntry(i, 13, true);
+    unsigned next[N];
+#pragma unroll
+    for (int u = 0; u < S; ++u, p += stride)
+        if (u < sectors) loadEntries<E>(p, next + u * E);
+    for (int s = 0; s < sectors; s += S) {
+        unsigned e[N];
+        bool ok[N];
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            ok[c] = (s + c / E) * 8 + lane * E + c % E < m;
+            e[c] = ok[c] ? next[c] : none;
+        }
+#pragma unroll
+        for (int c = 0; c < N; c += B) {
+            decltype(gather(0u)) g[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) g[u] = gather(e[c + u]);
+            if (c == (N / B / 2) * B) {
+#pragma unroll
+                for (int u = 0; u < S; ++u, p += stride)
+                    if (s + S + u < sectors) loadEntries<E>(p, next + u * E);
+            }
+            use(e + c, g, ok + c);
+        }
+    }
+}
+
+// A fluid partner's state read by the continuity and momentum terms of scenes
+// whose fluids differ (the buffers a pass reads are not written by it:
+// read-only loads).
 struct FluidPartner {
     float4 p, v, par;
     float dr;
 };
-
-template <bool U>
-__device__ __forceinline__ FluidPartner<U> gatherFluid(const DeviceState& d, int j, const float4* __restrict__ ph,
-                                                       const float4* __restrict__ vh, const float* __restrict__ dr,
-                                                       const float4* __restrict__ pd)
+__device__ __forceinline__ FluidPartner gatherFluid(const DeviceState& d, int j, const float4* __restrict__ ph,
+                                                    const float4* __restrict__ vh, const float* __restrict__ dr)
 {
-    FluidPartner<U> q;
-    if constexpr (U) {
-        q.p = __ldg(pd + j);
-        q.dr = q.p.w;
-    } else {
-        q.p = __ldg(ph + j);
-        q.dr = __ldg(dr + j);
-        q.par = __ldg(d.fpar + j);
+    return FluidPartner{__ldg(ph + j), __ldg(vh + j), __ldg(d.fpar + j), __ldg(dr + j)};
+}
+
+// A partner of a uniform fluid: the pass's record, one sector in one 32-byte load.
+__device__ __forceinline__ FluidRec loadRecord(const FluidRec* __restrict__ p)
+{
+    FluidRec r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.pc.x), "=f"(r.pc.y), "=f"(r.pc.z), "=f"(r.pc.w), "=f"(r.vd.x), "=f"(r.vd.y), "=f"(r.vd.z), "=f"(r.vd.w)
+        : "l"(p));
+    return r;
+}
+
+// The loop over the partners of a uniform fluid: term(r, record, ok), r the
+// relative position.  Entries whose walk cell does not give their offset (lists
+// made by the walk) are mended out of line.
+template <int L, int B, class Term>
+__device__ __forceinline__ void forFluidRecords(const DeviceState& d, const WalkTable& tab, const FluidRec* __restrict__ rec,
+                                                int i, int lane, int m, int4 ci, float4 pi, Term term)
+{
+    forFluidPartners<L, B>(
+        d.ff, d.nf, i, lane, m, [&](unsigned e) { return loadRecord(rec + ffPartner(e)); },
+        [&](const unsigned* e, const FluidRec* q, const bool* ok) {
+            float3 r[B];
+            unsigned all = e[0];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                const int t = entryWalk(e[u]);
+                r[u] = make_float3((pi.x - q[u].pc.x) - tab.o[0][t], (pi.y - q[u].pc.y) - tab.o[1][t],
+                                   (pi.z - q[u].pc.z) - tab.o[2][t]);
+                all &= e[u];
+            }
+            if (!ffRegular(all)) {
+#pragma unroll
+                for (int u = 0; u < B; ++u)
+                    if (!ffRegular(e[u])) r[u] = relF(ci, pi, d.fcell[ffPartner(e[u])], q[u].pc, d.grid);
+            }
+#pragma unroll
+            for (int u = 0; u < B; ++u) term(r[u], q[u], ok[u]);
+        });
+}
+
+// Reciprocal and square root of the pair terms: one operation of the special
+// function unit each (the plain operators also handle subnormal inputs, which
+// densities, their products and the distances of list partners are not).
+__device__ __forceinline__ float fastRcp(float x)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float fastSqrt(float x)
+{
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// term(e, state) for the entries inside the list, one by one.
+template <class Term>
+struct EachOf {
+    Term term;
+    template <class State, int B>
+    __device__ __forceinline__ void operator()(const unsigned* e, const State (&q)[B], const bool* ok) const
+    {
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            if (ok[u]) term(e[u], q[u]);
     }
-    q.v = __ldg(vh + j);
-    return q;
+};
+template <class Term>
+__device__ __forceinline__ EachOf<Term> eachOf(Term term)
+{
+    return EachOf<Term>{term};
 }
 
 // ---- lane groups ----
@@ -182,10 +250,15 @@ __device__ __forceinline__ float groupSum(const KahanF& k)
 }
 
 // ---- continuity (+ optional drift) ----
+// What bounds the pair loops: latency of the partner gathers at the warps the
+// registers allow (issue slots 50-60 % busy, L1 55 %, DRAM 15 %).  A partner is
+// one 32-byte record in one load, the terms of a round run without branches,
+// and two lanes share a list sector: 400k particles 160 to 133 us (momentum 202
+// to 143), 1.0M 354 to 301 (440 to 317), 48k 28 to 25 (33 to 31).
 struct ContinuityArgs {
     int ps, vs, ds, dd;  // position / velocity / density source, density destination
-    int rec;             // partner records read (uniform fluids): fpd[rec] holds position ps, density ds
-    int recOut;          // -1: none; else fpd[recOut] receives the drifted position and density dd
+    int rec;             // partner records read (uniform fluids): position ps, velocity vs, density ds
+    int recOut;          // -1: none; else frec[recOut] receives the drifted position, the velocity and density dd
     int driftTo;         // -1: no drift; else position buffer receiving x + v * drift
     int velCopyTo;       // -1: none; else velocity buffer receiving a copy of this particle's velocity
     int countStep;       // 1: the pass ends the step (nothing after it can raise a status): count it
@@ -197,7 +270,7 @@ template <int L, bool U>
 __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(DeviceState d, ContinuityArgs a)
 {
     stepKernelBegin();
-    __shared__ float4 walkTab[27];
+    __shared__ WalkTable walkTab;
     fillWalkTable(walkTab, d.grid.cs);
     if (a.countStep && blockIdx.x == 0 && threadIdx.x == 0 && *d.status == 0) atomicAdd(d.stepsDone, 1);
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -210,32 +283,32 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
         o = loadSelf(d, i, a.ps, a.vs, a.ds);
         const int n = d.nf;
         const int nff = min(d.ffc[i], d.kff);
-        // U: every fluid particle has the same rest density, sound speed,
-        // viscosity, mass and smoothing length - one gather fewer per
-        // neighbour, and the kernel's constants and the shared sound speed
-        // taken out of the loop (one division per pair instead of five)
-        const float negTwoRhoM = -2.f * o.rho * d.fparU.w;
-        const float4* __restrict__ ph = d.fph[a.ps];
-        const float4* __restrict__ vh = d.fvh[a.vs];
-        const float* __restrict__ drh = d.fdrho[a.ds];
-        const float4* __restrict__ pd = d.fpd[a.rec];
-        forFluidPartners<L, batchDepth<L>()>(
-            d.ff, n, i, lane, nff, [&](unsigned e) { return gatherFluid<U>(d, ffPartner(e), ph, vh, drh, pd); },
-            [&](unsigned e, const FluidPartner<U>& q) {
-                const float3 r = fluidRel(d, walkTab, o.c, o.p, e, ffPartner(e), q.p);
-                const float r2 = dot3(r, r);
-                if constexpr (U) {
-                    // the shared constants are read from the kernel parameters
-                    if (r2 >= d.fconstU.x) return;
-                    const float rhoj = d.fparU.x + q.dr;
-                    const float Pj = q.dr * d.fparU.y * d.fparU.y;
-                    const float rr = sqrtf(r2);
+        if constexpr (U) {
+            // every fluid particle has the same rest density, sound speed,
+            // viscosity, mass and smoothing length: the kernel's constants come
+            // from the kernel parameters, P_i - P_j = c^2 (dRho_i - dRho_j)
+            const float drhoI = d.fdrho[a.ds][i];
+            const float scale = -2.f * o.rho * d.fparU.w * d.fconstU.z;
+            forFluidRecords<L, BATCH>(
+                d, walkTab, d.frec[a.rec], i, lane, nff, o.c, o.p, [&](float3 r, const FluidRec& q, bool ok) {
+                    const float r2 = ok ? dot3(r, r) : d.fconstU.x;
+                    const float rhoj = d.fparU.x + q.vd.w;
+                    const float rr = fastSqrt(r2);
                     const float tt = 1.f - rr * d.fconstU.y;
-                    const float G = d.fconstU.z * tt * tt * tt;
-                    const float3 vij = o.v - xyz(q.v);
-                    acc.add(negTwoRhoM * G / (rhoj * (o.rho + rhoj)) *
-                            (rhoj * dot3(vij, r) + (o.P - Pj) * rr * d.fconstU.w));
-                } else {
+                    const float3 vij = o.v - xyz(q.vd);
+                    const float flux = rhoj * dot3(vij, r) + (drhoI - q.vd.w) * d.fparU.y * rr;
+                    const float term = scale * (tt * tt * tt) * fastRcp(rhoj * (o.rho + rhoj)) * flux;
+                    acc.add(r2 >= d.fconstU.x ? 0.f : term);
+                });
+        } else {
+            const float4* __restrict__ ph = d.fph[a.ps];
+            const float4* __restrict__ vh = d.fvh[a.vs];
+            const float* __restrict__ drh = d.fdrho[a.ds];
+            forFluidPartners<L, BATCH>(
+                d.ff, n, i, lane, nff, [&](unsigned e) { return gatherFluid(d, ffPartner(e), ph, vh, drh); },
+                eachOf([&](unsigned e, const FluidPartner& q) {
+                    const float3 r = fluidRel(d, walkTab, o.c, o.p, e, ffPartner(e), q.p);
+                    const float r2 = dot3(r, r);
                     const float h = 0.5f * (o.h + q.p.w);
                     if (r2 >= 4.f * h * h) return;
                     const float rhoj = q.par.x + q.dr;
@@ -248,12 +321,12 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
                     const float c = 0.5f * (o.cs + q.par.y);
                     const float3 vij = o.v - xyz(q.v);
                     acc.add(-2.f * o.rho * Vj * G / (o.rho + rhoj) * (rhoj * dot3(vij, r) + (o.P - Pj) * rr / c));
-                }
-            });
+                }));
+        }
         const int nfs = min(d.fsc[i], d.kfs);
         const float ci2 = o.cs * o.cs;
         for (int k = lane; k < nfs; k += L) {
-            const int sa = fsPartner(d.fs[(size_t)k * n + i]);
+            const int sa = fsPartner(d.fs[listAt(k, i, n)]);
             const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
             if (!sp.inside) continue;
             acc.add(-2.f * o.rho * sp.Va * sp.G / (o.rho + sp.rhoa) *
@@ -266,10 +339,12 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
     d.fdrho[a.dd][i] = drho;
     if (a.driftTo >= 0) {
         float4 xh = d.fph[a.ps][i], xl = d.fpl[a.ps][i];
-        dfAxpy(xh, xl, d.fvh[a.vs][i], d.fvl[a.vs][i], a.drift);
+        const float4 v = d.fvh[a.vs][i];
+        dfAxpy(xh, xl, v, d.fvl[a.vs][i], a.drift);
         d.fph[a.driftTo][i] = xh;
         d.fpl[a.driftTo][i] = xl;
-        if (U && a.recOut >= 0) d.fpd[a.recOut][i] = make_float4(xh.x, xh.y, xh.z, drho);
+        if (U && a.recOut >= 0)
+            d.frec[a.recOut][i] = FluidRec{make_float4(xh.x, xh.y, xh.z, 0.f), make_float4(v.x, v.y, v.z, drho)};
     }
     if (a.velCopyTo >= 0) {
         d.fvh[a.velCopyTo][i] = d.fvh[a.vs][i];
@@ -284,7 +359,7 @@ template <int L, bool U>
 __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceState d, dfl dtf, dfl halfDtf)
 {
     stepKernelBegin();
-    __shared__ float4 walkTab[27];
+    __shared__ WalkTable walkTab;
     fillWalkTable(walkTab, d.grid.cs);
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if ((t & ~31) >= d.nf * L || *d.status) return;
@@ -295,31 +370,34 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
         const Self o = loadSelf(d, i, 1, 0, 1);
         const int n = d.nf;
         const int nff = min(d.ffc[i], d.kff);
-        // U: the same parameters and smoothing length for every particle (see
-        // kContinuity): three divisions per pair instead of seven
-        const float twoNuRhoI = 2.f * d.fparU.z * o.rho, twoVi = 2.f * o.V;
-        forFluidPartners<L, batchDepth<L>()>(
-            d.ff, n, i, lane, nff,
-            [&](unsigned e) { return gatherFluid<U>(d, ffPartner(e), d.fph[1], d.fvh[0], d.fdrho[1], d.fpd[1]); },
-            [&](unsigned e, const FluidPartner<U>& q) {
-                const float3 r = fluidRel(d, walkTab, o.c, o.p, e, ffPartner(e), q.p);
-                const float r2 = dot3(r, r);
-                if constexpr (U) {
-                    if (r2 >= d.fconstU.x) return;
-                    const float rhoj = d.fparU.x + q.dr;
-                    const float Pj = q.dr * d.fparU.y * d.fparU.y;
-                    const float rr = sqrtf(r2);
+        if constexpr (U) {  // see kContinuity
+            const float c2 = d.fparU.y * d.fparU.y;
+            const float twoNuRhoI = 2.f * d.fparU.z * o.rho, scale = 2.f * o.V * d.fconstU.z;
+            forFluidRecords<L, BATCH>(
+                d, walkTab, d.frec[1], i, lane, nff, o.c, o.p, [&](float3 r, const FluidRec& q, bool ok) {
+                    const float r2 = ok ? dot3(r, r) : d.fconstU.x;
+                    const float rhoj = d.fparU.x + q.vd.w;
+                    const float Pj = q.vd.w * c2;
+                    const float rr = fastSqrt(r2);
                     const float tt = 1.f - rr * d.fconstU.y;
-                    const float G = d.fconstU.z * tt * tt * tt;
-                    const float3 vij = o.v - xyz(q.v);
-                    const float dU = -dot3(vij, r) / rr;  // U_L - U_R
+                    const float3 vij = o.v - xyz(q.vd);
+                    const float dU = -dot3(vij, r) * fastRcp(rr);  // U_L - U_R
                     const float beta = fminf(3.f * fmaxf(dU, 0.f), d.fparU.y);
-                    const float invSum = 1.f / (o.rho + rhoj);
+                    const float invSum = fastRcp(o.rho + rhoj);
                     const float Ps = (o.rho * Pj + rhoj * o.P + o.rho * rhoj * beta * dU) * invSum;
                     const float gbar = twoNuRhoI * rhoj * invSum;  // 2 g_i g_j / (g_i + g_j), g = nu rho
-                    const float w = twoVi * G / rhoj;              // 2 V_i V_j G / m, V_j = m / rho_j
-                    acc.add((r * Ps - vij * gbar) * w);
-                } else {
+                    // 2 V_i V_j G / m, V_j = m / rho_j
+                    const float w = scale * (tt * tt * tt) * fastRcp(rhoj);
+                    const float3 term = (r * Ps - vij * gbar) * w;
+                    acc.add(r2 >= d.fconstU.x ? make_float3(0.f, 0.f, 0.f) : term);
+                });
+        } else {
+            forFluidPartners<L, BATCH>(
+                d.ff, n, i, lane, nff,
+                [&](unsigned e) { return gatherFluid(d, ffPartner(e), d.fph[1], d.fvh[0], d.fdrho[1]); },
+                eachOf([&](unsigned e, const FluidPartner& q) {
+                    const float3 r = fluidRel(d, walkTab, o.c, o.p, e, ffPartner(e), q.p);
+                    const float r2 = dot3(r, r);
                     const float h = 0.5f * (o.h + q.p.w);
                     if (r2 >= 4.f * h * h) return;
                     const float rhoj = q.par.x + q.dr;
@@ -338,12 +416,12 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
                     const float gbar = 2.f * o.gam * gj / (o.gam + gj);
                     const float w = 2.f * o.V * Vj * G / o.m;
                     acc.add((r * Ps - vij * gbar) * w);
-                }
-            });
+                }));
+        }
         const int nfs = min(d.fsc[i], d.kfs);
         const float ci2 = o.cs * o.cs;
         for (int k = lane; k < nfs; k += L) {
-            const int sa = fsPartner(d.fs[(size_t)k * n + i]);
+            const int sa = fsPartner(d.fs[listAt(k, i, n)]);
             const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
             if (!sp.inside) continue;
             const float3 via = o.v - sp.v;
@@ -371,7 +449,8 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
     dfAxpy(xh, xl, vh, vl, halfDtf);
     d.fph[0][i] = xh;
     d.fpl[0][i] = xl;
-    if (U) d.fpd[2][i] = make_float4(xh.x, xh.y, xh.z, d.fdrho[1][i]);  // the second continuity pass's partners
+    if (U)  // the second continuity pass's partners
+        d.frec[2][i] = FluidRec{make_float4(xh.x, xh.y, xh.z, 0.f), make_float4(vh.x, vh.y, vh.z, d.fdrho[1][i])};
     // the fluid candidates go stale once a particle has moved half the margin
     const int4 c = d.fcell[i];
     const float4 p0 = d.fvref[i];
@@ -381,15 +460,14 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
     if (!(dx * dx + dy * dy + dz * dz <= half * half)) *(volatile int*)d.frebuild = 1;
 }
 
-// The first continuity pass's partner records: position 0 and density 0 as
-// the step's search and Shepard re-initialisation leave them.
-__global__ void kPackPartners(DeviceState d)
+// The first continuity pass's partner records from the state.
+__global__ void kFluidRecords(DeviceState d)
 {
     stepKernelBegin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= d.nf || *d.status) return;
-    const float4 x = d.fph[0][i];
-    d.fpd[0][i] = make_float4(x.x, x.y, x.z, d.fdrho[0][i]);
+    const float4 x = d.fph[0][i], v = d.fvh[0][i];
+    d.frec[0][i] = FluidRec{make_float4(x.x, x.y, x.z, packCell(d.fcell[i])), make_float4(v.x, v.y, v.z, d.fdrho[0][i])};
 }
 
 template <int L>
@@ -412,13 +490,13 @@ __global__ void __launch_bounds__(T) kDensityReinit(DeviceState d, int storeRefe
         struct PartnerPosition {
             float4 h, l;
         };
-        forFluidPartners<L, batchDepth<L>()>(
+        forFluidPartners<L, BATCH>(
             d.ff, n, i, lane, nff,
             [&](unsigned e) {
                 const int j = ffPartner(e);
                 return PartnerPosition{__ldg(d.fph[0] + j), __ldg(d.fpl[0] + j)};
             },
-            [&](unsigned e, const PartnerPosition& q) {
+            eachOf([&](unsigned e, const PartnerPosition& q) {
                 const unsigned code = (unsigned)entryWalk(e);
                 int4 cj;
                 if (ffRegular(e))
@@ -429,12 +507,12 @@ __global__ void __launch_bounds__(T) kDensityReinit(DeviceState d, int storeRefe
                 const dfl r = dfNorm(relDF(ci, pi, li, cj, q.h, q.l, d.grid));
                 if (df_ge0(df_sub(r, twoH))) return;  // q >= 2
                 S = df_add(S, shepardTerm(r, invh));
-            });
+            }));
         // V0_a / V0_i = (2 r_a / (h_i / 1.3))^3 = (2.6 r_a / h_i)^3
         const dfl k26 = df_from_double(2.6);
         const int nfs = min(d.fsc[i], d.kfs);
         for (int k = lane; k < nfs; k += L) {
-            const int a = fsPartner(d.fs[(size_t)k * n + i]);
+            const int a = fsPartner(d.fs[listAt(k, i, n)]);
             const dfl r = dfNorm(relDF(ci, pi, li, d.scell[a], d.sph[a], d.spl[a], d.grid));
             if (df_ge0(df_sub(r, twoH))) continue;
             const float4 ra = d.srad[a];
@@ -453,7 +531,9 @@ __global__ void __launch_bounds__(T) kDensityReinit(DeviceState d, int storeRefe
         const float rho0 = d.fpar[i].x;
         // max(rho*, rho0 S / S0) - rho0 = max(dRho, rho0 (S - S0) / S0)
         const float cand = rho0 * ((diff.hi + diff.lo) / s0.x);
-        d.fdrho[0][i] = fmaxf(d.fdrho[0][i], cand);
+        const float drho = fmaxf(d.fdrho[0][i], cand);
+        d.fdrho[0][i] = drho;
+        if (d.uniformFluid) d.frec[0][i].vd.w = drho;
     }
 }
 
@@ -506,7 +586,7 @@ __global__ void kCouplingPairs(DeviceState d, int src, float4* out)
     const int m = min(d.fsc[i], d.kfs);
     for (int k = 0; k < m; ++k) {
         bool inside;
-        const float3 f = couplingPairForce(d, src, i, fsPartner(d.fs[(size_t)k * d.nf + i]), inside);
+        const float3 f = couplingPairForce(d, src, i, fsPartner(d.fs[listAt(k, i, d.nf)]), inside);
         out[(size_t)k * d.nf + i] = f4(f);
     }
 }
@@ -522,7 +602,7 @@ void launchDensityReinit(const DeviceState& d, int iStep, cudaStream_t s)
 
 int fluidLanes(int nf)
 {
-    int L = 1;
+    int L = 2;
     while (L < 8 && (long long)nf * L < 152LL * 2048) L *= 2;
     return L;
 }
@@ -537,12 +617,17 @@ void launchContinuityPass(const DeviceState& d, int which, double dtf, cudaStrea
     a.drift = df_from_double(0.5 * dtf);
     if (which == 0) {  // first half step: densities 0 -> 1, drift positions 0 -> 1
         a.ps = 0; a.vs = 0; a.ds = 0; a.dd = 1; a.driftTo = 1; a.velCopyTo = -1; a.rec = 0; a.recOut = 1;
-        if (d.uniformFluid) launchStep(kPackPartners, blocksFor(d.nf, 256), 256, s, d);
     } else {           // second half step: densities 1 -> 0, velocity 1 -> 0
         a.ps = 0; a.vs = 1; a.ds = 1; a.dd = 0; a.driftTo = -1; a.velCopyTo = 0; a.rec = 2; a.recOut = -1;
     }
     if (d.uniformFluid) LAUNCH_LANES_U(kContinuity, true, d.lanes, d.nf, T, s, d, a);
     else LAUNCH_LANES_U(kContinuity, false, d.lanes, d.nf, T, s, d, a);
+}
+
+void launchFluidRecords(const DeviceState& d, cudaStream_t s)
+{
+    if (d.nf <= 0 || !d.uniformFluid) return;
+    launchStep(kFluidRecords, blocksFor(d.nf, 256), 256, s, d);
 }
 
 void launchMomentumPass(const DeviceState& d, double dtf, cudaStream_t s)

@@ -63,7 +63,7 @@ __device__ __forceinline__ void buildSolidPartners(const DeviceState& d, int p, 
             if (d2 < c2 * (1.f - 1.e-5f)) take = true;
             else if (d2 <= c2 * (1.f + 1.e-5f)) take = withinCut(ci, hi, li, ca, ha, d.spl, a, cutDF, d.grid);
             if (take) {
-                if (nfs < d.kfs) d.fs[(size_t)nfs * n + p] = fsEntry(a, t);
+                if (nfs < d.kfs) d.fs[listAt(nfs, p, n)] = fsEntry(a, t);
                 ++nfs;
             }
         }
@@ -120,7 +120,7 @@ __device__ __forceinline__ void continuitySolids(const DeviceState& d, const Sel
     const int nfs = min(d.fsc[p], d.kfs);
     const float ci2 = o.cs * o.cs;
     for (int k = 0; k < nfs; ++k) {
-        const int sa = fsPartner(d.fs[(size_t)k * d.nf + p]);
+        const int sa = fsPartner(d.fs[listAt(k, p, d.nf)]);
         const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
         if (!sp.inside) continue;
         acc.add(-2.f * o.rho * sp.Va * sp.G / (o.rho + sp.rhoa) *
@@ -132,7 +132,7 @@ __device__ __forceinline__ void momentumSolids(const DeviceState& d, const Self&
     const int nfs = min(d.fsc[p], d.kfs);
     const float ci2 = o.cs * o.cs;
     for (int k = 0; k < nfs; ++k) {
-        const int sa = fsPartner(d.fs[(size_t)k * d.nf + p]);
+        const int sa = fsPartner(d.fs[listAt(k, p, d.nf)]);
         const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
         if (!sp.inside) continue;
         const float3 via = o.v - sp.v;
@@ -191,7 +191,7 @@ __device__ __forceinline__ void shepardFinish(const DeviceState& d, int p, int4 
     const dfl k26 = df_from_double(2.6);
     const int nfs = min(d.fsc[p], d.kfs);
     for (int k = 0; k < nfs; ++k) {
-        const int a = fsPartner(d.fs[(size_t)k * d.nf + p]);
+        const int a = fsPartner(d.fs[listAt(k, p, d.nf)]);
         const dfl r = dfNorm(relDF(ci, pi, li, d.scell[a], d.sph[a], d.spl[a], d.grid));
         if (df_ge0(df_sub(r, twoH))) continue;
         const float4 ra = d.srad[a];
@@ -445,7 +445,7 @@ __global__ void kBitsToLists(DeviceState d)
         for (int j = d.fcellStart[key], e = d.fcellStart[key + 1]; j < e; ++j, ++k) {
             if (k >= 32 * d.kbits) return;
             if (!((d.fbits[(size_t)(k >> 5) * d.nf + p] >> (k & 31)) & 1u)) continue;
-            if (cnt < d.kff) d.ff[(size_t)cnt * d.nf + p] = ffEntry(j, t, true);
+            if (cnt < d.kff) d.ff[listAt(cnt, p, d.nf)] = ffEntry(j, t, true);
             ++cnt;
         }
     }

@@ -126,11 +126,11 @@ __global__ void kPairFrame(DeviceState d, const int* count, const int* offset, f
     if (m == 0) return;
     const double3 pf = fluidPosition(d, s);
     for (int k = 0; k < m; ++k) {
-        const int v = d.fs[(size_t)k * n + s];
+        const int v = d.fs[listAt(k, s, n)];
         const long long key = (long long)entryWalk((unsigned)v) * d.ns + fsPartner(v);
         int rank = 0;
         for (int q = 0; q < m; ++q) {
-            const int u = d.fs[(size_t)q * n + s];
+            const int u = d.fs[listAt(q, s, n)];
             rank += (long long)entryWalk((unsigned)u) * d.ns + fsPartner(u) < key ? 1 : 0;
         }
         const long long w = first + rank;
