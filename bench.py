@@ -272,6 +272,7 @@ def stage_bytes(stage, c):
     kff = c.get("fluid_partners", 0.0)
     kfs = c.get("fluid_solid_partners", 0.0)
     table = {
+        # (with a contact list; a step of a run on contact pairs moves less)
         # per pair, once: partner id 4 + springs in 48 + springs out 48 + F T TA TB out 64; per
         # active solid: cell ph pl vh vl wh wl rad flags 144 + count 4; per bond: 160 (below)
         "pair_forces": 164 * P + 148 * Ns + 160 * Nb,

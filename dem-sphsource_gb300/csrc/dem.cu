@@ -14,6 +14,7 @@
 //
 // The per-particle gather adds forward pairs and subtracts reverse pairs in
 // list order - no atomics, so results are bit-reproducible run to run.
+#include "cell_sort.cuh"
 #include "kernels.cuh"
 #include "contact_rows.cuh"
 #include "warp_items.cuh"
@@ -165,10 +166,9 @@ __device__ __forceinline__ float3 contactVel(const DeviceState& d, int a, int b,
 struct PairForce {
     float3 F, T, TA, TB;
 };
-__device__ __forceinline__ PairForce pairForce(const DeviceState& d, int a, int b, float3& es, float3& er,
-                                               float3& et, float dt)
+__device__ __forceinline__ PairForce pairForceAt(const DeviceState& d, const PairGeom& g, int a, int b, float3& es,
+                                                 float3& er, float3& et, float dt)
 {
-    const PairGeom g = pairGeometry(d, a, b);
     const float4 ra = d.srad[a], rb = d.srad[b];
     const float R = ra.x * rb.x / (ra.x + rb.x);
     const float m = 1.f / (d.sph[a].w + d.sph[b].w);
@@ -184,6 +184,11 @@ __device__ __forceinline__ PairForce pairForce(const DeviceState& d, int a, int 
     p.TA = Tq + nxF * g.sA;
     p.TB = Tq + nxF * g.sB;
     return p;
+}
+__device__ __forceinline__ PairForce pairForce(const DeviceState& d, int a, int b, float3& es, float3& er,
+                                               float3& et, float dt)
+{
+    return pairForceAt(d, pairGeometry(d, a, b), a, b, es, er, et, dt);
 }
 
 // Slot (index into the per-slot arrays) of the forward contact (a, b), b > a,
@@ -224,8 +229,10 @@ __device__ __forceinline__ void addDF3(float4& h, float4& l, float3 dv)
 }
 
 // One parallel bond's update (integrate.cu:717-804): its state, force and
-// torques on both solids.
-__device__ __forceinline__ void bondUpdate(const DeviceState& d, int par, float dt, int b)
+// torques on both solids.  listed(i, j): whether the pair is in the step's
+// contact list.
+template <class Listed>
+__device__ __forceinline__ void bondUpdate(const DeviceState& d, float dt, int b, Listed listed)
 {
     // Every load the update needs is issued before the bond's checks (a broken
     // bond, a pair that left the contact list), which end in stores: the
@@ -242,7 +249,7 @@ __device__ __forceinline__ void bondUpdate(const DeviceState& d, int par, float 
     const float3 wr = spinDiff(d, i, j);
     const float4 ri = d.srad[i], rj = d.srad[j];
     const int ms = tableSlot(d.tab, d.sflags[i].x, d.sflags[j].x);
-    const long long slot = forwardSlot(d, par, i, j);
+    const bool inList = listed(i, j);
     if (bonded == 0) {
         d.bFnTt[b] = make_float4(0, 0, 0, 0);
         d.bFsH[b] = d.bFsL[b] = d.bTbH[b] = d.bTbL[b] = make_float4(0, 0, 0, 0);
@@ -250,7 +257,7 @@ __device__ __forceinline__ void bondUpdate(const DeviceState& d, int par, float 
         d.bF[b] = d.bTA[b] = d.bTB[b] = make_float4(0, 0, 0, 0);
         return;
     }
-    if (slot < 0) {  // the pair left the contact list: the bond breaks
+    if (!inList) {  // the pair left the contact list: the bond breaks
         d.bon[b] = 0;
         d.bF[b] = d.bTA[b] = d.bTB[b] = make_float4(0, 0, 0, 0);
         return;
@@ -423,7 +430,7 @@ __global__ void __launch_bounds__(T, DEMSPH_PAIR_FORCE_BLOCKS) kPairForces(Devic
     if (*d.status) return;
     if ((int)blockIdx.x >= contactBlocks) {
         const int b = ((int)blockIdx.x - contactBlocks) * blockDim.x + threadIdx.x;
-        if (b < d.nb) bondUpdate(d, par, dt, b);
+        if (b < d.nb) bondUpdate(d, dt, b, [&](int i, int j) { return forwardSlot(d, par, i, j) >= 0; });
         return;
     }
     // this step's flag has been read by every row's contact detection (the
@@ -484,6 +491,31 @@ __global__ void __launch_bounds__(T, DEMSPH_PAIR_FORCE_BLOCKS) kPairForces(Devic
 // GATHER_BATCH at a time before their sums (the slots [k * nrow + row] of
 // neighbouring rows are neighbouring words).
 constexpr int GATHER_BATCH = 4;
+// The row's bonds in bond order.
+__device__ __forceinline__ void addBondForces(const DeviceState& d, int a, int b0, int b1, KahanF3& F, KahanF3& Tq)
+{
+    for (int q0 = b0; q0 < b1; q0 += GATHER_BATCH) {
+        int bi[GATHER_BATCH];
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u) bi[u] = q0 + u < b1 ? d.bondList[q0 + u] : 0;
+        float4 f[GATHER_BATCH], t[GATHER_BATCH];
+        bool sideA[GATHER_BATCH];
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u)
+            if (q0 + u < b1) {
+                f[u] = d.bF[bi[u]];
+                sideA[u] = d.bab[bi[u]].x == a;
+                t[u] = sideA[u] ? d.bTA[bi[u]] : d.bTB[bi[u]];
+            }
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u)
+            if (q0 + u < b1) {
+                F.add(sideA[u] ? xyz(f[u]) : -xyz(f[u]));
+                Tq.add(sideA[u] ? xyz(t[u]) : -xyz(t[u]));
+            }
+    }
+}
+
 // Row `row`'s sums and tail; returns its solid.
 __device__ __forceinline__ int solidForcesRow(const DeviceState& d, int par, float dt, int withCoupling, int row)
 {
@@ -524,26 +556,7 @@ __device__ __forceinline__ int solidForcesRow(const DeviceState& d, int par, flo
                 Tq.add(xyz(t[u]));
             }
     }
-    for (int q0 = b0; q0 < b1; q0 += GATHER_BATCH) {
-        int bi[GATHER_BATCH];
-#pragma unroll
-        for (int u = 0; u < GATHER_BATCH; ++u) bi[u] = q0 + u < b1 ? d.bondList[q0 + u] : 0;
-        float4 f[GATHER_BATCH], t[GATHER_BATCH];
-        bool sideA[GATHER_BATCH];
-#pragma unroll
-        for (int u = 0; u < GATHER_BATCH; ++u)
-            if (q0 + u < b1) {
-                f[u] = d.bF[bi[u]];
-                sideA[u] = d.bab[bi[u]].x == a;
-                t[u] = sideA[u] ? d.bTA[bi[u]] : d.bTB[bi[u]];
-            }
-#pragma unroll
-        for (int u = 0; u < GATHER_BATCH; ++u)
-            if (q0 + u < b1) {
-                F.add(sideA[u] ? xyz(f[u]) : -xyz(f[u]));
-                Tq.add(sideA[u] ? xyz(t[u]) : -xyz(t[u]));
-            }
-    }
+    addBondForces(d, a, b0, b1, F, Tq);
     solidRowTail(d, par, a, F, Tq, withCoupling, dt);
     return a;
 }
@@ -679,6 +692,290 @@ __global__ void __launch_bounds__(T, 6) kContactForces(DeviceState d, int par, f
         });
     if (!live) return;
     solidRowTail(d, par, a, F, Tq, withCoupling, dt);
+}
+
+// ---- runs of plain DEM steps on contact pairs ----
+// Building a step's contact list, finding each pair's springs in the previous
+// list and each pair's reverse slot took half of a dense bed's step; between
+// two rebuilds of the candidates none of it changes but the membership.  So
+// inside a run of plain DEM steps the forward candidates are the pairs: each
+// is tested against the reference's list criterion on the end-of-step offsets
+// (where the list would be built), evaluated once, and keeps its springs and
+// results in its slot; a row finds a reverse pair through the slot stored with
+// the candidate.  The tests, the contact law and the order of every sum are
+// those of the list kernels: the same bits.
+
+// The end-of-step view of the solids: offsets sphE/splE.
+__device__ __forceinline__ DeviceState endView(const DeviceState& d)
+{
+    DeviceState e = d;
+    e.sph = d.sphE;
+    e.spl = d.splE;
+    return e;
+}
+
+// Candidates of row r below its own solid a (the candidates are in index order).
+__device__ __forceinline__ int reverseCandidates(const DeviceState& d, int r, int a, int n)
+{
+    int v = 0;
+    while (v < n && d.vcand[(size_t)v * d.nrow + r] < a) ++v;
+    return v;
+}
+
+// The slots of row r's reverse pairs, in the rows of the lower solids (a pair's
+// two candidates are each other's: the test is symmetric).
+__device__ __forceinline__ void linkRow(const DeviceState& d, int r, int a, int reverse)
+{
+    const size_t nr = (size_t)d.nrow;
+    for (int k = 0; k < reverse; ++k) {
+        const int A = d.vcand[(size_t)k * nr + r];
+        const int ra = rowOf(d, A);
+        int link = -1;
+        if (ra >= 0) {
+            const int n = min(d.vcnt[ra], d.vcap);
+            int q = 0;  // forward rank
+            for (int m = 0; m < n; ++m) {
+                const int b = d.vcand[(size_t)m * nr + ra];
+                if (b == a) {
+                    link = (int)((size_t)q * nr + ra);
+                    break;
+                }
+                q += b > A ? 1 : 0;
+            }
+        }
+        d.plink[(size_t)k * nr + r] = link;
+    }
+}
+
+// After the first step of a run: every forward candidate's slot from the
+// step's list (in index order as the candidates are).
+__global__ void __launch_bounds__(T) kPairsOpen(DeviceState d, int par)
+{
+    stepKernelBegin();
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= d.nrow || *d.status) return;
+    const size_t nr = (size_t)d.nrow;
+    const int a = solidOf(d, r), n = min(d.vcnt[r], d.vcap);
+    const int vf = reverseCandidates(d, r, a, n), listed = min(d.fcnt[par][r], d.scap);
+    d.pfirst[r] = vf;
+    int m = 0;
+    for (int k = vf; k < n; ++k) {
+        const size_t slot = (size_t)(k - vf) * nr + r;
+        const int b = d.vcand[(size_t)k * nr + r];
+        while (m < listed && d.fwd[par][(size_t)m * nr + r] < b) ++m;
+        const bool in = m < listed && d.fwd[par][(size_t)m * nr + r] == b;
+        if (in)
+            for (int j = 0; j < d.pairSprings; ++j) d.pspring[j][slot] = d.springOut[par][j][(size_t)m * nr + r];
+        d.pflag[slot] = in ? PAIR_LIVE : PAIR_OUT;  // the springs of a listed pair without contact are zeros
+    }
+    linkRow(d, r, a, vf);
+}
+
+// At the start of every later step of a run: nothing, or the rebuild of stale
+// candidates - the solids' sort by cell, each row's candidates on the
+// end-of-step offsets with its pairs' flags and springs carried over, then the
+// links - as phases of one cooperative launch.  In the walk mode the run cannot
+// go on: ST_SPLIT_CONTACTS, before anything is written.
+__global__ void __launch_bounds__(SORT_THREADS) kPairsRebuild(DeviceState d, int par)
+{
+    stepKernelBegin();
+    if (*d.status) return;
+    if (*d.slowMode) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(d.status, ST_SPLIT_CONTACTS);
+        return;
+    }
+    if (!d.rebuild[par]) return;  // uniform: cleared below, once every block is past the barriers
+    unsigned gen = ((volatile unsigned*)d.gridBar)[1];
+    if (!solidSortPhases(d, gen)) return;
+    if (!gridBarrier(d.gridBar, gen, d.status)) return;
+    const DeviceState atEnd = endView(d);
+    const size_t nr = (size_t)d.nrow;
+    const int stride = gridDim.x * blockDim.x;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < d.nrow; r += stride) {
+        const int a = solidOf(d, r);
+        const int vf0 = d.pfirst[r], old = min(d.vcnt[r], d.vcap) - vf0;
+        d.oldCount[r] = old;
+        for (int q = 0; q < old; ++q) {
+            const size_t slot = (size_t)q * nr + r;
+            d.oldId[slot] = d.vcand[(size_t)(vf0 + q) * nr + r];
+            const unsigned char f = d.pflag[slot];
+            d.oldFlag[slot] = f;
+            if (f == PAIR_LIVE)
+                for (int j = 0; j < d.pairSprings; ++j) d.oldSpring[j][slot] = d.pspring[j][slot];
+        }
+        verletBuildRow(atEnd, r);
+        const int n = min(d.vcnt[r], d.vcap), vf = reverseCandidates(d, r, a, n);
+        d.pfirst[r] = vf;
+        int m = 0;
+        for (int k = vf; k < n; ++k) {
+            const size_t slot = (size_t)(k - vf) * nr + r;
+            const int b = d.vcand[(size_t)k * nr + r];
+            while (m < old && d.oldId[(size_t)m * nr + r] < b) ++m;
+            const bool live = m < old && d.oldId[(size_t)m * nr + r] == b && d.oldFlag[(size_t)m * nr + r] == PAIR_LIVE;
+            if (live)
+                for (int j = 0; j < d.pairSprings; ++j) d.pspring[j][slot] = d.oldSpring[j][(size_t)m * nr + r];
+            d.pflag[slot] = live ? PAIR_LIVE : PAIR_OUT;
+        }
+    }
+    if (!gridBarrier(d.gridBar, gen, d.status)) return;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < d.nrow; r += stride) linkRow(d, r, solidOf(d, r), d.pfirst[r]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)&d.rebuild[par] = 0;
+}
+
+// The pairs of a step, G lanes per row taking its forward candidates in turn
+// (the bonds in blocks of their own, from contactBlocks on).  A candidate's
+// list test and overlap need five 16-byte reads of its solid, issued together;
+// only a pair in contact reads the other five.
+//
+// What bounds it: latency of those reads, then issue (17 of 32 lanes active: a
+// third of the candidates are not in contact).  A packed bed of 200k grains (6
+// candidates, 4.7 listed pairs a grain): 60 us, and 40 for the sums with the
+// integration, where the contact list and both sides' forces in one launch took
+// 169 and the integration 18.
+#ifndef DEMSPH_PAIR_STEP_BLOCKS
+#define DEMSPH_PAIR_STEP_BLOCKS 6  // resident blocks of T per SM the registers allow
+#endif
+template <int G>
+__global__ void __launch_bounds__(T, DEMSPH_PAIR_STEP_BLOCKS) kPairStep(DeviceState d, int par, float dt, int contactBlocks)
+{
+    stepKernelBegin();
+    if (*d.status) return;
+    const DeviceState atEnd = endView(d);
+    if ((int)blockIdx.x >= contactBlocks) {
+        const int b = ((int)blockIdx.x - contactBlocks) * blockDim.x + threadIdx.x;
+        if (b < d.nb) bondUpdate(d, dt, b, [&](int i, int j) { return solidsTouch(atEnd, i, j); });
+        return;
+    }
+    // both flags are free for this step's closing drift (kPairsRebuild has read them)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *(volatile int*)&d.rebuild[par] = 0;
+        *(volatile int*)&d.rebuild[par ^ 1] = 0;
+    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = t / G;
+    if (r >= d.nrow) return;
+    const size_t nr = (size_t)d.nrow;
+    const int vf = d.pfirst[r], forward = min(d.vcnt[r], d.vcap) - vf;
+    const int a = solidOf(d, r);
+    for (int q = t % G; q < forward; q += G) {
+        const size_t slot = (size_t)q * nr + r;
+        const int b = d.vcand[slot + (size_t)vf * nr];
+        const int before = d.pflag[slot];
+        const bool in = solidsTouch(atEnd, a, b);
+        const PairGeom g = pairGeometry(d, a, b);
+        int now = PAIR_OUT;
+        if (in && !(g.delta > 0.f)) now = PAIR_LISTED;
+        if (in && g.delta > 0.f) {
+            now = PAIR_LIVE;
+            float3 s[3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) s[j] = make_float3(0.f, 0.f, 0.f);
+            if (before == PAIR_LIVE) {
+                s[0] = xyz(d.pspring[0][slot]);
+                if (d.pairSprings == 3) {
+                    s[1] = xyz(d.pspring[1][slot]);
+                    s[2] = xyz(d.pspring[2][slot]);
+                }
+            }
+            const PairForce p = pairForceAt(d, g, a, b, s[0], s[1], s[2], dt);
+            d.pspring[0][slot] = f4(s[0]);
+            if (d.pairSprings == 3) {
+                d.pspring[1][slot] = f4(s[1]);
+                d.pspring[2][slot] = f4(s[2]);
+            }
+            d.pforce[slot] = f4(p.F);
+            d.ptorqueA[slot] = f4(p.TA);
+            d.ptorqueB[slot] = f4(p.TB);
+        }
+        if (now != before) d.pflag[slot] = (unsigned char)now;
+    }
+}
+
+// Row `row`'s sums over the pairs and its tail (see solidForcesRow: the same
+// items in the same order, a listed pair without contact adds zeros); returns
+// its solid.
+__device__ __forceinline__ int pairSumsRow(const DeviceState& d, int par, float dt, int withCoupling, int row)
+{
+    const int a = solidOf(d, row);
+    const size_t nr = (size_t)d.nrow;
+    const int vf = d.pfirst[row], forward = min(d.vcnt[row], d.vcap) - vf;
+    const int b0 = d.bondStart[a], b1 = d.bondStart[a + 1];
+    KahanF3 F, Tq;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q0 = 0; q0 < forward; q0 += GATHER_BATCH) {
+        int flag[GATHER_BATCH];
+        float4 f[GATHER_BATCH], t[GATHER_BATCH];
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u) flag[u] = q0 + u < forward ? d.pflag[(size_t)(q0 + u) * nr + row] : PAIR_OUT;
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u) {
+            const size_t slot = (size_t)(q0 + u) * nr + row;
+            f[u] = flag[u] == PAIR_LIVE ? d.pforce[slot] : zero;
+            t[u] = flag[u] == PAIR_LIVE ? d.ptorqueA[slot] : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u)
+            if (flag[u] != PAIR_OUT) {
+                F.add(xyz(f[u]));
+                Tq.add(xyz(t[u]));
+            }
+    }
+    for (int q0 = 0; q0 < vf; q0 += GATHER_BATCH) {
+        int link[GATHER_BATCH], flag[GATHER_BATCH];
+        float4 f[GATHER_BATCH], t[GATHER_BATCH];
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u) link[u] = q0 + u < vf ? d.plink[(size_t)(q0 + u) * nr + row] : -1;
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u) flag[u] = link[u] >= 0 ? d.pflag[link[u]] : PAIR_OUT;
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u) {
+            f[u] = flag[u] == PAIR_LIVE ? d.pforce[link[u]] : zero;
+            t[u] = flag[u] == PAIR_LIVE ? d.ptorqueB[link[u]] : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < GATHER_BATCH; ++u)
+            if (flag[u] != PAIR_OUT) {
+                F.add(-xyz(f[u]));
+                Tq.add(-xyz(t[u]));
+            }
+    }
+    addBondForces(d, a, b0, b1, F, Tq);
+    solidRowTail(d, par, a, F, Tq, withCoupling, dt);
+    return a;
+}
+
+__global__ void __launch_bounds__(T) kPairSums(DeviceState d, int par, float dt, int withCoupling)
+{
+    stepKernelBegin();
+    if (*d.status) return;
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row < d.nrow) pairSumsRow(d, par, dt, withCoupling, row);
+}
+
+// The springs of the live pairs back into the lists of parity par (see
+// launchPairsClose); count: only need[0].
+__global__ void __launch_bounds__(T) kPairsClose(DeviceState d, int par, int old, int count)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= d.nrow) return;
+    const size_t nr = (size_t)d.nrow;
+    const int vf = d.pfirst[r];
+    const int m = old ? d.oldCount[r] : min(d.vcnt[r], d.vcap) - vf;
+    int n = 0;
+    for (int q = 0; q < m; ++q) {
+        const size_t slot = (size_t)q * nr + r;
+        if ((old ? d.oldFlag[slot] : d.pflag[slot]) != PAIR_LIVE) continue;
+        if (!count && n < d.scap) {
+            const size_t to = (size_t)n * nr + r;
+            d.fwd[par][to] = old ? d.oldId[slot] : d.vcand[slot + (size_t)vf * nr];
+            for (int j = 0; j < 3; ++j)
+                d.springOut[par][j][to] = j >= d.pairSprings ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                                             : (old ? d.oldSpring[j][slot] : d.pspring[j][slot]);
+        }
+        ++n;
+    }
+    if (count) atomicMax(&d.need[0], n);
+    else d.fcnt[par][r] = min(n, d.scap);
 }
 
 // x_i - centroid of pebble i as double-float per axis, then float.
@@ -1029,6 +1326,20 @@ __global__ void __launch_bounds__(T) kSolidForcesIntegrate(DeviceState d, int pa
     solidIntegrateOne<MODE>(d, a, half, d.rebuild + (par ^ 1));
 }
 
+// The same from the pairs of a run (the steps between its first and its last
+// always open the next one).
+__global__ void __launch_bounds__(T) kPairSumsIntegrate(DeviceState d, int par, float dt, int withCoupling, dfl half,
+                                                        int countStep)
+{
+    stepKernelBegin();
+    if (countStep && blockIdx.x == 0 && threadIdx.x == 0 && *d.status == 0) atomicAdd(d.stepsDone, 1);
+    if (*d.status) return;
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= d.nrow) return;
+    const int a = pairSumsRow(d, par, dt, withCoupling, row);
+    solidIntegrateOne<INTEGRATE_FUSED>(d, a, half, d.rebuild + (par ^ 1));
+}
+
 
 
 }  // namespace
@@ -1057,6 +1368,47 @@ void launchContactForces(const DeviceState& d, int par, float dt, cudaStream_t s
     if (d.nrow <= 0) return;
     launchStep(kContactForces, blocksFor(d.nrow, T), T, s, d, par, dt, d.nf > 0 ? 1 : 0);
 }
+void launchPairsOpen(const DeviceState& d, int par, cudaStream_t s)
+{
+    launchStep(kPairsOpen, blocksFor(d.nrow, T), T, s, d, par);
+}
+void launchPairsRebuild(const DeviceState& d, int par, cudaStream_t s)
+{
+    launchCooperative(kPairsRebuild, (unsigned)d.sortBlocks, SORT_THREADS, s, d, par);
+}
+#ifndef DEMSPH_PAIR_LANES
+#define DEMSPH_PAIR_LANES 0  // 0: the rule below
+#endif
+void launchPairStep(const DeviceState& d, int par, float dt, cudaStream_t s)
+{
+    // lanes per row: 16 warps' worth of threads per SM on small scenes.  A step
+    // of 3k grains takes 30.5 / 23.9 / 20.9 / 18.4 us with 1 / 2 / 4 / 8 lanes,
+    // of 20k 32.7 / 26.6 / 23.7 / 25.3, of 60k 40.3 / 40.4 / 41.3 / 41.0, of 200k
+    // 110 / 114 / 127 / 139.
+    int G = DEMSPH_PAIR_LANES;
+    if (G == 0)
+        for (G = 1; G < 8 && (long long)d.nrow * G < 152LL * 512;) G *= 2;
+    const int cb = blocksFor((long long)d.nrow * G, T), bb = d.nb > 0 ? blocksFor(d.nb, T) : 0;
+    auto* k = G == 8 ? kPairStep<8> : G == 4 ? kPairStep<4> : G == 2 ? kPairStep<2> : kPairStep<1>;
+    launchStep(k, cb + bb, T, s, d, par, dt, cb);
+}
+void launchPairSums(const DeviceState& d, int par, double dt, cudaStream_t s, int integrate, bool countStep)
+{
+    const int blocks = blocksFor(d.nrow, T), cpl = d.nf > 0 ? 1 : 0;
+    if (integrate == INTEGRATE_FUSED)
+        launchStep(kPairSumsIntegrate, blocks, T, s, d, par, (float)dt, cpl, df_from_double(0.5 * dt), countStep ? 1 : 0);
+    else
+        launchStep(kPairSums, blocks, T, s, d, par, (float)dt, cpl);
+}
+void launchPairsCount(const DeviceState& d, bool old, cudaStream_t s)
+{
+    ++t_kernelLaunches, kPairsClose<<<blocksFor(d.nrow, T), T, 0, s>>>(d, 0, old ? 1 : 0, 1);
+}
+void launchPairsClose(const DeviceState& d, int par, bool old, cudaStream_t s)
+{
+    ++t_kernelLaunches, kPairsClose<<<blocksFor(d.nrow, T), T, 0, s>>>(d, par, old ? 1 : 0, 0);
+}
+
 void launchClumpForce(const DeviceState& d, cudaStream_t s)
 {
     if (d.nc <= 0) return;

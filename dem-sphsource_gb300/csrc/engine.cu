@@ -189,6 +189,49 @@ void allocContactLists(demsph_engine* e)
     }
 }
 
+// The contact pairs of runs of plain DEM steps (a slot per forward candidate).
+void freePairs(demsph_engine* e)
+{
+    DeviceState& d = e->d;
+    void* ptrs[] = {d.pfirst, d.plink, d.pflag, d.pforce, d.ptorqueA, d.ptorqueB, d.oldCount, d.oldId, d.oldFlag,
+                    d.pspring[0], d.pspring[1], d.pspring[2], d.oldSpring[0], d.oldSpring[1], d.oldSpring[2]};
+    for (void* p : ptrs) freeOne(e, p);
+    d.pflag = nullptr;
+    for (int k = 0; k < 3; ++k) d.pspring[k] = d.oldSpring[k] = nullptr;
+}
+void allocPairs(demsph_engine* e)
+{
+    DeviceState& d = e->d;
+    const size_t nr = (size_t)d.nrow, c = (size_t)d.vcap * nr;
+    // slot indices are ints; the rebuild is a cooperative launch
+    if (!e->pairRuns || d.nrow <= 0 || d.sortBlocks <= 0 || c > 2000000000ull) return;
+    d.pfirst = dalloc<int>(nr, e->owned, e->stream);
+    d.plink = dalloc<int>(c, e->owned, e->stream, false);
+    d.pflag = dalloc<unsigned char>(c, e->owned, e->stream);
+    d.pforce = dalloc<float4>(c, e->owned, e->stream, false);
+    d.ptorqueA = dalloc<float4>(c, e->owned, e->stream, false);
+    d.ptorqueB = dalloc<float4>(c, e->owned, e->stream, false);
+    d.oldCount = dalloc<int>(nr, e->owned, e->stream);
+    d.oldId = dalloc<int>(c, e->owned, e->stream, false);
+    d.oldFlag = dalloc<unsigned char>(c, e->owned, e->stream);
+    for (int k = 0; k < d.pairSprings; ++k) {
+        d.pspring[k] = dalloc<float4>(c, e->owned, e->stream, false);
+        d.oldSpring[k] = dalloc<float4>(c, e->owned, e->stream, false);
+    }
+}
+
+// Springs a contact keeps: one (sliding) unless some material pair has rolling
+// or torsion friction (the law leaves those springs zero otherwise).
+int contactSprings(const demsph_scene* sc)
+{
+    const int n = sc->n_material * (sc->n_material + 1) / 2;
+    for (int k = 0; k < n; ++k)
+        if (sc->hertzian[8 * k + 6] > 0 || sc->hertzian[8 * k + 7] > 0 || sc->linear[11 * k + 9] > 0 ||
+            sc->linear[11 * k + 10] > 0)
+            return 3;
+    return 1;
+}
+
 // Tile mode of the fluid lists and pair loops (sph_tiles.cu) is used when
 // every fluid particle has the same parameters, the grid has at least three
 // cells along every axis (the walk's cells are then distinct), every particle
@@ -263,6 +306,11 @@ struct StageTimer {
     }
 };
 #define TIMED(tag) StageTimer _stage_timer(e, tag)
+// A stage whose work rides in another stage's launch: counted, without a time.
+void countStage(demsph_engine* e, const char* tag)
+{
+    if (e->profiling) e->timed.push_back({tag, nullptr, nullptr});
+}
 
 // ---- the five stages ----
 // endView: the solids' integration has already opened this step (a fused
@@ -271,8 +319,12 @@ struct StageTimer {
 // (launchContactForces).
 // beforeDetect: enqueued after the sorts and lists, before the contact
 // detection (a fork to the side stream).
+// pairs: a step of a run on contact pairs after its first: the pairs are rebuilt
+// when stale; PAIRS_STEP builds no list, PAIRS_LAST builds it with the springs
+// of the pairs.
+enum PairSearch { PAIRS_NONE = 0, PAIRS_STEP = 1, PAIRS_LAST = 2 };
 void stageNeighborSearch(demsph_engine* e, int iStep, int gap, bool endView = false, bool detect = true,
-                         const std::function<void()>* beforeDetect = nullptr)
+                         const std::function<void()>* beforeDetect = nullptr, PairSearch pairs = PAIRS_NONE)
 {
     e->keysAdvanced = false;  // this search's keys are the current ones until an integration rehashes
     const int npar = e->par ^ 1;  // the parity of the list this step builds
@@ -300,7 +352,10 @@ void stageNeighborSearch(demsph_engine* e, int iStep, int gap, bool endView = fa
         launchFluidHash(d, e->forceWalk || d.fluidTiles, s);
         launchFluidReorder(d, e->forceWalk || d.fluidTiles, s);
     }
-    if (solidsMove || e->forceWalk) {
+    if (pairs != PAIRS_NONE) {
+        TIMED("solid_hash_sort");  // with the candidates' rebuild
+        launchPairsRebuild(e->d, npar, s);
+    } else if (solidsMove || e->forceWalk) {
         TIMED("solid_hash_sort");
         launchSolidHash(d, forceSort, fluidStep, npar, s);
         launchSolidSort(d, forceSort, fluidStep, npar, s);
@@ -332,9 +387,9 @@ void stageNeighborSearch(demsph_engine* e, int iStep, int gap, bool endView = fa
     e->par = npar;
     e->walkOrder[e->par] = e->forceWalk;
     if (beforeDetect) (*beforeDetect)();
-    if (!detect) return;
+    if (!detect || pairs == PAIRS_STEP) return;
     TIMED("solid_contact_list");  // with the candidate rebuild when they are stale
-    launchContactDetect(d, e->par, e->forceWalk, s);
+    launchContactDetect(d, e->par, e->forceWalk, s, pairs == PAIRS_LAST);
 }
 
 void stageBefore(demsph_engine* e, double dt)
@@ -452,10 +507,18 @@ void fullStep(demsph_engine* e, double dt, int iStep, int gap, bool opened = fal
 // Without bonds (a bond reads the contact list) the opened steps build their
 // contact list in the contact stage, in the launch of the contact forces: the
 // fluid stage of a plain DEM step (the coupling force) does not read it.
+// Runs of three or more steps evaluate their contact candidates as pairs from
+// the second step to the last but one (pairRun): no list is built there.
+// Whether a run of `length` steps does.
+bool pairRun(const demsph_engine* e, int length)
+{
+    return e->pairRuns && e->d.pflag && length >= 3 && !e->forceWalk;
+}
 void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
 {
     DeviceState& d = e->d;
-    const bool merge = e->mergeContacts && d.nb == 0 && d.nrow > 0;
+    const bool pairs = pairRun(e, length);
+    const bool merge = !pairs && e->mergeContacts && d.nb == 0 && d.nrow > 0;
     stageNeighborSearch(e, iStep, gap);
     const long long pebbles = std::count(e->moveKind.begin(), e->moveKind.end(), (unsigned char)0);
     if (d.ns - d.nmove - pebbles > 0) {
@@ -484,7 +547,17 @@ void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
         if (!forked) stageFluid(e, dt, iStep + k, gap);
         const bool last = k == length - 1;
         bool integrated = false;
-        if (k > 0 && merge) {
+        if (pairs && k > 0 && !last) {
+            {
+                TIMED("pair_forces");  // with the bonds
+                launchPairStep(d, e->par, (float)dt, e->stream);
+            }
+            if (forked) join();
+            TIMED("solid_forces");
+            launchPairSums(d, e->par, dt, e->stream, fold ? INTEGRATE_FUSED : -1, true);
+            integrated = fold;
+            if (fold) countStage(e, "integrate_after");
+        } else if (k > 0 && merge) {
             TIMED("contact_forces");  // with the contact list of the step
             launchContactForces(d, e->par, (float)dt, e->stream);
         } else {
@@ -494,6 +567,10 @@ void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
                          fold ? (last ? INTEGRATE_AFTER : INTEGRATE_FUSED) : -1, true);
         }
         forked = false;
+        if (pairs && k == 0) {
+            TIMED("solid_contact_list");  // its springs into the pairs' slots
+            launchPairsOpen(d, e->par, e->stream);
+        }
         if (last) {
             if (integrated) e->keysAdvanced = true;  // as stageAfter
             else stageAfter(e, dt, d.nc > 0, true);
@@ -503,7 +580,8 @@ void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
             TIMED("integrate_after");  // the closing half of this step and the opening half of the next
             launchSolidIntegrate(d, dt, INTEGRATE_FUSED, e->par, d.nc > 0, true, e->stream);
         }
-        stageNeighborSearch(e, iStep + k + 1, gap, true, !merge, branch ? &fork : nullptr);
+        stageNeighborSearch(e, iStep + k + 1, gap, true, !merge, branch ? &fork : nullptr,
+                            !pairs ? PAIRS_NONE : (k + 1 < length - 1 ? PAIRS_STEP : PAIRS_LAST));
         forked = branch;
     }
 }
@@ -561,6 +639,8 @@ void grow(demsph_engine* e, int status)
             freeOne(e, p);
             d.vcap = std::max(d.vcap * 2, need[1] + need[1] / 2 + 1);
             d.vcand = dalloc<int>((size_t)d.vcap * nr, e->owned, e->stream, false);
+            freePairs(e);  // the springs are in the lists again (closePairs)
+            allocPairs(e);
             CK(cudaMemsetAsync(d.rebuild, 0xff, 2 * sizeof(int), e->stream));  // rebuild on the retry
         }
     }
@@ -597,7 +677,7 @@ void grow(demsph_engine* e, int status)
         d.kbits = std::max(2 * d.kbits, (need + 31) / 32 + 1);
         d.fbits = dalloc<unsigned>((size_t)d.kbits * d.nf, e->owned, e->stream, false);
     }
-    if (status & ST_SPLIT_CONTACTS) e->mergeContacts = false;  // the lists come from the walk from now on
+    if (status & ST_SPLIT_CONTACTS) e->mergeContacts = e->pairRuns = false;  // the lists come from the walk from now on
     if ((status & ST_MODE_CHANGE) && d.fluidTiles) {
         // a particle left the domain: the lists come from the reference's walk
         // (the list kernels) from now on
@@ -612,6 +692,26 @@ void grow(demsph_engine* e, int status)
     }
     CK(cudaMemsetAsync(d.status, 0, sizeof(int), e->stream));
     dropGraph(e);
+}
+
+// A step failed with status `st` after the steps before it completed (e->par is
+// their last list's parity).  Where the last of them ran on contact pairs, its
+// springs go back into the lists of that parity, which the retry reads.  runs:
+// the first step and length of each fused run.
+void closePairs(demsph_engine* e, const std::vector<std::pair<int, int>>& runs, int step, int st)
+{
+    DeviceState& d = e->d;
+    bool onPairs = false;
+    for (const auto& r : runs) onPairs |= pairRun(e, r.second) && step >= r.first + 2 && step < r.first + r.second;
+    if (!onPairs) return;
+    const bool old = st & ST_VERLET_OVERFLOW;  // the failed step had begun to rebuild the candidates
+    int most = 0;
+    launchPairsCount(d, old, e->stream);
+    CK(cudaMemcpyAsync(&most, d.need, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    CK(cudaStreamSynchronize(e->stream));
+    if (most > d.scap) grow(e, ST_SS_OVERFLOW);
+    launchPairsClose(d, e->par, old, e->stream);
+    e->walkOrder[e->par] = false;
 }
 
 constexpr int ALL_OVERFLOWS = ST_FF_OVERFLOW | ST_FS_OVERFLOW | ST_SS_OVERFLOW | ST_COUPLE_OVERFLOW |
@@ -992,6 +1092,7 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
             d.vcap = 2 * perParticle;
             d.vcand = dalloc<int>((size_t)d.vcap * nr, e->owned, e->stream, false);
             d.vcnt = dalloc<int>(nr, e->owned, e->stream);
+            d.pairSprings = contactSprings(sc);
             d.vref = dalloc<float4>(ns, e->owned, e->stream);
             d.svref = dalloc<float4>(ns, e->owned, e->stream);
             d.rebuild = dalloc<int>(2, e->owned, e->stream);
@@ -1011,6 +1112,12 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
             {
                 const char* v = std::getenv("DEMSPH_FUSE_INTEGRATION");
                 e->fuseIntegration = !(v && v[0] == '0');
+            }
+            {
+                const char* v = std::getenv("DEMSPH_PAIR_RUNS");
+                e->pairRuns = !(v && v[0] == '0') && e->fuseIntegration && o.solid_verlet_skin >= 0 && d.grid.gx >= 3 &&
+                              d.grid.gy >= 3 && d.grid.gz >= 3 && (e->nMassive > 0 || e->movingDummies > 0);
+                allocPairs(e);
             }
             d.forceRows = o.contact_rows_per_warp > 0 ? o.contact_rows_per_warp : 32;
             e->adaptRows = o.contact_rows_per_warp == 0;
@@ -1332,12 +1439,22 @@ static int stepKind(const DeviceState& d, int i, int gap)
     return (i % gap == 0 ? 1 : 0) | (i % (5 * gap) == 0 ? 2 : 0);
 }
 
+// Steps of a graph, and graphs kept: a graph's first and last step cost about
+// twice the others, and instantiating one about 5 us per launch.
+constexpr int MAX_GRAPH_STEPS = 32;
+constexpr size_t MAX_GRAPHS = 64;
+
 // The graph of `length` steps of `kind` starting from the current parity,
 // captured on first use.
 static const demsph_engine::CachedGraph& graphFor(demsph_engine* e, int kind, int length, double dt, int step, int gap)
 {
     for (const auto& g : e->graphs)
         if (g.kind == kind && g.parity == e->par && g.length == length) return g;
+    if (e->graphs.size() >= MAX_GRAPHS) {  // runs of ever new lengths: the oldest goes
+        CK(cudaStreamSynchronize(e->stream));
+        cudaGraphExecDestroy(e->graphs.front().exec);
+        e->graphs.erase(e->graphs.begin());
+    }
     const int parity = e->par;
     cudaGraph_t g;
     const long long before = t_kernelLaunches;
@@ -1419,13 +1536,14 @@ static int runUpdate(demsph_engine* e, double dt, int first_step, int n_steps, i
                 e->resumeOpened = false;
                 continue;
             }
-            // a run of plain DEM steps replays 10- and 2-step graphs (parity
-            // unchanged), an odd last step or a fluid step a 1-step graph
+            // a run of plain DEM steps replays one graph of its length, longer
+            // ones in parts (the first and last step of a part build contact
+            // lists), a fluid step a 1-step graph
             int run = 1;
             if (kind == 0)
                 while (s + run < end && stepKind(d, s + run, gap) == 0) ++run;
             while (run > 0) {
-                const int len = kind != 0 ? 1 : (run >= 10 ? 10 : (run >= 2 ? 2 : 1));
+                const int len = kind != 0 ? 1 : std::min(run, MAX_GRAPH_STEPS);
                 bool fusedRun;
                 if (eagerFused) {
                     fusedRun = e->fuseIntegration && kind == 0 && len >= 2;
@@ -1475,6 +1593,7 @@ static int runUpdate(demsph_engine* e, double dt, int first_step, int n_steps, i
             if (step > r.first && step < r.first + r.second) e->resumeOpened = true;
         if (e->resumeOpened) ++e->runStats.resumed_steps;
         ++e->runStats.list_growths;
+        closePairs(e, fusedRuns, step, st);
         grow(e, st);
     }
     if (afterSteps && n_steps == 0) {
@@ -1632,7 +1751,7 @@ long long demsph_estimate_bytes(const demsph_scene* sc, const demsph_options* op
     // list parities, springs in and out, candidates; per cell: counts and starts
     const long long kvf = kff + kff / 2, kvs = kfs + kfs / 2;
     return nf * (444 + 4 * (kff + kfs) + 4 * (kvf + kvs) + 64) + ns * (248 + 48LL * sc->n_wall) +
-           rows * (72 + slots * 184 + 2 * slots * 4) + (cells + 1) * 16 + (long long)sc->n_clump * 160 +
+           rows * (80 + slots * 184 + 2 * slots * 4 + 2 * slots * (58 + 32 * contactSprings(sc))) + (cells + 1) * 16 + (long long)sc->n_clump * 160 +
            std::min(64 * rows + 1024, std::max(1LL, kfs * nf)) * 4 + (1 << 20);
 }
 
@@ -1658,7 +1777,7 @@ int demsph_profile_report(demsph_engine* e, char* buf, int cap)
     std::vector<std::pair<int, double>> acc;
     for (auto& t : e->timed) {
         float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, t.a, t.b));
+        if (t.a) CK(cudaEventElapsedTime(&ms, t.a, t.b));
         size_t k = 0;
         while (k < order.size() && order[k] != t.tag) ++k;
         if (k == order.size()) {
@@ -1667,6 +1786,7 @@ int demsph_profile_report(demsph_engine* e, char* buf, int cap)
         }
         acc[k].first += 1;
         acc[k].second += ms;
+        if (!t.a) continue;
         cudaEventDestroy(t.a);
         cudaEventDestroy(t.b);
     }
@@ -2000,6 +2120,9 @@ int demsph_batch_update(demsph_batch* b, demsph_engine* const* engines, int coun
                 if (step > first + fr.first && step < first + fr.first + fr.second) e->resumeOpened = true;
             if (e->resumeOpened) ++e->runStats.resumed_steps;
             ++e->runStats.list_growths;
+            std::vector<std::pair<int, int>> runs;
+            for (const auto& fr : mb.r->fusedRuns) runs.emplace_back(first + fr.first, fr.second);
+            closePairs(e, runs, step, st);
             grow(e, st);
             status_out[i] = runUpdate(e, dt[i], step, first + n - step, g, 1, nullptr);
         } catch (const CudaError& c) {

@@ -85,6 +85,11 @@ struct demsph_engine {
     // lists come from candidates (DEMSPH_MERGE_CONTACTS=0 keeps two launches;
     // off for good once the lists come from the walk).
     bool mergeContacts = true;
+    // Runs of three or more plain DEM steps evaluate the contact candidates as
+    // pairs between their first and last step, without contact lists
+    // (DEMSPH_PAIR_RUNS=0 keeps the lists; off for good once the lists come from
+    // the walk).
+    bool pairRuns = true;
     // The per-solid sums run the solids' integration pass in the same launch
     // when the integrated solids are exactly the contact rows
     // (DEMSPH_FOLD_INTEGRATION=0 keeps the separate pass).

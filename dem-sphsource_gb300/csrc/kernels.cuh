@@ -335,6 +335,23 @@ struct DeviceState {
     int* dummyIdx;
     unsigned char* dummyMoving;
     int* moveChanged;
+    // ---- contact pairs of runs of plain DEM steps (dem.cu) ----
+    // A forward candidate (A, B), B > A, of the Verlet rows is a pair slot
+    // [q * nrow + row of A], q its rank among A's forward candidates; its
+    // springs and results stay there until the candidates are rebuilt.
+    int pairSprings;         // springs kept per pair: 1 (sliding) where no material has rolling or torsion friction, else 3
+    int* pfirst;             // per row: its candidates below its own solid (the reverse ones come first)
+    int* plink;              // reverse candidate k of row r: the pair's slot, at [k * nrow + r]
+    unsigned char* pflag;    // per slot, of the last step: PAIR_OUT, PAIR_LISTED or PAIR_LIVE
+    float4* pspring[3];      // springs after the last step (valid while PAIR_LIVE)
+    float4* pforce;          // force on A (while PAIR_LIVE)
+    float4* ptorqueA;        // torque on A and on B of the pair's contact, with its lever arms
+    float4* ptorqueB;
+    // the history as it was before the last rebuild of the candidates
+    int* oldCount;           // forward candidates of each row
+    int* oldId;              // their solids, flags and springs, by slot
+    unsigned char* oldFlag;
+    float4* oldSpring[3];
     int* need;               // [0] most contacts of a row, [1] most candidates of a row,
                              // [2] / [3] most fluid / solid candidates of a fluid particle,
                              // [4] most walk candidates of a fluid particle in tile mode (for growing)
@@ -494,7 +511,8 @@ void launchBitsToLists(const DeviceState& d, cudaStream_t s);
 // The contact rows of the step, each row first rebuilding its candidates when
 // they are stale (launchContactDetect; forceWalk: from the reference's 27-cell
 // walk, in the reference's order).
-void launchContactDetect(const DeviceState& d, int parity, bool forceWalk, cudaStream_t s);
+// fromPairs: the springs come from the contact pairs' slots, not the previous list.
+void launchContactDetect(const DeviceState& d, int parity, bool forceWalk, cudaStream_t s, bool fromPairs = false);
 // Contact items over a sample of rows, into rowStats.
 void launchRowStats(const DeviceState& d, int parity, cudaStream_t s);
 int launchBondFlags(const DeviceState& d, int parity, int* flag, int* pos, int* work, cudaStream_t s);
@@ -525,6 +543,26 @@ void launchPairForces(const DeviceState& d, int parity, float dt, cudaStream_t s
 // countStep as launchSolidIntegrate's.
 void launchSolidForces(const DeviceState& d, int parity, double dt, cudaStream_t s, int integrate = -1,
                        bool countStep = false);
+// ---- runs of plain DEM steps on contact pairs ----
+// Between the first and the last step of a run no contact list is built: the
+// forward candidates themselves are the pairs, each with its springs in a slot
+// of its own.  launchPairsOpen fills the slots from the list of the run's first
+// step; launchPairsRebuild (every later step) rebuilds stale candidates and
+// carries the springs over; launchPairStep evaluates the pairs of the step (and
+// the bonds); launchPairSums sums them per solid as launchSolidForces does.  The
+// last step builds its list as always, its springs taken from the slots
+// (launchContactDetect's fromPairs).
+enum PairFlag { PAIR_OUT = 0, PAIR_LISTED = 1, PAIR_LIVE = 2 };
+void launchPairsOpen(const DeviceState& d, int parity, cudaStream_t s);
+void launchPairsRebuild(const DeviceState& d, int parity, cudaStream_t s);
+void launchPairStep(const DeviceState& d, int parity, float dt, cudaStream_t s);
+void launchPairSums(const DeviceState& d, int parity, double dt, cudaStream_t s, int integrate, bool countStep);
+// The pairs' springs back into the list arrays of `parity` (a run that ended
+// early); old: as they were before the last rebuild.  Most live pairs of a row
+// first: launchPairsCount raises need[0] to it.
+void launchPairsCount(const DeviceState& d, bool old, cudaStream_t s);
+void launchPairsClose(const DeviceState& d, int parity, bool old, cudaStream_t s);
+
 // The contact list of a plain DEM step opened by a fused integration pass and
 // its contact forces in one launch (no bonds; candidates, not the walk):
 // each row filters its candidates on the end-of-step offsets (sphE/splE) and

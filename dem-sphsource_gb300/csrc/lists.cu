@@ -821,10 +821,35 @@ __global__ void kCoupSort(DeviceState d)
 // stays in walk order: bonds are numbered in it.
 // The spring history of the forward pairs q = first, first + step, ... of row
 // r from the previous list (the pair's springs there, or zeros).
-__device__ __forceinline__ void remapSprings(const DeviceState& d, int par, int r, int nf, int first, int step)
+__device__ __forceinline__ void remapSprings(const DeviceState& d, int par, int r, int nf, int first, int step,
+                                             int fromPairs)
 {
     const int prev = par ^ 1;
     const size_t nr = (size_t)d.nrow;
+    if (fromPairs) {  // the springs are in the candidates' slots
+        const int vf = d.pfirst[r], forward = min(d.vcnt[r], d.vcap) - vf;
+        for (int q = first; q < nf; q += step) {
+            const size_t slot = (size_t)q * nr + r;
+            const int b = d.fwd[par][slot];
+            float4 s0 = make_float4(0, 0, 0, 0), s1 = s0, s2 = s0;
+            for (int k = 0; k < forward; ++k) {
+                const size_t ps = (size_t)k * nr + r;
+                if (d.vcand[ps + (size_t)vf * nr] != b) continue;
+                if (d.pflag[ps] == PAIR_LIVE) {
+                    s0 = d.pspring[0][ps];
+                    if (d.pairSprings == 3) {
+                        s1 = d.pspring[1][ps];
+                        s2 = d.pspring[2][ps];
+                    }
+                }
+                break;
+            }
+            d.springIn[0][slot] = s0;
+            d.springIn[1][slot] = s1;
+            d.springIn[2][slot] = s2;
+        }
+        return;
+    }
     const int prevCnt = min(d.fcnt[prev][r], d.scap);
     for (int q = first; q < nf; q += step) {
         const size_t slot = (size_t)q * nr + r;
@@ -845,7 +870,7 @@ __device__ __forceinline__ void remapSprings(const DeviceState& d, int par, int 
     }
 }
 
-__device__ __forceinline__ void detectRow(const DeviceState& d, int par, int forceWalk, bool walk, int r)
+__device__ __forceinline__ void detectRow(const DeviceState& d, int par, int forceWalk, bool walk, int r, int fromPairs)
 {
     // stale candidates are rebuilt first, row by row (the contact force
     // kernel clears the flag once every row has read it)
@@ -892,7 +917,7 @@ __device__ __forceinline__ void detectRow(const DeviceState& d, int par, int for
         sortSlots(d.rev, r, d.nrow, nb);
     }
     for (int q = 0; q < nb; ++q) d.revF[(size_t)q * nr + r].w = 0.f;  // until a forward row's pair force writes it
-    remapSprings(d, par, r, nf, 0, 1);
+    remapSprings(d, par, r, nf, 0, 1, fromPairs);
 }
 
 
@@ -903,7 +928,7 @@ __device__ __forceinline__ void detectRow(const DeviceState& d, int par, int for
 // left the domain) and stale candidates (their rebuild) run on the row's
 // first lane.
 template <int L>
-__global__ void __launch_bounds__(T) kContactDetect(DeviceState d, int par, int forceWalk)
+__global__ void __launch_bounds__(T) kContactDetect(DeviceState d, int par, int forceWalk, int fromPairs)
 {
     stepKernelBegin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -912,7 +937,7 @@ __global__ void __launch_bounds__(T) kContactDetect(DeviceState d, int par, int 
     const bool live = r < d.nrow;
     const bool walk = forceWalk || *d.slowMode;
     if (L == 1 || walk) {
-        if (live && lane == 0) detectRow(d, par, forceWalk, walk, r);
+        if (live && lane == 0) detectRow(d, par, forceWalk, walk, r, fromPairs);
         return;
     }
     // stale candidates are rebuilt first (the contact force kernel clears the
@@ -968,7 +993,7 @@ __global__ void __launch_bounds__(T) kContactDetect(DeviceState d, int par, int 
         }
         return;
     }
-    remapSprings(d, par, r, nf, lane, L);
+    remapSprings(d, par, r, nf, lane, L, fromPairs);
 }
 
 // Contact items (forward and reverse contacts, bonds) per row over at most
@@ -1195,15 +1220,15 @@ void launchCouplingLists(const DeviceState& d, cudaStream_t s)
     launchStep(kCoupSort, blocksFor(d.ns, 256), 256, s, d);
 }
 
-void launchContactDetect(const DeviceState& d, int par, bool forceWalk, cudaStream_t s)
+void launchContactDetect(const DeviceState& d, int par, bool forceWalk, cudaStream_t s, bool fromPairs)
 {
     if (d.nrow <= 0) return;
     // rows holding many contacts and bonds (the force kernel's rows per warp
     // adapted down to 16 or fewer) have many candidates: four lanes per row
     if (d.forceRows <= 16)
-        launchStep(kContactDetect<4>, blocksFor((long long)d.nrow * 4, T), T, s, d, par, forceWalk ? 1 : 0);
+        launchStep(kContactDetect<4>, blocksFor((long long)d.nrow * 4, T), T, s, d, par, forceWalk ? 1 : 0, fromPairs ? 1 : 0);
     else
-        launchStep(kContactDetect<1>, blocksFor(d.nrow, T), T, s, d, par, forceWalk ? 1 : 0);
+        launchStep(kContactDetect<1>, blocksFor(d.nrow, T), T, s, d, par, forceWalk ? 1 : 0, fromPairs ? 1 : 0);
 }
 
 void launchRowStats(const DeviceState& d, int par, cudaStream_t s)
