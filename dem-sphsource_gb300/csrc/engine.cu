@@ -688,7 +688,17 @@ void grow(demsph_engine* e, int status)
     if (status & ST_MODE_CHANGE) {
         // the abandoned step may have counted some particles into cells
         CK(cudaMemsetAsync(d.scellCount, 0, sizeof(int) * d.grid.num, e->stream));
-        if (d.nf > 0) CK(cudaMemsetAsync(d.fcellCount, 0, sizeof(int) * d.grid.num, e->stream));
+        if (d.nf > 0) {
+            CK(cudaMemsetAsync(d.fcellCount, 0, sizeof(int) * d.grid.num, e->stream));
+            int slow = FSLOW_OFF;
+            CK(cudaMemcpyAsync(&slow, d.fslowMode, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+            CK(cudaStreamSynchronize(e->stream));
+            if (slow == FSLOW_RAISED) {
+                slow = FSLOW_ON;
+                CK(cudaMemcpyAsync(d.fslowMode, &slow, sizeof(int), cudaMemcpyHostToDevice, e->stream));
+                CK(cudaStreamSynchronize(e->stream));
+            }
+        }
     }
     CK(cudaMemsetAsync(d.status, 0, sizeof(int), e->stream));
     dropGraph(e);

@@ -168,6 +168,7 @@ struct demsph_engine {
         swap(movingDummies, o.movingDummies);
         swap(fuseIntegration, o.fuseIntegration);
         swap(mergeContacts, o.mergeContacts);
+        swap(pairRuns, o.pairRuns);
         swap(foldIntegration, o.foldIntegration);
         swap(resumeOpened, o.resumeOpened);
         swap(keysAdvanced, o.keysAdvanced);
@@ -194,6 +195,7 @@ struct demsph_engine {
     ~demsph_engine()
     {
         for (auto& t : timed) {
+            if (!t.a) continue;  // a counted stage (no events)
             cudaEventDestroy(t.a);
             cudaEventDestroy(t.b);
         }

@@ -40,7 +40,7 @@ __device__ __forceinline__ void fluidHashOne(const DeviceState& d, int i, const 
     if (key == d.grid.num - 1 && !*d.fslowMode) {
         // a fluid particle left the domain: from now on its lists come from the
         // reference's walk (which reaches it through the overflow cell); redo the step
-        *(volatile int*)d.fslowMode = 1;
+        *(volatile int*)d.fslowMode = FSLOW_RAISED;
         atomicOr(d.status, ST_MODE_CHANGE);
     }
     if (!sortNow.active()) {
@@ -191,16 +191,20 @@ __global__ void __launch_bounds__(SORT_THREADS) kSolidSortCoop(DeviceState d, Ru
 
 // The fluid hash of a fluid step and, when the fluids are reordered, the
 // reorder (scan of the counts, scatter, stable gather) in ONE cooperative
-// launch.  Whether to reorder is decided after the hash, from flags and a
-// status no later phase changes: a fluid leaving the domain in the hash sets
-// the status (the step is redone) and every block returns.
+// launch.  The decisions before the first barrier are the same in every block,
+// whenever it starts: the hash of this launch may set ST_MODE_CHANGE and
+// FSLOW_RAISED (a fluid left the domain: the step is redone), and neither is
+// looked at before the barrier.  Without a reorder the hash is all, and no block
+// waits for another.
 __global__ void __launch_bounds__(SORT_THREADS) kFluidReorderCoop(DeviceState d, RunIf when)
 {
     stepKernelBegin();
-    if (*d.status) return;
+    if (*(volatile int*)d.status & ~ST_MODE_CHANGE) return;
     unsigned gen = ((volatile unsigned*)d.gridBar)[1];
     const int stride = gridDim.x * blockDim.x;
+    const bool reorder = when.always || *d.frebuild || *(volatile int*)d.fslowMode == FSLOW_ON;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nf; i += stride) fluidHashOne(d, i, when);
+    if (!reorder) return;
     if (!gridBarrier(d.gridBar, gen, d.status)) return;
     if (*(volatile int*)d.status || !when.active()) return;
     if (!cooperativeScan(d.fcellCount, d.fcellStart, d.grid.num, d.scanWork, d.gridBar, gen, d.status)) return;

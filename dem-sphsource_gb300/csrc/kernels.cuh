@@ -164,6 +164,10 @@ inline void launchStepSmem(void (*kernel)(KArgs...), unsigned grid, unsigned blo
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Values of fslowMode: raised by a fluid hash (with ST_MODE_CHANGE; the host turns
+// it into FSLOW_ON before the step is redone).
+enum FluidSlowMode { FSLOW_OFF = 0, FSLOW_ON = 1, FSLOW_RAISED = 2 };
+
 // A fluid partner in one sector: position offset and packed cell (packCell),
 // velocity and density difference.
 struct alignas(32) FluidRec {
@@ -230,7 +234,7 @@ struct DeviceState {
     float fskin;
     float fhmax;             // largest fluid smoothing length
     int* frebuild;           // 1: fluid candidates are stale (a fluid or solid moved fskin / 2)
-    int* fslowMode;          // 1: fluid lists from the 27-cell walk every fluid step
+    int* fslowMode;          // not 0 (FSLOW_ON): fluid lists from the 27-cell walk every fluid step
     // Membership bits (sph_tiles.cu, opt-in): with fluidTiles set the fluids
     // are sorted by cell every fluid step and list membership is kept as one
     // bit per candidate of each particle's 27-cell walk ([w * nf + i], kbits
