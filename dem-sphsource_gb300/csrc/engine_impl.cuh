@@ -41,6 +41,11 @@ inline T* dalloc(size_t n, std::vector<Allocation>& owned, cudaStream_t s, bool 
     return p;
 }
 
+// Two pinned words of a process-wide slab for the status read of one engine
+// (null when all are in use: the read then goes through pageable memory).
+int2* takeStatusSlot();
+void releaseStatusSlot(int2* slot);
+
 }  // namespace demsph
 
 struct demsph_engine {
@@ -135,6 +140,10 @@ struct demsph_engine {
     // demsph_update_io moves them on the second stream
     double* dscratch[2] = {nullptr, nullptr};
     size_t dscratchN[2] = {0, 0};
+    // Where the status and the step count are copied (pinned; statusSlot), and
+    // the step count as last read: the device's only grows.
+    int2* statusHost = nullptr;
+    int stepsSeen = 0;
 
     // Exchanges everything two engines hold (device memory, stream, graphs,
     // state), field by field: demsph_append hands the caller's handle the
@@ -190,6 +199,8 @@ struct demsph_engine {
         swap(dscratch[1], o.dscratch[1]);
         swap(dscratchN[0], o.dscratchN[0]);
         swap(dscratchN[1], o.dscratchN[1]);
+        swap(statusHost, o.statusHost);
+        swap(stepsSeen, o.stepsSeen);
     }
 
     ~demsph_engine()
@@ -212,6 +223,7 @@ struct demsph_engine {
             cudaStreamSynchronize(stream);
             cudaStreamDestroy(stream);
         }
+        demsph::releaseStatusSlot(statusHost);
     }
 };
 

@@ -183,7 +183,7 @@ struct DeviceState {
     Tables tab;
     int fixes;
     int* status;             // StatusBits, sticky until the host clears it
-    int* stepsDone;          // steps completed since the last reset
+    int* stepsDone;          // steps completed (next to status)
     int* scanWork;
 
     // ---- fluid (slots in cell order) ----
