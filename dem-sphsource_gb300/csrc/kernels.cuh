@@ -641,8 +641,9 @@ __device__ __forceinline__ void checkDisplacement(const DeviceState& d, int* sta
 // rehashSolidTo leaves the renormalised offset in h, l and stores it to
 // outH, outL (sph, spl; sphE, splE when the next step's first half is
 // integrated in the same pass).
+// key0, centre0: its key and centre before.
 __device__ __forceinline__ void rehashSolidTo(const DeviceState& d, int i, int row, int4 c, float4& h, float4& l,
-                                              float4* outH, float4* outL)
+                                              float4* outH, float4* outL, int key0, int4 centre0)
 {
     renormAxis(c.x, h.x, l.x, d.grid.csx);
     renormAxis(c.y, h.y, l.y, d.grid.csy);
@@ -652,13 +653,20 @@ __device__ __forceinline__ void rehashSolidTo(const DeviceState& d, int i, int r
     d.scell[i] = c;
     outH[i] = h;
     outL[i] = l;
-    d.skeySearch[i] = d.skey[i];
+    d.skeySearch[i] = key0;
     d.skey[i] = key;
     if (row >= 0) {
-        d.scentreSearch[row] = d.scentre[row];
+        d.scentreSearch[row] = centre0;
         d.scentre[row] = make_int4(truncAxis(c.x, h.x, l.x), truncAxis(c.y, h.y, l.y), truncAxis(c.z, h.z, l.z), 0);
         if (key == d.grid.num - 1) *(volatile int*)d.slowMode = 1;
     }
+}
+__device__ __forceinline__ void rehashSolidTo(const DeviceState& d, int i, int row, int4 c, float4& h, float4& l,
+                                              float4* outH, float4* outL)
+{
+    const int key0 = d.skey[i];
+    const int4 centre0 = row >= 0 ? d.scentre[row] : make_int4(0, 0, 0, 0);
+    rehashSolidTo(d, i, row, c, h, l, outH, outL, key0, centre0);
 }
 __device__ __forceinline__ void rehashSolidOf(const DeviceState& d, int i, int row, int4 c, float4 h, float4 l)
 {
