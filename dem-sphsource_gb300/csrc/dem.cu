@@ -774,29 +774,30 @@ __device__ __forceinline__ int reverseCandidates(const DeviceState& d, int r, in
     return v;
 }
 
-// The slots of row r's reverse pairs, in the rows of the lower solids (a pair's
-// two candidates are each other's: the test is symmetric).
-__device__ __forceinline__ void linkRow(const DeviceState& d, int r, int a, int reverse)
+// The first of row r's n candidates (in index order) that is not below b.
+__device__ __forceinline__ int firstNotBelow(const DeviceState& d, int r, int n, int b)
+{
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int m = (lo + hi) >> 1;
+        if (d.vcand[(size_t)m * d.nrow + r] < b) lo = m + 1;
+        else hi = m;
+    }
+    return lo;
+}
+// The slot of row r's reverse pair k (its solid a), in the row of the lower
+// solid (a pair's two candidates are each other's: the test is symmetric).
+__device__ __forceinline__ void linkPair(const DeviceState& d, int r, int a, int k)
 {
     const size_t nr = (size_t)d.nrow;
-    for (int k = 0; k < reverse; ++k) {
-        const int A = d.vcand[(size_t)k * nr + r];
-        const int ra = rowOf(d, A);
-        int link = -1;
-        if (ra >= 0) {
-            const int n = min(d.vcnt[ra], d.vcap);
-            int q = 0;  // forward rank
-            for (int m = 0; m < n; ++m) {
-                const int b = d.vcand[(size_t)m * nr + ra];
-                if (b == a) {
-                    link = (int)((size_t)q * nr + ra);
-                    break;
-                }
-                q += b > A ? 1 : 0;
-            }
-        }
-        d.plink[(size_t)k * nr + r] = link;
+    const int A = d.vcand[(size_t)k * nr + r];
+    const int ra = rowOf(d, A);
+    int link = -1;
+    if (ra >= 0) {
+        const int n = min(d.vcnt[ra], d.vcap), m = firstNotBelow(d, ra, n, a);
+        if (m < n && d.vcand[(size_t)m * nr + ra] == a) link = (int)((size_t)(m - firstNotBelow(d, ra, n, A)) * nr + ra);
     }
+    d.plink[(size_t)k * nr + r] = link;
 }
 
 // After the first step of a run: every forward candidate's slot from the
@@ -820,58 +821,209 @@ __global__ void __launch_bounds__(T) kPairsOpen(DeviceState d, int par)
             for (int j = 0; j < d.pairSprings; ++j) d.pspring[j][slot] = d.springOut[par][j][(size_t)m * nr + r];
         d.pflag[slot] = in ? PAIR_LIVE : PAIR_OUT;  // the springs of a listed pair without contact are zeros
     }
-    linkRow(d, r, a, vf);
+    for (int k = 0; k < vf; ++k) linkPair(d, r, a, k);
+}
+
+// The new candidates of row r by one lane, on the end-of-step offsets, with its
+// pairs' flags and springs carried over.
+__device__ __forceinline__ void rebuildRow(const DeviceState& d, const DeviceState& atEnd, int r)
+{
+    const size_t nr = (size_t)d.nrow;
+    const int a = solidOf(d, r);
+    const int vf0 = d.pfirst[r], old = min(d.vcnt[r], d.vcap) - vf0;
+    d.oldCount[r] = old;
+    for (int q = 0; q < old; ++q) {
+        const size_t slot = (size_t)q * nr + r;
+        d.oldId[slot] = d.vcand[(size_t)(vf0 + q) * nr + r];
+        const unsigned char f = d.pflag[slot];
+        d.oldFlag[slot] = f;
+        if (f == PAIR_LIVE)
+            for (int j = 0; j < d.pairSprings; ++j) d.oldSpring[j][slot] = d.pspring[j][slot];
+    }
+    verletBuildRow(atEnd, r);
+    const int n = min(d.vcnt[r], d.vcap), vf = reverseCandidates(d, r, a, n);
+    d.pfirst[r] = vf;
+    int m = 0;
+    for (int k = vf; k < n; ++k) {
+        const size_t slot = (size_t)(k - vf) * nr + r;
+        const int b = d.vcand[(size_t)k * nr + r];
+        while (m < old && d.oldId[(size_t)m * nr + r] < b) ++m;
+        const bool live = m < old && d.oldId[(size_t)m * nr + r] == b && d.oldFlag[(size_t)m * nr + r] == PAIR_LIVE;
+        if (live)
+            for (int j = 0; j < d.pairSprings; ++j) d.pspring[j][slot] = d.oldSpring[j][(size_t)m * nr + r];
+        d.pflag[slot] = live ? PAIR_LIVE : PAIR_OUT;
+    }
+}
+
+// The same by the ROW_LANES lanes of a row (whole warps; live false past the
+// last row).  One lane walks its cells, tests their members, sorts its list in
+// place and merges the old one as one chain of dependent reads, half the time
+// of a rebuild in a small scene.  Here the lanes take the rows of cells (each
+// one range of the sorted order), list their members in shared memory, test
+// them eight at a time, and each lane finds the place of its candidates by
+// counting those below.  A row with more than ROW_MEMBERS members in its cells
+// goes to its first lane.
+//
+// What bounds it: the latency of six barriers and some fifteen reads, of 25 us
+// on top of a step with 3k grains (116 by one lane a row).
+constexpr int ROW_LANES = 8, ROW_MEMBERS = 88;
+__device__ __forceinline__ void rebuildRowGroup(const DeviceState& d, const DeviceState& atEnd, int* mine, int r, bool live)
+{
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & (ROW_LANES - 1), shift = (threadIdx.x & 31) & ~(ROW_LANES - 1);
+    const unsigned below = (1u << lane) - 1u, group = (1u << ROW_LANES) - 1u;
+    const size_t nr = (size_t)d.nrow;
+    const GridDev& g = d.grid;
+    const int a = solidOf(d, live ? r : 0);
+    const int4 fa = d.sflags[a], ca = d.scell[a];
+    const float4 ha = atEnd.sph[a];
+    const float effA = d.srad[a].z, reach = effA + d.vmaxEff + d.skin;
+    // verletBuildRow's box
+    const int x0 = max(0, ca.x + (int)floorf((ha.x - reach) / g.cs.x)), x1 = min(g.gx - 1, ca.x + (int)floorf((ha.x + reach) / g.cs.x));
+    const int y0 = max(0, ca.y + (int)floorf((ha.y - reach) / g.cs.y)), y1 = min(g.gy - 1, ca.y + (int)floorf((ha.y + reach) / g.cs.y));
+    const int z0 = max(0, ca.z + (int)floorf((ha.z - reach) / g.cs.z)), z1 = min(g.gz - 1, ca.z + (int)floorf((ha.z + reach) / g.cs.z));
+    const int ny = max(1, y1 - y0 + 1);
+    const int rows = live && x0 <= x1 && y0 <= y1 && z0 <= z1 ? ny * (z1 - z0 + 1) : 0;
+    int total = 0;
+    for (int base = 0; __any_sync(FULL, base < rows); base += ROW_LANES) {
+        const int c = base + lane;
+        int p = 0, pe = 0;
+        if (c < rows) {
+            const int dz = c / ny, first = ((z0 + dz) * g.gy + y0 + c - dz * ny) * g.gx;
+            p = d.scellStart[first + x0];
+            pe = d.scellStart[first + x1 + 1];
+        }
+        int end = pe - p;  // inclusive scan over the lanes
+#pragma unroll
+        for (int o = 1; o < ROW_LANES; o <<= 1) {
+            const int y = __shfl_up_sync(FULL, end, o, ROW_LANES);
+            if (lane >= o) end += y;
+        }
+        int to = total + end - (pe - p);
+        for (; p < pe && to < ROW_MEMBERS; ++p, ++to) mine[to] = p;
+        total += __shfl_sync(FULL, end, ROW_LANES - 1, ROW_LANES);
+    }
+    __syncwarp();
+    const bool fits = total <= ROW_MEMBERS;
+    // the old list
+    const int vf0 = live && fits ? d.pfirst[r] : 0, old = live && fits ? min(d.vcnt[r], d.vcap) - vf0 : 0;
+    for (int q = lane; q < old; q += ROW_LANES) {
+        const size_t slot = (size_t)q * nr + r;
+        const unsigned char f = d.pflag[slot];
+        d.oldId[slot] = d.vcand[(size_t)(vf0 + q) * nr + r];
+        d.oldFlag[slot] = f;
+        if (f == PAIR_LIVE)
+            for (int j = 0; j < d.pairSprings; ++j) d.oldSpring[j][slot] = d.pspring[j][slot];
+    }
+    // the candidates, unsorted, over the members already read
+    int n = 0, low = 0;
+    const int count = fits ? total : 0;
+    for (int base = 0; __any_sync(FULL, base < count); base += 2 * ROW_LANES) {
+        int b[2];
+        bool in[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int e = base + u * ROW_LANES + lane;
+            b[u] = e < count ? d.ssorted[mine[e]] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            in[u] = false;
+            if (b[u] >= 0 && solidPairCandidate(d, a, fa, b[u])) {
+                const float3 rr = relF(ca, ha, d.scell[b[u]], atEnd.sph[b[u]], g);
+                const float c = (effA + d.srad[b[u]].z + d.skin) * 1.0001f;
+                in[u] = !(dot3(rr, rr) > c * c);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const unsigned m = (__ballot_sync(FULL, in[u]) >> shift) & group;
+            if (in[u]) mine[n + __popc(m & below)] = b[u];
+            n += __popc(m);
+            low += __popc((__ballot_sync(FULL, in[u] && b[u] < a) >> shift) & group);
+        }
+        __syncwarp();
+    }
+    // in index order
+    for (int k = lane; k < n; k += ROW_LANES) {
+        const int id = mine[k];
+        int place = 0;
+        for (int q = 0; q < n; ++q) place += mine[q] < id;
+        if (place < d.vcap) d.vcand[(size_t)place * nr + r] = id;
+    }
+    if (live && fits && lane == 0) {
+        d.oldCount[r] = old;
+        d.vcnt[r] = n;
+        d.pfirst[r] = min(low, min(n, d.vcap));
+        d.vref[a] = f4(gridPos(ca, ha, g));
+        if (n > d.vcap) {
+            atomicOr(d.status, ST_VERLET_OVERFLOW);
+            atomicMax(&d.need[1], n);
+        }
+    }
+    __syncwarp();
+    for (int k = low + lane; k < min(n, d.vcap); k += ROW_LANES) {
+        const size_t slot = (size_t)(k - low) * nr + r;
+        const int b = d.vcand[(size_t)k * nr + r];
+        int m = -1;
+        for (int q = 0; q < old; ++q)
+            if (d.oldId[(size_t)q * nr + r] == b) m = q;
+        const bool on = m >= 0 && d.oldFlag[(size_t)m * nr + r] == PAIR_LIVE;
+        if (on)
+            for (int j = 0; j < d.pairSprings; ++j) d.pspring[j][slot] = d.oldSpring[j][(size_t)m * nr + r];
+        d.pflag[slot] = on ? PAIR_LIVE : PAIR_OUT;
+    }
+    if (live && !fits && lane == 0) rebuildRow(d, atEnd, r);
 }
 
 // At the start of every later step of a run: nothing, or the rebuild of stale
 // candidates - the solids' sort by cell, each row's candidates on the
 // end-of-step offsets with its pairs' flags and springs carried over, then the
-// links - as phases of one cooperative launch.  In the walk mode the run cannot
+// links - as phases of one launch.  In the walk mode the run cannot
 // go on: ST_SPLIT_CONTACTS, before anything is written.
-__global__ void __launch_bounds__(SORT_THREADS) kPairsRebuild(DeviceState d, int par)
+template <class Wait, bool ROWS_IN_GROUPS>
+__device__ __forceinline__ void pairsRebuild(const DeviceState& d, int par)
 {
-    stepKernelBegin();
-    if (*d.status) return;
-    if (*d.slowMode) {
+    // one read's latency, not three.  Uniform over the blocks: the status and
+    // the flag change below, once every block is past the barriers
+    const int status = *(volatile int*)d.status, slow = *(volatile int*)d.slowMode, stale = *(volatile int*)&d.rebuild[par];
+    if (status) return;
+    if (slow) {
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(d.status, ST_SPLIT_CONTACTS);
         return;
     }
-    if (!d.rebuild[par]) return;  // uniform: cleared below, once every block is past the barriers
-    unsigned gen = ((volatile unsigned*)d.gridBar)[1];
-    if (!solidSortPhases(d, gen)) return;
-    if (!gridBarrier(d.gridBar, gen, d.status)) return;
+    if (!stale) return;
+    Wait wait(d);
+    if (!solidSortPhases(d, wait)) return;
+    if (!wait()) return;
     const DeviceState atEnd = endView(d);
-    const size_t nr = (size_t)d.nrow;
-    const int stride = gridDim.x * blockDim.x;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < d.nrow; r += stride) {
-        const int a = solidOf(d, r);
-        const int vf0 = d.pfirst[r], old = min(d.vcnt[r], d.vcap) - vf0;
-        d.oldCount[r] = old;
-        for (int q = 0; q < old; ++q) {
-            const size_t slot = (size_t)q * nr + r;
-            d.oldId[slot] = d.vcand[(size_t)(vf0 + q) * nr + r];
-            const unsigned char f = d.pflag[slot];
-            d.oldFlag[slot] = f;
-            if (f == PAIR_LIVE)
-                for (int j = 0; j < d.pairSprings; ++j) d.oldSpring[j][slot] = d.pspring[j][slot];
-        }
-        verletBuildRow(atEnd, r);
-        const int n = min(d.vcnt[r], d.vcap), vf = reverseCandidates(d, r, a, n);
-        d.pfirst[r] = vf;
-        int m = 0;
-        for (int k = vf; k < n; ++k) {
-            const size_t slot = (size_t)(k - vf) * nr + r;
-            const int b = d.vcand[(size_t)k * nr + r];
-            while (m < old && d.oldId[(size_t)m * nr + r] < b) ++m;
-            const bool live = m < old && d.oldId[(size_t)m * nr + r] == b && d.oldFlag[(size_t)m * nr + r] == PAIR_LIVE;
-            if (live)
-                for (int j = 0; j < d.pairSprings; ++j) d.pspring[j][slot] = d.oldSpring[j][(size_t)m * nr + r];
-            d.pflag[slot] = live ? PAIR_LIVE : PAIR_OUT;
-        }
+    const int lanes = ROWS_IN_GROUPS ? ROW_LANES : 1, stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (ROWS_IN_GROUPS) {
+        __shared__ int members[Wait::THREADS / ROW_LANES][ROW_MEMBERS];
+        for (int t = t0; (t & ~31) < d.nrow * ROW_LANES; t += stride)
+            rebuildRowGroup(d, atEnd, members[threadIdx.x / ROW_LANES], t / ROW_LANES, t / ROW_LANES < d.nrow);
+    } else {
+        for (int r = t0; r < d.nrow; r += stride) rebuildRow(d, atEnd, r);
     }
-    if (!gridBarrier(d.gridBar, gen, d.status)) return;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < d.nrow; r += stride) linkRow(d, r, solidOf(d, r), d.pfirst[r]);
+    if (!wait()) return;
+    for (int t = t0; t < d.nrow * lanes; t += stride) {
+        const int r = t / lanes, a = solidOf(d, r), reverse = d.pfirst[r];
+        for (int k = t % lanes; k < reverse; k += lanes) linkPair(d, r, a, k);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)&d.rebuild[par] = 0;
+}
+template <bool ROWS_IN_GROUPS>
+__global__ void __launch_bounds__(SORT_THREADS) kPairsRebuildCoop(DeviceState d, int par)
+{
+    stepKernelBegin();
+    pairsRebuild<GridWait, ROWS_IN_GROUPS>(d, par);
+}
+__global__ void __cluster_dims__(SORT_CLUSTER, 1, 1) __launch_bounds__(ClusterWait::THREADS, 1)
+    kPairsRebuildCluster(DeviceState d, int par)
+{
+    stepKernelBegin();
+    pairsRebuild<ClusterWait, true>(d, par);
 }
 
 // The pairs of a step, G lanes per row taking its forward candidates in turn
@@ -1563,7 +1715,19 @@ void launchPairsOpen(const DeviceState& d, int par, cudaStream_t s)
 }
 void launchPairsRebuild(const DeviceState& d, int par, cudaStream_t s)
 {
-    launchCooperative(kPairsRebuild, (unsigned)d.sortBlocks, SORT_THREADS, s, d, par);
+    // the cluster's threads are the lanes of 1024 rows: a step of 500 grains takes
+    // 15.4 us with it and 16.2 with the cooperative launch, of 3000 18.7 and 18.1
+    if (sortInCluster(d) && d.nrow <= SORT_CLUSTER * ClusterWait::THREADS / ROW_LANES)
+        launchStep(kPairsRebuildCluster, SORT_CLUSTER, ClusterWait::THREADS, s, d, par);
+    else if (d.nrow < 152 * 256)
+        // by the lanes of a row: a step that rebuilds takes 46 us instead of 134
+        // with 3k grains, 52 instead of 135 with 8k, 95 instead of 155 with 40k,
+        // 180 instead of 185 with 120k
+        launchCooperative(kPairsRebuildCoop<true>,
+                          (unsigned)std::min(d.wideBlocks, std::max(d.sortBlocks, blocksFor((long long)d.nrow * ROW_LANES, SORT_THREADS))),
+                          SORT_THREADS, s, d, par);
+    else
+        launchCooperative(kPairsRebuildCoop<false>, (unsigned)d.sortBlocks, SORT_THREADS, s, d, par);
 }
 #ifndef DEMSPH_PAIR_LANES
 #define DEMSPH_PAIR_LANES 0  // 0: the rule below

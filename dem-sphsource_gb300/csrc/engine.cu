@@ -1166,8 +1166,9 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
                 // at most two blocks per SM, and no more than two elements per
                 // thread need: small scenes leave the GPU to the others
                 const long long n = std::max<long long>(d.nf, ns);
+                d.wideBlocks = cooperativeSortBlocks();
                 d.sortBlocks = (v && v[0] == '0') ? 0
-                                                 : (int)std::min<long long>(cooperativeSortBlocks(),
+                                                 : (int)std::min<long long>(d.wideBlocks,
                                                                             std::max<long long>(1, (n + 511) / 512));
             }
             {

@@ -177,16 +177,27 @@ __global__ void kSolidRank(DeviceState d, RunIf when)
 
 // The sort by cell of a step in ONE launch (keys from the last integration):
 // the slots in the cells, the scan of the counts, the scatter and the stable
-// rank of kSolidSlots, scanExclusive, kScatter and kSolidRank, as phases of a
-// cooperative launch separated by grid barriers.  Steps that do not sort pay
-// one launch that returns at once instead of four.
+// rank of kSolidSlots, scanExclusive, kScatter and kSolidRank, as phases
+// separated by barriers.  Steps that do not sort pay one launch that returns at
+// once instead of four.
+template <class Wait>
+__device__ __forceinline__ void solidSort(const DeviceState& d, RunIf when)
+{
+    // uniform over the blocks: no phase changes these flags or the status
+    if (*d.status || !when.active()) return;
+    Wait wait(d);
+    solidSortPhases(d, wait);
+}
 __global__ void __launch_bounds__(SORT_THREADS) kSolidSortCoop(DeviceState d, RunIf when)
 {
     stepKernelBegin();
-    // uniform over the blocks: no phase changes these flags or the status
-    if (*d.status || !when.active()) return;
-    unsigned gen = ((volatile unsigned*)d.gridBar)[1];
-    solidSortPhases(d, gen);
+    solidSort<GridWait>(d, when);
+}
+__global__ void __cluster_dims__(SORT_CLUSTER, 1, 1) __launch_bounds__(ClusterWait::THREADS, 1)
+    kSolidSortCluster(DeviceState d, RunIf when)
+{
+    stepKernelBegin();
+    solidSort<ClusterWait>(d, when);
 }
 
 // The fluid hash of a fluid step and, when the fluids are reordered, the
@@ -200,17 +211,17 @@ __global__ void __launch_bounds__(SORT_THREADS) kFluidReorderCoop(DeviceState d,
 {
     stepKernelBegin();
     if (*(volatile int*)d.status & ~ST_MODE_CHANGE) return;
-    unsigned gen = ((volatile unsigned*)d.gridBar)[1];
+    GridWait wait(d);
     const int stride = gridDim.x * blockDim.x;
     const bool reorder = when.always || *d.frebuild || *(volatile int*)d.fslowMode == FSLOW_ON;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nf; i += stride) fluidHashOne(d, i, when);
     if (!reorder) return;
-    if (!gridBarrier(d.gridBar, gen, d.status)) return;
+    if (!wait()) return;
     if (*(volatile int*)d.status || !when.active()) return;
-    if (!cooperativeScan(d.fcellCount, d.fcellStart, d.grid.num, d.scanWork, d.gridBar, gen, d.status)) return;
+    if (!cooperativeScan(d.fcellCount, d.fcellStart, d.grid.num, d.scanWork, wait)) return;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nf; i += stride)
         d.fsortTmp[d.fcellStart[d.fkey[i]] + d.fslotInCell[i]] = i;
-    if (!gridBarrier(d.gridBar, gen, d.status)) return;
+    if (!wait()) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < d.nf; p += stride) fluidGatherOne(d, p);
 }
 
@@ -310,6 +321,10 @@ void launchSolidHash(const DeviceState& d, bool force, bool fluidStep, int par, 
 void launchSolidSort(const DeviceState& d, bool force, bool fluidStep, int par, cudaStream_t s)
 {
     if (d.ns <= 0) return;
+    if (!force && d.sortBlocks > 0 && sortInCluster(d)) {
+        launchStep(kSolidSortCluster, SORT_CLUSTER, ClusterWait::THREADS, s, d, solidSortWhen(d, force, fluidStep, par));
+        return;
+    }
     if (!force && d.sortBlocks > 0) {
         // the slots were not taken by launchSolidHash: the cooperative launch does everything
         launchCooperative(kSolidSortCoop, (unsigned)d.sortBlocks, SORT_THREADS, s, d,

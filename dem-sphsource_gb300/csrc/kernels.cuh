@@ -366,6 +366,7 @@ struct DeviceState {
     int* rowStats;           // [0] contact items, [1] rows, over a sample of rows
     unsigned* gridBar;       // [2]: grid barrier of the cooperative sort (arrivals, generation)
     int sortBlocks;          // blocks of the cooperative sort (0: the four-launch sort)
+    int wideBlocks;          // the most blocks of a cooperative launch
 
     // ---- infinite walls ----
     int nw;
