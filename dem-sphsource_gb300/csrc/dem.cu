@@ -17,6 +17,7 @@
 #include "cell_sort.cuh"
 #include "kernels.cuh"
 #include "contact_rows.cuh"
+#include "sph_common.cuh"
 #include "warp_items.cuh"
 
 namespace demsph {
@@ -746,6 +747,66 @@ __global__ void __launch_bounds__(T, 6) kContactForces(DeviceState d, int par, f
     solidRowTail(d, par, a, F, Tq, withCoupling, dt);
 }
 
+// ---- coupling force, per massive solid: sum over its fluid partners of
+// m_i x (solid term of momentum) (integrate.cu:282-330, gathered per solid
+// as calSolidForceTorque does through fluidSolidRange, :847-854) ----
+__device__ __forceinline__ float3 couplingPairForce(const DeviceState& d, int src, int i, int a, bool& inside)
+{
+    using namespace sph;
+    const Self o = loadSelf(d, i, src, 0, src);
+    const SolidPartner s = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, o.cs * o.cs, a);
+    inside = s.inside;
+    if (!s.inside) return make_float3(0.f, 0.f, 0.f);
+    const float3 via = o.v - s.v;
+    const float dU = -2.f * dot3(via, xyz(d.snormal[a]));
+    const float beta = fminf(3.f * fmaxf(dU, 0.f), o.cs);
+    const float Ps = (o.rho * s.Pa + s.rhoa * o.P + o.rho * s.rhoa * beta * dU) / (o.rho + s.rhoa);
+    return (s.r * Ps - via * (2.f * o.gam)) * (2.f * o.V * s.Va * s.G);
+}
+
+// Only contact rows can hold solids with mass, the only solids with fluid
+// partners here (the coupling lists take no others); L lanes of a row take
+// its partners in turn, each Kahan-summing its share, and the shares are
+// added in a fixed tree (groupSum).
+constexpr int COUPLING_LANES = 8;  // rows hold tens of fluid partners
+__device__ __forceinline__ void couplingRow(const DeviceState& d, int src, int t)
+{
+    constexpr int L = COUPLING_LANES;
+    if ((t & ~31) >= d.nrow * L) return;  // whole warps: the group sums shuffle
+    const int row = t / L, lane = t % L;
+    const bool live = row < d.nrow;
+    const int a = live ? solidOf(d, row) : 0;
+    KahanF3 f;
+    if (live)
+        for (int p = d.coupStart[a] + lane, e = d.coupStart[a + 1]; p < e; p += L) {
+            bool inside;
+            const float3 fi = couplingPairForce(d, src, d.coupList[p], a, inside);
+            if (inside) f.add(fi);
+        }
+    const float x = sph::groupSum<L>(f.x), y = sph::groupSum<L>(f.y), z = sph::groupSum<L>(f.z);
+    if (live && lane == 0) d.sfcoup[a] = make_float4(x, y, z, 0.f);
+}
+
+__global__ void kCoupling(DeviceState d, int src)
+{
+    stepKernelBegin();
+    if (!*d.status) couplingRow(d, src, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// Per-pair coupling force in the fluid's list order (for export only).
+__global__ void kCouplingPairs(DeviceState d, int src, float4* out)
+{
+    stepKernelBegin();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.nf) return;
+    const int m = min(d.fsc[i], d.kfs);
+    for (int k = 0; k < m; ++k) {
+        bool inside;
+        const float3 f = couplingPairForce(d, src, i, fsPartner(d.fs[listAt(k, i, d.nf)]), inside);
+        out[(size_t)k * d.nf + i] = f4(f);
+    }
+}
+
 // ---- runs of plain DEM steps on contact pairs ----
 // Building a step's contact list, finding each pair's springs in the previous
 // list and each pair's reverse slot took half of a dense bed's step; between
@@ -1027,7 +1088,9 @@ __global__ void __cluster_dims__(SORT_CLUSTER, 1, 1) __launch_bounds__(ClusterWa
 }
 
 // The pairs of a step, G lanes per row taking its forward candidates in turn
-// (the bonds in blocks of their own, from contactBlocks on).  A candidate's
+// (the bonds in blocks of their own, from contactBlocks on, and the coupling
+// force of a step with fluid in those behind: on a side stream of its own it
+// cost a fork and a join a step, 18.3 us to 17.7 without them for 512 solids).  A candidate's
 // list test and overlap need five 16-byte reads of its solid, issued together;
 // only a pair in contact reads the other five.
 //
@@ -1039,11 +1102,16 @@ __global__ void __cluster_dims__(SORT_CLUSTER, 1, 1) __launch_bounds__(ClusterWa
 #ifndef DEMSPH_PAIR_STEP_BLOCKS
 #define DEMSPH_PAIR_STEP_BLOCKS 6  // resident blocks of T per SM the registers allow
 #endif
-template <int G>
-__global__ void __launch_bounds__(T, DEMSPH_PAIR_STEP_BLOCKS) kPairStep(DeviceState d, int par, float dt, int contactBlocks)
+template <int G, bool COUPLING>
+__global__ void __launch_bounds__(T, DEMSPH_PAIR_STEP_BLOCKS) kPairStep(DeviceState d, int par, float dt, int contactBlocks,
+                                                                      int bondBlocks)
 {
     stepKernelBegin();
     if (*d.status) return;
+    if (COUPLING && (int)blockIdx.x >= contactBlocks + bondBlocks) {
+        couplingRow(d, 0, ((int)blockIdx.x - contactBlocks - bondBlocks) * blockDim.x + threadIdx.x);
+        return;
+    }
     const DeviceState atEnd = endView(d);
     if ((int)blockIdx.x >= contactBlocks) {
         const int b = ((int)blockIdx.x - contactBlocks) * blockDim.x + threadIdx.x;
@@ -1732,7 +1800,7 @@ void launchPairsRebuild(const DeviceState& d, int par, cudaStream_t s)
 #ifndef DEMSPH_PAIR_LANES
 #define DEMSPH_PAIR_LANES 0  // 0: the rule below
 #endif
-void launchPairStep(const DeviceState& d, int par, float dt, cudaStream_t s)
+void launchPairStep(const DeviceState& d, int par, float dt, bool coupling, cudaStream_t s)
 {
     // lanes per row: 16 warps' worth of threads per SM on small scenes.  A step
     // of 3k grains takes 30.5 / 23.9 / 20.9 / 18.4 us with 1 / 2 / 4 / 8 lanes,
@@ -1742,8 +1810,10 @@ void launchPairStep(const DeviceState& d, int par, float dt, cudaStream_t s)
     if (G == 0)
         for (G = 1; G < 8 && (long long)d.nrow * G < 152LL * 512;) G *= 2;
     const int cb = blocksFor((long long)d.nrow * G, T), bb = d.nb > 0 ? blocksFor(d.nb, T) : 0;
-    auto* k = G == 8 ? kPairStep<8> : G == 4 ? kPairStep<4> : G == 2 ? kPairStep<2> : kPairStep<1>;
-    launchStep(k, cb + bb, T, s, d, par, dt, cb);
+    const int fb = coupling ? blocksFor((long long)d.nrow * COUPLING_LANES, T) : 0;
+    auto* k = G == 8 ? kPairStep<8, false> : G == 4 ? kPairStep<4, false> : G == 2 ? kPairStep<2, false> : kPairStep<1, false>;
+    if (coupling) k = G == 8 ? kPairStep<8, true> : G == 4 ? kPairStep<4, true> : G == 2 ? kPairStep<2, true> : kPairStep<1, true>;
+    launchStep(k, cb + bb + fb, T, s, d, par, dt, cb, bb);
 }
 void launchPairSums(const DeviceState& d, int par, double dt, cudaStream_t s, int integrate, bool countStep)
 {
@@ -1789,5 +1859,16 @@ void launchSolidIntegrate(const DeviceState& d, double dt, int mode, int par, bo
         launchStep(kIntegrate<INTEGRATE_AFTER>, blocks, 256, s, d, h, d.clumpLanes, cb, cf, cs, par);
 }
 
+void launchCoupling(const DeviceState& d, int src, cudaStream_t s)
+{
+    if (d.nf <= 0 || d.ns <= 0 || d.nrow <= 0) return;
+    launchStep(kCoupling, blocksFor((long long)d.nrow * COUPLING_LANES, T), T, s, d, src);
+}
+
+void launchCouplingPairForces(const DeviceState& d, int src, float4* out, cudaStream_t s)
+{
+    if (d.nf <= 0 || d.ns <= 0) return;
+    launchStep(kCouplingPairs, blocksFor(d.nf, 128), 128, s, d, src, out);
+}
 
 }  // namespace demsph

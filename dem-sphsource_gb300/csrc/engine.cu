@@ -576,10 +576,10 @@ void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
         CK(cudaMemcpyAsync(d.splE, d.spl, sizeof(float4) * d.ns, cudaMemcpyDeviceToDevice, e->stream));
     }
     stageBefore(e, dt);
-    // the coupling force of an opened step reads the fluids and the solids as
-    // the fused pass leaves them, and nothing the search writes: it runs on
-    // the side stream beside the contact detection (and the coupling force
-    // of a plain DEM step is all its fluid stage does)
+    // the coupling force of an opened step (all its fluid stage does) reads the
+    // fluids and the solids as the fused pass leaves them, and nothing the search
+    // writes: a step on pairs computes it in the launch of its pairs, another on
+    // the side stream beside the contact detection
     const bool branch = !merge && !e->profiling && e->nMassive > 0 && d.nf > 0 && d.ns > 0 && d.nrow > 0;
     const std::function<void()> fork = [&] {
         CK(cudaEventRecord(e->forkEv, e->stream));
@@ -592,15 +592,16 @@ void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
     // the branch; the pair forces and bonds before them do not
     const std::function<void()> join = [&] { CK(cudaStreamWaitEvent(e->stream, e->joinEv, 0)); };
     const bool fold = sumsIntegrate(e);
+    const bool withPairs = branch && pairs && !d.fsPairForce;
     bool forked = false;
     for (int k = 0; k < length; ++k) {
-        if (!forked) stageFluid(e, dt, iStep + k, gap);
-        const bool last = k == length - 1;
+        const bool last = k == length - 1, onPairs = pairs && k > 0 && !last;
+        if (!forked && !(withPairs && onPairs)) stageFluid(e, dt, iStep + k, gap);
         bool integrated = false;
-        if (pairs && k > 0 && !last) {
+        if (onPairs) {
             {
                 TIMED("pair_forces");  // with the bonds
-                launchPairStep(d, e->par, (float)dt, e->stream);
+                launchPairStep(d, e->par, (float)dt, withPairs, e->stream);
             }
             if (forked) join();
             TIMED("solid_forces");
@@ -630,9 +631,9 @@ void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
             TIMED("integrate_after");  // the closing half of this step and the opening half of the next
             launchSolidIntegrate(d, dt, INTEGRATE_FUSED, e->par, d.nc > 0, true, e->stream);
         }
-        stageNeighborSearch(e, iStep + k + 1, gap, true, !merge, branch ? &fork : nullptr,
+        forked = branch && !(withPairs && k + 1 < length - 1);
+        stageNeighborSearch(e, iStep + k + 1, gap, true, !merge, forked ? &fork : nullptr,
                             !pairs ? PAIRS_NONE : (k + 1 < length - 1 ? PAIRS_STEP : PAIRS_LAST));
-        forked = branch;
     }
 }
 

@@ -560,7 +560,7 @@ void launchSolidForces(const DeviceState& d, int parity, double dt, cudaStream_t
 enum PairFlag { PAIR_OUT = 0, PAIR_LISTED = 1, PAIR_LIVE = 2 };
 void launchPairsOpen(const DeviceState& d, int parity, cudaStream_t s);
 void launchPairsRebuild(const DeviceState& d, int parity, cudaStream_t s);
-void launchPairStep(const DeviceState& d, int parity, float dt, cudaStream_t s);
+void launchPairStep(const DeviceState& d, int par, float dt, bool coupling, cudaStream_t s);
 void launchPairSums(const DeviceState& d, int parity, double dt, cudaStream_t s, int integrate, bool countStep);
 // The pairs' springs back into the list arrays of `parity` (a run that ended
 // early); old: as they were before the last rebuild.  Most live pairs of a row

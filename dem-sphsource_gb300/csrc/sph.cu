@@ -231,24 +231,6 @@ __device__ __forceinline__ EachOf<Term> eachOf(Term term)
 // GPU); the lanes' compensated partial sums are added in a fixed tree, so the
 // result does not depend on timing.  Kernels return early only for whole
 // warps: the shuffles take every lane.
-template <int L>
-__device__ __forceinline__ dfl groupSum(dfl v)
-{
-#pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) {
-        const dfl u = df_make(__shfl_xor_sync(0xffffffffu, v.hi, o, L), __shfl_xor_sync(0xffffffffu, v.lo, o, L));
-        v = (threadIdx.x & o) ? df_add(u, v) : df_add(v, u);
-    }
-    return v;
-}
-template <int L>
-__device__ __forceinline__ float groupSum(const KahanF& k)
-{
-    if (L == 1) return k.value();
-    const dfl v = groupSum<L>(df_two_sum(k.s, -k.c));
-    return v.hi + v.lo;
-}
-
 // ---- continuity (+ optional drift) ----
 // What bounds the pair loops: latency of the partner gathers at the warps the
 // registers allow (issue slots 50-60 % busy, L1 55 %, DRAM 15 %).  A partner is
@@ -627,60 +609,6 @@ __global__ void __launch_bounds__(T) kDensityReinit(DeviceState d, int storeRefe
     }
 }
 
-// ---- coupling force, per massive solid: sum over its fluid partners of
-// m_i x (solid term of momentum) (integrate.cu:282-330, gathered per solid
-// as calSolidForceTorque does through fluidSolidRange, :847-854) ----
-__device__ __forceinline__ float3 couplingPairForce(const DeviceState& d, int src, int i, int a, bool& inside)
-{
-    const Self o = loadSelf(d, i, src, 0, src);
-    const SolidPartner s = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, o.cs * o.cs, a);
-    inside = s.inside;
-    if (!s.inside) return make_float3(0.f, 0.f, 0.f);
-    const float3 via = o.v - s.v;
-    const float dU = -2.f * dot3(via, xyz(d.snormal[a]));
-    const float beta = fminf(3.f * fmaxf(dU, 0.f), o.cs);
-    const float Ps = (o.rho * s.Pa + s.rhoa * o.P + o.rho * s.rhoa * beta * dU) / (o.rho + s.rhoa);
-    return (s.r * Ps - via * (2.f * o.gam)) * (2.f * o.V * s.Va * s.G);
-}
-
-// Only contact rows can hold solids with mass, the only solids with fluid
-// partners here (the coupling lists take no others); L lanes of a row take
-// its partners in turn, each Kahan-summing its share, and the shares are
-// added in a fixed tree (groupSum).
-template <int L>
-__global__ void kCoupling(DeviceState d, int src)
-{
-    stepKernelBegin();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((t & ~31) >= d.nrow * L || *d.status) return;  // whole warps: the group sums shuffle
-    const int row = t / L, lane = t % L;
-    const bool live = row < d.nrow;
-    const int a = live ? solidOf(d, row) : 0;
-    KahanF3 f;
-    if (live)
-        for (int p = d.coupStart[a] + lane, e = d.coupStart[a + 1]; p < e; p += L) {
-            bool inside;
-            const float3 fi = couplingPairForce(d, src, d.coupList[p], a, inside);
-            if (inside) f.add(fi);
-        }
-    const float x = groupSum<L>(f.x), y = groupSum<L>(f.y), z = groupSum<L>(f.z);
-    if (live && lane == 0) d.sfcoup[a] = make_float4(x, y, z, 0.f);
-}
-
-// Per-pair coupling force in the fluid's list order (for export only).
-__global__ void kCouplingPairs(DeviceState d, int src, float4* out)
-{
-    stepKernelBegin();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.nf) return;
-    const int m = min(d.fsc[i], d.kfs);
-    for (int k = 0; k < m; ++k) {
-        bool inside;
-        const float3 f = couplingPairForce(d, src, i, fsPartner(d.fs[listAt(k, i, d.nf)]), inside);
-        out[(size_t)k * d.nf + i] = f4(f);
-    }
-}
-
 }  // namespace
 
 void launchDensityReinit(const DeviceState& d, int iStep, cudaStream_t s)
@@ -726,19 +654,6 @@ void launchMomentumPass(const DeviceState& d, double dtf, cudaStream_t s)
     if (d.fluidTiles) return launchTileMomentum(d, dtf, s);
     if (d.uniformFluid) LAUNCH_LANES_U(kMomentum, true, d.lanes, d.nf, T, s, d, df_from_double(dtf), df_from_double(0.5 * dtf));
     else LAUNCH_LANES_U(kMomentum, false, d.lanes, d.nf, T, s, d, df_from_double(dtf), df_from_double(0.5 * dtf));
-}
-
-void launchCoupling(const DeviceState& d, int src, cudaStream_t s)
-{
-    if (d.nf <= 0 || d.ns <= 0 || d.nrow <= 0) return;
-    constexpr int L = 8;  // lanes per row: rows hold tens of fluid partners
-    launchStep(kCoupling<L>, blocksFor((long long)d.nrow * L, 256), 256, s, d, src);
-}
-
-void launchCouplingPairForces(const DeviceState& d, int src, float4* out, cudaStream_t s)
-{
-    if (d.nf <= 0 || d.ns <= 0) return;
-    launchStep(kCouplingPairs, blocksFor(d.nf, 128), 128, s, d, src, out);
 }
 
 }  // namespace demsph

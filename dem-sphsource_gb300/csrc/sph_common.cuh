@@ -95,5 +95,25 @@ __device__ __forceinline__ dfl shepardTerm(dfl r, dfl invh)
     return df_mul(df_mul(t2, t2), df_add_f(df_mul_f(q, 2.0f), 1.0f));
 }
 
+// Sum over the L lanes of a group in double-float, in a fixed tree: every lane
+// gets the same bits.
+template <int L>
+__device__ __forceinline__ dfl groupSum(dfl v)
+{
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+        const dfl u = df_make(__shfl_xor_sync(0xffffffffu, v.hi, o, L), __shfl_xor_sync(0xffffffffu, v.lo, o, L));
+        v = (threadIdx.x & o) ? df_add(u, v) : df_add(v, u);
+    }
+    return v;
+}
+template <int L>
+__device__ __forceinline__ float groupSum(const KahanF& k)
+{
+    if (L == 1) return k.value();
+    const dfl v = groupSum<L>(df_two_sum(k.s, -k.c));
+    return v.hi + v.lo;
+}
+
 }  // namespace sph
 }  // namespace demsph
