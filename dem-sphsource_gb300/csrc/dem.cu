@@ -1378,14 +1378,16 @@ __global__ void __launch_bounds__(T) kPairsClose(DeviceState d, int par, int old
 }
 
 // x_i - centroid of pebble i as double-float per axis, then float.
-__device__ __forceinline__ float3 pebbleLever(const DeviceState& d, int i, float4 cH, float4 cL)
+__device__ __forceinline__ float3 pebbleLever(const DeviceState& d, int4 c, float4 h, float4 l, float4 cH, float4 cL)
 {
-    const int4 c = d.scell[i];
-    const float4 h = d.sph[i], l = d.spl[i];
     const dfl x = df_sub(df_add(df_mul_f(d.grid.csx, (float)c.x), df_make(h.x, l.x)), df_make(cH.x, cL.x));
     const dfl y = df_sub(df_add(df_mul_f(d.grid.csy, (float)c.y), df_make(h.y, l.y)), df_make(cH.y, cL.y));
     const dfl z = df_sub(df_add(df_mul_f(d.grid.csz, (float)c.z), df_make(h.z, l.z)), df_make(cH.z, cL.z));
     return make_float3(x.hi + x.lo, y.hi + y.lo, z.hi + z.lo);
+}
+__device__ __forceinline__ float3 pebbleLever(const DeviceState& d, int i, float4 cH, float4 cL)
+{
+    return pebbleLever(d, d.scell[i], d.sph[i], d.spl[i], cH, cL);
 }
 
 // Double-float sum over the `width` lanes of a group (width a power of two
@@ -1501,8 +1503,9 @@ __device__ __forceinline__ void solidIntegrateLoaded(const DeviceState& d, int i
     if (MODE != INTEGRATE_BEFORE) {
         driftRegs(ph, pl, vh, vl, half);
         kickRegs(vh, vl, wh, wl, a, tq, r, ph.w, spin, half);
-        checkDisplacementOf(d, stale, k.row, in.c, ph, k.p0, k.q0);
-        rehashSolidTo(d, i, k.row, in.c, ph, pl, MODE == INTEGRATE_FUSED ? d.sphE : d.sph,
+        int4 c = in.c;
+        checkDisplacementOf(d, stale, k.row, c, ph, k.p0, k.q0);
+        rehashSolidTo(d, i, k.row, c, ph, pl, MODE == INTEGRATE_FUSED ? d.sphE : d.sph,
                       MODE == INTEGRATE_FUSED ? d.splE : d.spl, k.key, k.centre);
     }
     if (MODE != INTEGRATE_AFTER) {
@@ -1667,6 +1670,125 @@ __device__ __forceinline__ void clumpIntegrateGroup(const DeviceState& d, dfl ha
     }
 }
 
+// The same (with clumpForce the force sums first, with MODE fused both halves)
+// where no clump has more pebbles than its group has lanes: a lane keeps its
+// pebble, and every lane the clump's state, in registers from one read to one
+// write.  Through memory each half, and the sums before them, waited for the
+// writes of the one before: a step of 6k grains and clumps 30.4 us, here 27.7.
+template <int MODE>
+__device__ __forceinline__ void clumpIntegrateLanes(const DeviceState& d, dfl half, int width, int t, int clumpForce, int* stale)
+{
+    const int c = t / width, lane = t % width;
+    // whole warps only: the shuffles below take every lane of the warp
+    if ((t & ~31) >= d.nc * width || *d.status) return;
+    const bool live = c < d.nc;
+    const int cc = live ? c : 0, i = d.cstart[cc] + lane;
+    const bool has = live && i < d.cend[cc];
+    SolidIn p = {};
+    CheckIn k = {};
+    float3 acc = make_float3(0.f, 0.f, 0.f), tq = acc, normal = acc;
+    if (has) {
+        p = loadSolid(d, i);
+        acc = xyz(d.sacc[i]);
+        tq = xyz(d.storque[i]);
+        normal = xyz(d.snormal[i]);
+        if (MODE != INTEGRATE_BEFORE) k = loadCheck(d, i);
+    }
+    float4 cH = d.cpH[cc], cL = d.cpL[cc], vH = d.cvH[cc], vL = d.cvL[cc], wH = d.cwH[cc], wL = d.cwL[cc];
+    const float im = d.cinvm[cc];
+    float I[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) I[j] = d.cIw[6 * cc + j];
+    float3 a, T;
+    if (clumpForce) {  // clumpForceGroup
+        const dfl zero = df_make(0.f, 0.f);
+        dfl Fx = zero, Fy = zero, Fz = zero, Tx = zero, Ty = zero, Tz = zero;
+        if (has) {
+            float3 fi = make_float3(0.f, 0.f, 0.f);
+            if (p.f.w & F_MASSIVE) fi = acc / p.ph.w;
+            const float3 ti = tq + cross3(pebbleLever(d, p.c, p.ph, p.pl, cH, cL), fi);
+            Fx = df_add_f(Fx, fi.x);
+            Fy = df_add_f(Fy, fi.y);
+            Fz = df_add_f(Fz, fi.z);
+            Tx = df_add_f(Tx, ti.x);
+            Ty = df_add_f(Ty, ti.y);
+            Tz = df_add_f(Tz, ti.z);
+            d.storque[i] = make_float4(0, 0, 0, 0);
+        }
+        Fx = groupSumDF(Fx, width);
+        Fy = groupSumDF(Fy, width);
+        Fz = groupSumDF(Fz, width);
+        Tx = groupSumDF(Tx, width);
+        Ty = groupSumDF(Ty, width);
+        Tz = groupSumDF(Tz, width);
+        a = make_float3(Fx.hi + Fx.lo, Fy.hi + Fy.lo, Fz.hi + Fz.lo) * im;
+        if (im > 0.f) a = a + d.g;
+        T = make_float3(Tx.hi + Tx.lo, Ty.hi + Ty.lo, Tz.hi + Tz.lo);
+        if (live && lane == 0) {
+            d.cacc[c] = f4(a);
+            d.ctorque[c] = make_float4(T.x, T.y, T.z, 0.f);
+        }
+    } else {
+        a = xyz(d.cacc[cc]);
+        T = xyz(d.ctorque[cc]);
+    }
+    const float hdt = half.hi;
+    // the clump's kick, and its pebble's motion from the kicked state about the
+    // centroid (aH, aL) (pebbleKick)
+    const auto kick = [&](float4 aH, float4 aL) {
+        const float3 w0 = xyz(wH);
+        addDF(vH, vL, a * hdt);
+        if (im > 0.f) addDF(wH, wL, symTimes(I, T) * hdt);
+        if (d.fixes & DEMSPH_FIX_CLUMP_ROTATION) {
+            if (live && lane == 0) clumpRotate(d, c, w0, xyz(wH), hdt);
+            __syncwarp();
+            for (int j = 0; j < 6; ++j) I[j] = ((volatile const float*)d.cIw)[6 * cc + j];
+        }
+        const float3 r = pebbleLever(d, p.c, p.ph, p.pl, aH, aL), w = xyz(wH);
+        acc = a + cross3(a, r) + cross3(w, cross3(w, r));
+        p.vh = vH;
+        p.vl = vL;
+        addDF(p.vh, p.vl, cross3(w, r));
+        normal = rotateF(normal, (w0 + w) * (0.5f * half.hi));
+    };
+    if (MODE != INTEGRATE_BEFORE) {
+        driftRegs(p.ph, p.pl, p.vh, p.vl, half);
+        axpyDF(cH, cL, vH, vL, half);
+        kick(cH, cL);
+        if (has) {
+            if (k.row >= 0) checkDisplacementOf(d, stale, k.row, p.c, p.ph, k.p0, k.q0);
+            rehashSolidTo(d, i, k.row, p.c, p.ph, p.pl, MODE == INTEGRATE_FUSED ? d.sphE : d.sph,
+                          MODE == INTEGRATE_FUSED ? d.splE : d.spl, k.key, k.centre);
+        }
+    }
+    if (MODE != INTEGRATE_AFTER) {
+        const float4 aH = cH, aL = cL;
+        kick(aH, aL);
+        axpyDF(cH, cL, vH, vL, half);
+        driftRegs(p.ph, p.pl, p.vh, p.vl, half);
+        if (has) {
+            d.sph[i] = p.ph;
+            d.spl[i] = p.pl;
+        }
+    }
+    if (has) {
+        d.sacc[i] = f4(acc);
+        d.svh[i] = p.vh;
+        d.svl[i] = p.vl;
+        d.swh[i] = make_float4(wH.x, wH.y, wH.z, 0.f);
+        d.swl[i] = make_float4(wL.x, wL.y, wL.z, 0.f);
+        d.snormal[i] = f4(normal);
+    }
+    if (live && lane == 0) {
+        d.cpH[c] = cH;
+        d.cpL[c] = cL;
+        d.cvH[c] = vH;
+        d.cvL[c] = vL;
+        d.cwH[c] = wH;
+        d.cwL[c] = wL;
+    }
+}
+
 __global__ void kClumpForce(DeviceState d, int width)
 {
     stepKernelBegin();
@@ -1681,9 +1803,9 @@ __global__ void kClumpForce(DeviceState d, int width)
 // forces (kClumpForce's work, for runs of whole steps where nothing happens
 // between the contact phase and this integration); countStep: the step has
 // completed (the status can no longer change) and is counted.
-template <int MODE>
-__global__ void kIntegrate(DeviceState d, dfl half, int width, int clumpBlocks, int clumpForce, int countStep,
-                           int par)
+template <int MODE, bool SINGLE>
+__global__ void __launch_bounds__(256, 2) kIntegrate(DeviceState d, dfl half, int width, int clumpBlocks, int clumpForce,
+                                                     int countStep, int par)
 {
     stepKernelBegin();
     int* stale = d.rebuild + (par ^ 1);  // the next step's candidate flag
@@ -1695,6 +1817,10 @@ __global__ void kIntegrate(DeviceState d, dfl half, int width, int clumpBlocks, 
         return;
     }
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (SINGLE) {
+        clumpIntegrateLanes<MODE>(d, half, width, t, clumpForce, stale);
+        return;
+    }
     if (clumpForce) clumpForceGroup(d, width, t);
     if (MODE == INTEGRATE_FUSED) {
         // the group's lanes take the same pebbles in both halves, and lane 0
@@ -1851,12 +1977,14 @@ void launchSolidIntegrate(const DeviceState& d, double dt, int mode, int par, bo
     const int cb = d.nc > 0 ? blocksFor((long long)d.nc * d.clumpLanes, 256) : 0;
     if (sb + cb == 0 && !countStep) return;
     const int blocks = std::max(1, sb + cb), cf = clumpForce ? 1 : 0, cs = countStep ? 1 : 0;
-    if (mode == INTEGRATE_FUSED)
-        launchStep(kIntegrate<INTEGRATE_FUSED>, blocks, 256, s, d, h, d.clumpLanes, cb, cf, cs, par);
-    else if (mode == INTEGRATE_BEFORE)
-        launchStep(kIntegrate<INTEGRATE_BEFORE>, blocks, 256, s, d, h, d.clumpLanes, cb, cf, cs, par);
-    else
-        launchStep(kIntegrate<INTEGRATE_AFTER>, blocks, 256, s, d, h, d.clumpLanes, cb, cf, cs, par);
+    auto* k = kIntegrate<INTEGRATE_FUSED, false>;
+    if (d.clumpSingle)
+        k = mode == INTEGRATE_FUSED    ? kIntegrate<INTEGRATE_FUSED, true>
+            : mode == INTEGRATE_BEFORE ? kIntegrate<INTEGRATE_BEFORE, true>
+                                       : kIntegrate<INTEGRATE_AFTER, true>;
+    else if (mode != INTEGRATE_FUSED)
+        k = mode == INTEGRATE_BEFORE ? kIntegrate<INTEGRATE_BEFORE, false> : kIntegrate<INTEGRATE_AFTER, false>;
+    launchStep(k, blocks, 256, s, d, h, d.clumpLanes, cb, cf, cs, par);
 }
 
 void launchCoupling(const DeviceState& d, int src, cudaStream_t s)

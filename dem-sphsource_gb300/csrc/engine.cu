@@ -1269,6 +1269,7 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
             for (int c = 0; c < nc; ++c) most = std::max(most, sc->clump_pebble_end[c] - sc->clump_pebble_start[c]);
             d.clumpLanes = 1;
             while (d.clumpLanes < most && d.clumpLanes < 32) d.clumpLanes *= 2;
+            d.clumpSingle = nc > 0 && most <= d.clumpLanes ? 1 : 0;
             if (nc > 0) {
                 std::vector<float4> pH(nc), pL(nc), vH(nc), vL(nc), wH(nc), wL(nc), acc(nc), tq(nc);
                 std::vector<float> Iw(6 * (size_t)nc), im(nc);

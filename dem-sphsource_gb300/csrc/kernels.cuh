@@ -418,6 +418,7 @@ struct DeviceState {
     int* cstart;
     int* cend;
     int clumpLanes;          // lanes per clump in the clump kernels: a power of two <= 32 covering most pebbles
+    int clumpSingle;         // no clump has more pebbles than lanes
 };
 
 // Device-side launch condition: a kernel given one does its work when
@@ -642,8 +643,8 @@ __device__ __forceinline__ void checkDisplacement(const DeviceState& d, int* sta
 // rehashSolidTo leaves the renormalised offset in h, l and stores it to
 // outH, outL (sph, spl; sphE, splE when the next step's first half is
 // integrated in the same pass).
-// key0, centre0: its key and centre before.
-__device__ __forceinline__ void rehashSolidTo(const DeviceState& d, int i, int row, int4 c, float4& h, float4& l,
+// key0, centre0: its key and centre before; c becomes the new cell.
+__device__ __forceinline__ void rehashSolidTo(const DeviceState& d, int i, int row, int4& c, float4& h, float4& l,
                                               float4* outH, float4* outL, int key0, int4 centre0)
 {
     renormAxis(c.x, h.x, l.x, d.grid.csx);
