@@ -652,7 +652,7 @@ class Server:
                  batch=False, batch_round_steps=0):
         """graphs: CUDA graphs for a scene's turns - 0 only while it is the
         only active scene, 1 always, -1 never.  batch: every active scene
-        advances in one graph launch per round (demsph_batch_update), rounds
+        advances together round by round (demsph_batch_update), rounds
         of about batch_round_steps steps."""
         self.lib = load_library()
         cfg = ServerConfig(device, workers, chunk_steps, int(hbm_budget_bytes), 1 if autotune else 0, int(graphs),

@@ -1,6 +1,7 @@
 // Host-side engine object shared by engine.cu (life cycle, step schedule,
 // batching) and engine_io.cu (state transfer, setters, artefact export).
 #pragma once
+#include <atomic>
 #include <algorithm>
 #include <string>
 #include <vector>
@@ -111,6 +112,11 @@ struct demsph_engine {
     // Step rounds captured for demsph_batch_update (graphs, not instantiated:
     // a batch takes them as child graphs), keyed like the cached graphs plus
     // the round's phase in the fluid and Shepard schedule.
+    // unique over all engines of the process (batches tell their member sets apart by it)
+    long long serial = [] {
+        static std::atomic<long long> last{0};
+        return ++last;
+    }();
     struct RoundGraph {
         int phase, length, parity, gap;
         double dt;

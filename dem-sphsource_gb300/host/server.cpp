@@ -12,7 +12,7 @@
 // launches its kernels directly (graph capture and instantiation next to
 // other scenes' work cost hundreds of times more than on an idle GPU, more
 // than the graphs save).  In batch mode one thread advances every active
-// scene together instead, a round of steps per scene in one graph launch
+// scene together instead, a round of steps per scene in one call
 // (demsph_batch_update); the workers then create engines (and run each
 // scene's first step) and download finished scenes.  A scene that arrives while others run is
 // admitted as soon as memory frees up (continuous batching).  A finished

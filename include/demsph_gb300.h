@@ -422,15 +422,17 @@ DEMSPH_API int demsph_audit(demsph_engine* e, demsph_audit_values* out);
 /* Shepard reference sums sumW0 (core/integrate.cu:44-47). */
 DEMSPH_API int demsph_export_fluid_sumw0(demsph_engine* e, double* sumw0);
 
-/* ---- many scenes in one graph launch ----
+/* ---- many scenes in one call ----
    No counterpart in the reference (one scene per process).  One call advances
    engines[0..count) by n_steps[k] steps from first_step[k] each (time step
-   dt[k], fluid gap gap[k]), all in one CUDA graph launch: each engine's round
-   of steps is a child graph, captured once per (phase in the fluid and
-   Shepard schedule, length, contact-list parity, dt, gap), the children run as
-   independent branches, and the executable graph is reused while every
-   member's round repeats (rounds of even length that are multiples of
-   5 gap steps repeat).  Every scene's state afterwards is bit for bit its state
+   dt[k], fluid gap gap[k]), the scenes' kernels overlapping on the device.  A
+   set of rounds that has come before goes in one CUDA graph launch: each
+   engine's round of steps is a child graph, captured once per (phase in the
+   fluid and Shepard schedule, length, contact-list parity, dt, gap), the
+   children run as independent branches, and the executable graph is reused
+   while every member's round repeats (rounds of even length that are multiples
+   of 5 gap steps repeat).  A set that has not is launched as each engine's own
+   step graphs on its own stream.  Every scene's state afterwards is bit for bit its state
    after demsph_update over the same steps.  Step 1 and profiled runs go
    through demsph_update first; a member whose lists overflowed grows them and
    finishes its steps alone before the call returns.  status_out[k] receives
@@ -439,7 +441,7 @@ DEMSPH_API int demsph_export_fluid_sumw0(demsph_engine* e, double* sumw0);
    device; none may be used by another thread during the call. */
 typedef struct demsph_batch demsph_batch;
 typedef struct demsph_batch_info {
-    long long launches;      /* graph launches so far */
+    long long launches;      /* rounds launched so far */
     long long graph_builds;  /* executable graphs instantiated (member rounds changed) */
     long long members;       /* engines in the last built graph */
     long long nodes;         /* nodes in it */
