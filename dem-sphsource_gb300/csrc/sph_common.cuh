@@ -115,5 +115,48 @@ __device__ __forceinline__ float groupSum(const KahanF& k)
     return v.hi + v.lo;
 }
 
+// Groups of four lanes and more end a pass axis by axis: after groupSumAxes the
+// first quarter of the lanes carries x, the second y, the others z, and the
+// first lane of each (axisLead) moves and stores that component of the particle.
+template <int L>
+__device__ __forceinline__ int axisOf(int lane)
+{
+    return min(lane / (L / 4), 2);
+}
+template <int L>
+__device__ __forceinline__ bool axisLead(int lane)
+{
+    return lane % (L / 4) == 0 && lane < 3 * (L / 4);
+}
+__device__ __forceinline__ float component(const float4* p, int i, int axis) { return ((const float*)(p + i))[axis]; }
+__device__ __forceinline__ float& component(float4* p, int i, int axis) { return ((float*)(p + i))[axis]; }
+__device__ __forceinline__ float component(float3 v, int axis) { return axis == 0 ? v.x : axis == 1 ? v.y : v.z; }
+// groupSum of three sums at once, the lanes sharing them out as they go: the
+// same trees with the same operands in the same order, but four double-float
+// additions where three butterflies over eight lanes take nine.
+template <int L>
+__device__ __forceinline__ float groupSumAxes(const KahanF3& k)
+{
+    static_assert(L >= 4, "an axis per quarter");
+    constexpr unsigned FULL = 0xffffffffu;
+    const auto passed = [&](dfl v, int o) { return df_make(__shfl_xor_sync(FULL, v.hi, o, L), __shfl_xor_sync(FULL, v.lo, o, L)); };
+    const auto ordered = [&](dfl own, dfl other, bool upper) { return upper ? df_add(other, own) : df_add(own, other); };
+    dfl x = df_two_sum(k.x.s, -k.x.c), y = df_two_sum(k.y.s, -k.y.c);
+    const dfl z = df_two_sum(k.z.s, -k.z.c);
+    const bool half = threadIdx.x & (L / 2), quarter = threadIdx.x & (L / 4);
+    {   // the lower half keeps x and y, the upper z (in x)
+        const dfl otherX = passed(half ? x : z, L / 2), otherY = passed(y, L / 2);
+        x = ordered(half ? z : x, otherX, half);
+        y = df_add(y, otherY);
+    }
+    {   // the second quarter keeps y (in x)
+        const dfl other = passed(half || quarter ? x : y, L / 4);
+        x = ordered(quarter && !half ? y : x, other, quarter);
+    }
+#pragma unroll
+    for (int o = L / 8; o > 0; o >>= 1) x = ordered(x, passed(x, o), threadIdx.x & o);
+    return x.hi + x.lo;
+}
+
 }  // namespace sph
 }  // namespace demsph
