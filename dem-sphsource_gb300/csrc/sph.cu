@@ -63,18 +63,19 @@ __device__ __forceinline__ float3 fluidRel(const DeviceState& d, const WalkTable
 
 // ---- batched partner loops ----
 // Partners whose state is gathered before any of them is used: B gathers per
-// lane are in flight instead of one.  Depths and block counts measured on GB300
-// (ms per fluid period of the 1.0M coupled dam break, one lane per particle):
-// the one-by-one loop 3.889, depth 2 with 8 continuity and 6 momentum blocks
-// 3.829, depth 4 3.89-4.15 (spills), depth 8 4.43.
+// lane are in flight instead of one (depths 1 and 4 are slower; 4 spills).
+// Blocks per SM: what the registers of the loop need without spills in it.  A
+// pass over 410k particles with 8 / 7 / 6 continuity blocks takes 135 / 124 / 128
+// us, with 8 / 7 / 6 momentum blocks 148 / 140 / 142; over 19k with parameters
+// of their own the momentum takes 19.9 / 17.9 / 20.0.
 #ifndef DEMSPH_PAIR_BATCH
 #define DEMSPH_PAIR_BATCH 2
 #endif
 #ifndef DEMSPH_CONTINUITY_BLOCKS
-#define DEMSPH_CONTINUITY_BLOCKS 8  // resident blocks of T per SM the registers allow
+#define DEMSPH_CONTINUITY_BLOCKS 7  // resident blocks of T per SM the registers allow
 #endif
 #ifndef DEMSPH_MOMENTUM_BLOCKS
-#define DEMSPH_MOMENTUM_BLOCKS 6
+#define DEMSPH_MOMENTUM_BLOCKS 7
 #endif
 constexpr int BATCH = DEMSPH_PAIR_BATCH;
 
@@ -167,7 +168,7 @@ __device__ __forceinline__ FluidRec loadRecord(const FluidRec* __restrict__ p)
 // made by the walk) are mended out of line.
 template <int L, int B, class Term>
 __device__ __forceinline__ void forFluidRecords(const DeviceState& d, const WalkTable& tab, const FluidRec* __restrict__ rec,
-                                                int i, int lane, int m, int4 ci, float4 pi, Term term)
+                                                int i, int lane, int m, float4 pi, Term term)
 {
     forFluidPartners<L, B>(
         d.ff, d.nf, i, lane, m, [&](unsigned e) { return loadRecord(rec + ffPartner(e)); },
@@ -184,7 +185,7 @@ __device__ __forceinline__ void forFluidRecords(const DeviceState& d, const Walk
             if (!ffRegular(all)) {
 #pragma unroll
                 for (int u = 0; u < B; ++u)
-                    if (!ffRegular(e[u])) r[u] = relF(ci, pi, d.fcell[ffPartner(e[u])], q[u].pc, d.grid);
+                    if (!ffRegular(e[u])) r[u] = relF(d.fcell[i], pi, d.fcell[ffPartner(e[u])], q[u].pc, d.grid);
             }
 #pragma unroll
             for (int u = 0; u < B; ++u) term(r[u], q[u], ok[u]);
@@ -232,11 +233,15 @@ __device__ __forceinline__ EachOf<Term> eachOf(Term term)
 // result does not depend on timing.  Kernels return early only for whole
 // warps: the shuffles take every lane.
 // ---- continuity (+ optional drift) ----
-// What bounds the pair loops: latency of the partner gathers at the warps the
-// registers allow (issue slots 50-60 % busy, L1 55 %, DRAM 15 %).  A partner is
-// one 32-byte record in one load, the terms of a round run without branches,
-// and two lanes share a list sector: 400k particles 160 to 133 us (momentum 202
-// to 143), 1.0M 354 to 301 (440 to 317), 48k 28 to 25 (33 to 31).
+// What bounds the pair loops: in large scenes L1 wavefronts, one for nearly every
+// sector gathered (90 % of their peak at 410k particles, spills in the loop a
+// fifteenth of them), in small ones latency of the gathers.  A partner is one
+// 32-byte record in one load, the terms of a round run without branches, two
+// lanes share a list sector, and a uniform fluid's own state is its position,
+// velocity and density (its parameters are kernel constants, and what its solid
+// partners need is read again where it has any): 400k particles 131 to 124 us
+// with the last (160 with four reads a partner; momentum 202, 140), 1.0M 306 to
+// 286 (327 to 321).
 struct ContinuityArgs {
     int ps, vs, ds, dd;  // position / velocity / density source, density destination
     int rec;             // partner records read (uniform fluids): position ps, velocity vs, density ds
@@ -260,29 +265,30 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
     const int i = t / L, lane = t % L;
     const bool live = i < d.nf;
     KahanF acc;
-    Self o;
     if (live) {
-        o = loadSelf(d, i, a.ps, a.vs, a.ds);
         const int n = d.nf;
         const int nff = min(d.ffc[i], d.kff);
         if constexpr (U) {
             // every fluid particle has the same rest density, sound speed,
             // viscosity, mass and smoothing length: the kernel's constants come
             // from the kernel parameters, P_i - P_j = c^2 (dRho_i - dRho_j)
-            const float drhoI = d.fdrho[a.ds][i];
-            const float scale = -2.f * o.rho * d.fparU.w * d.fconstU.z;
+            const float4 pI = d.fph[a.ps][i];
+            const float3 vI = xyz(d.fvh[a.vs][i]);
+            const float drhoI = d.fdrho[a.ds][i], rhoI = d.fparU.x + drhoI;
+            const float scale = -2.f * rhoI * d.fparU.w * d.fconstU.z;
             forFluidRecords<L, BATCH>(
-                d, walkTab, d.frec[a.rec], i, lane, nff, o.c, o.p, [&](float3 r, const FluidRec& q, bool ok) {
+                d, walkTab, d.frec[a.rec], i, lane, nff, pI, [&](float3 r, const FluidRec& q, bool ok) {
                     const float r2 = ok ? dot3(r, r) : d.fconstU.x;
                     const float rhoj = d.fparU.x + q.vd.w;
                     const float rr = fastSqrt(r2);
                     const float tt = 1.f - rr * d.fconstU.y;
-                    const float3 vij = o.v - xyz(q.vd);
+                    const float3 vij = vI - xyz(q.vd);
                     const float flux = rhoj * dot3(vij, r) + (drhoI - q.vd.w) * d.fparU.y * rr;
-                    const float term = scale * (tt * tt * tt) * fastRcp(rhoj * (o.rho + rhoj)) * flux;
+                    const float term = scale * (tt * tt * tt) * fastRcp(rhoj * (rhoI + rhoj)) * flux;
                     acc.add(r2 >= d.fconstU.x ? 0.f : term);
                 });
         } else {
+            const Self o = loadSelf(d, i, a.ps, a.vs, a.ds);
             const float4* __restrict__ ph = d.fph[a.ps];
             const float4* __restrict__ vh = d.fvh[a.vs];
             const float* __restrict__ drh = d.fdrho[a.ds];
@@ -306,13 +312,16 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
                 }));
         }
         const int nfs = min(d.fsc[i], d.kfs);
-        const float ci2 = o.cs * o.cs;
-        for (int k = lane; k < nfs; k += L) {
-            const int sa = fsPartner(d.fs[listAt(k, i, n)]);
-            const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
-            if (!sp.inside) continue;
-            acc.add(-2.f * o.rho * sp.Va * sp.G / (o.rho + sp.rhoa) *
-                    (2.f * sp.rhoa * dot3(o.v - sp.v, sp.r) + (o.P - sp.Pa) * sp.rr / o.cs));
+        if (lane < nfs) {  // near a wall: the particle's state again, not kept through the fluid loop
+            const Self o = loadSelf<U>(d, i, a.ps, a.vs, a.ds);
+            const float ci2 = o.cs * o.cs;
+            for (int k = lane; k < nfs; k += L) {
+                const int sa = fsPartner(d.fs[listAt(k, i, n)]);
+                const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
+                if (!sp.inside) continue;
+                acc.add(-2.f * o.rho * sp.Va * sp.G / (o.rho + sp.rhoa) *
+                        (2.f * sp.rhoa * dot3(o.v - sp.v, sp.r) + (o.P - sp.Pa) * sp.rr / o.cs));
+            }
         }
     }
     const float sum = groupSum<L>(acc);
@@ -328,7 +337,7 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
             if (axisLead<L>(lane)) {
                 component(d.fph[a.driftTo], i, x) = p.hi;
                 component(d.fpl[a.driftTo], i, x) = p.lo;
-                if (x == 2) d.fph[a.driftTo][i].w = o.h;
+                if (x == 2) d.fph[a.driftTo][i].w = U ? d.fhmax : d.fph[a.ps][i].w;
                 if (U && a.recOut >= 0) {
                     FluidRec& rec = d.frec[a.recOut][i];
                     component(&rec.pc, 0, x) = p.hi;
@@ -370,24 +379,26 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
     const bool live = i < d.nf;
     KahanF3 acc;
     if (live) {
-        const Self o = loadSelf(d, i, 1, 0, 1);
         const int n = d.nf;
         const int nff = min(d.ffc[i], d.kff);
         if constexpr (U) {  // see kContinuity
-            const float c2 = d.fparU.y * d.fparU.y;
-            const float twoNuRhoI = 2.f * d.fparU.z * o.rho, scale = 2.f * o.V * d.fconstU.z;
+            const float4 pI = d.fph[1][i];
+            const float3 vI = xyz(d.fvh[0][i]);
+            const float drhoI = d.fdrho[1][i], rhoI = d.fparU.x + drhoI;
+            const float c2 = d.fparU.y * d.fparU.y, PI = drhoI * d.fparU.y * d.fparU.y;
+            const float twoNuRhoI = 2.f * d.fparU.z * rhoI, scale = 2.f * (d.fparU.w / rhoI) * d.fconstU.z;
             forFluidRecords<L, BATCH>(
-                d, walkTab, d.frec[1], i, lane, nff, o.c, o.p, [&](float3 r, const FluidRec& q, bool ok) {
+                d, walkTab, d.frec[1], i, lane, nff, pI, [&](float3 r, const FluidRec& q, bool ok) {
                     const float r2 = ok ? dot3(r, r) : d.fconstU.x;
                     const float rhoj = d.fparU.x + q.vd.w;
                     const float Pj = q.vd.w * c2;
                     const float rr = fastSqrt(r2);
                     const float tt = 1.f - rr * d.fconstU.y;
-                    const float3 vij = o.v - xyz(q.vd);
+                    const float3 vij = vI - xyz(q.vd);
                     const float dU = -dot3(vij, r) * fastRcp(rr);  // U_L - U_R
                     const float beta = fminf(3.f * fmaxf(dU, 0.f), d.fparU.y);
-                    const float invSum = fastRcp(o.rho + rhoj);
-                    const float Ps = (o.rho * Pj + rhoj * o.P + o.rho * rhoj * beta * dU) * invSum;
+                    const float invSum = fastRcp(rhoI + rhoj);
+                    const float Ps = (rhoI * Pj + rhoj * PI + rhoI * rhoj * beta * dU) * invSum;
                     const float gbar = twoNuRhoI * rhoj * invSum;  // 2 g_i g_j / (g_i + g_j), g = nu rho
                     // 2 V_i V_j G / m, V_j = m / rho_j
                     const float w = scale * (tt * tt * tt) * fastRcp(rhoj);
@@ -395,6 +406,7 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
                     acc.add(r2 >= d.fconstU.x ? make_float3(0.f, 0.f, 0.f) : term);
                 });
         } else {
+            const Self o = loadSelf(d, i, 1, 0, 1);
             forFluidPartners<L, BATCH>(
                 d.ff, n, i, lane, nff,
                 [&](unsigned e) { return gatherFluid(d, ffPartner(e), d.fph[1], d.fvh[0], d.fdrho[1]); },
@@ -422,17 +434,20 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
                 }));
         }
         const int nfs = min(d.fsc[i], d.kfs);
-        const float ci2 = o.cs * o.cs;
-        for (int k = lane; k < nfs; k += L) {
-            const int sa = fsPartner(d.fs[listAt(k, i, n)]);
-            const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
-            if (!sp.inside) continue;
-            const float3 via = o.v - sp.v;
-            const float dU = -2.f * dot3(via, xyz(d.snormal[sa]));
-            const float beta = fminf(3.f * fmaxf(dU, 0.f), o.cs);
-            const float Ps = (o.rho * sp.Pa + sp.rhoa * o.P + o.rho * sp.rhoa * beta * dU) / (o.rho + sp.rhoa);
-            const float w = 2.f * o.V * sp.Va * sp.G / o.m;
-            acc.add((sp.r * Ps - via * (2.f * o.gam)) * w);
+        if (lane < nfs) {
+            const Self o = loadSelf<U>(d, i, 1, 0, 1);
+            const float ci2 = o.cs * o.cs;
+            for (int k = lane; k < nfs; k += L) {
+                const int sa = fsPartner(d.fs[listAt(k, i, n)]);
+                const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
+                if (!sp.inside) continue;
+                const float3 via = o.v - sp.v;
+                const float dU = -2.f * dot3(via, xyz(d.snormal[sa]));
+                const float beta = fminf(3.f * fmaxf(dU, 0.f), o.cs);
+                const float Ps = (o.rho * sp.Pa + sp.rhoa * o.P + o.rho * sp.rhoa * beta * dU) / (o.rho + sp.rhoa);
+                const float w = 2.f * o.V * sp.Va * sp.G / o.m;
+                acc.add((sp.r * Ps - via * (2.f * o.gam)) * w);
+            }
         }
     }
     float dx, dy, dz;  // moved since the candidates were listed

@@ -50,6 +50,9 @@ struct Self {
     float h, rho0, cs, nu, m, rho, P, V, gam;
 };
 
+// U: every fluid particle has the parameters fparU and the smoothing length
+// fhmax, kernel constants that take no registers through the loop.
+template <bool U = false>
 __device__ __forceinline__ Self loadSelf(const DeviceState& d, int i, int ps, int vs, int ds)
 {
     Self o;
@@ -57,8 +60,8 @@ __device__ __forceinline__ Self loadSelf(const DeviceState& d, int i, int ps, in
     o.p = d.fph[ps][i];
     o.v = xyz(d.fvh[vs][i]);
     const float dr = d.fdrho[ds][i];
-    const float4 par = d.fpar[i];
-    o.h = o.p.w;
+    const float4 par = U ? d.fparU : d.fpar[i];
+    o.h = U ? d.fhmax : o.p.w;
     o.rho0 = par.x;
     o.cs = par.y;
     o.nu = par.z;
