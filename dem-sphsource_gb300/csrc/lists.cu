@@ -740,17 +740,17 @@ __global__ void __launch_bounds__(T) kFluidFilter(DeviceState d)
     const int4 ci = d.fcell[self];
     const float4 hi = d.fph[0][self], li = d.fpl[0][self];
     const int nc = live ? min(d.fvcn[i], d.kvf) : 0, ns = live ? min(d.fvsn[i], d.kvs) : 0;
+    int sn = lane < ns ? d.fvsc[listAt(lane, i, n)] : 0;  // the first solid candidate, read beside the fluids
     int nff;
     if constexpr (P) nff = filterRecords(d, tab, ListWriter(ring, d.ff, self, n, d.kff), self, lane, nc, ci, hi, li);
     else nff = filterCells(d, ListWriter(ring, d.ff, self, n, d.kff), self, lane, nc, ci, hi, li);
     ListWriter to(ring, (unsigned*)d.fs, self, n, d.kfs);
     for (int k = lane; __any_sync(0xffffffffu, k - lane < ns); k += LIST_LANES) {
         bool take = false;
-        int a = 0, t = 0;
-        if (k < ns) {
-            a = d.fvsc[listAt(k, i, n)];
-            take = solidPartnerOf(d, ci, hi, li, a, d.scell[a], d.sph[a], t);
-        }
+        int t = 0;
+        const int a = sn;
+        if (k + LIST_LANES < ns) sn = d.fvsc[listAt(k + LIST_LANES, i, n)];
+        if (k < ns) take = solidPartnerOf(d, ci, hi, li, a, d.scell[a], d.sph[a], t);
         to.add(take, (unsigned)fsEntry(a, t));
     }
     const int nfs = to.finish();
