@@ -267,7 +267,9 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
     KahanF acc;
     if (live) {
         const int n = d.nf;
-        const int nff = min(d.ffc[i], d.kff);
+        const int nff = min(d.ffc[i], d.kff), nfs = min(d.fsc[i], d.kfs);
+        int next = 0;  // solid partner, read ahead (the first beside the fluids in groups of four lanes and more)
+        if (L >= 4 && lane < nfs) next = d.fs[listAt(lane, i, n)];
         if constexpr (U) {
             // every fluid particle has the same rest density, sound speed,
             // viscosity, mass and smoothing length: the kernel's constants come
@@ -311,12 +313,13 @@ __global__ void __launch_bounds__(T, DEMSPH_CONTINUITY_BLOCKS) kContinuity(Devic
                     acc.add(-2.f * o.rho * Vj * G / (o.rho + rhoj) * (rhoj * dot3(vij, r) + (o.P - Pj) * rr / c));
                 }));
         }
-        const int nfs = min(d.fsc[i], d.kfs);
+        if (L < 4 && lane < nfs) next = d.fs[listAt(lane, i, n)];
         if (lane < nfs) {  // near a wall: the particle's state again, not kept through the fluid loop
             const Self o = loadSelf<U>(d, i, a.ps, a.vs, a.ds);
             const float ci2 = o.cs * o.cs;
             for (int k = lane; k < nfs; k += L) {
-                const int sa = fsPartner(d.fs[listAt(k, i, n)]);
+                const int sa = fsPartner(next);
+                if (k + L < nfs) next = d.fs[listAt(k + L, i, n)];
                 const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
                 if (!sp.inside) continue;
                 acc.add(-2.f * o.rho * sp.Va * sp.G / (o.rho + sp.rhoa) *
@@ -380,7 +383,9 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
     KahanF3 acc;
     if (live) {
         const int n = d.nf;
-        const int nff = min(d.ffc[i], d.kff);
+        const int nff = min(d.ffc[i], d.kff), nfs = min(d.fsc[i], d.kfs);
+        int next = 0;  // solid partner, read ahead (the first beside the fluids in groups of four lanes and more)
+        if (L >= 4 && lane < nfs) next = d.fs[listAt(lane, i, n)];
         if constexpr (U) {  // see kContinuity
             const float4 pI = d.fph[1][i];
             const float3 vI = xyz(d.fvh[0][i]);
@@ -433,12 +438,13 @@ __global__ void __launch_bounds__(T, DEMSPH_MOMENTUM_BLOCKS) kMomentum(DeviceSta
                     acc.add((r * Ps - vij * gbar) * w);
                 }));
         }
-        const int nfs = min(d.fsc[i], d.kfs);
+        if (L < 4 && lane < nfs) next = d.fs[listAt(lane, i, n)];
         if (lane < nfs) {
             const Self o = loadSelf<U>(d, i, 1, 0, 1);
             const float ci2 = o.cs * o.cs;
             for (int k = lane; k < nfs; k += L) {
-                const int sa = fsPartner(d.fs[listAt(k, i, n)]);
+                const int sa = fsPartner(next);
+                if (k + L < nfs) next = d.fs[listAt(k + L, i, n)];
                 const SolidPartner sp = solidPartner(d, o.c, o.p, o.h, o.P, o.rho, o.rho0, ci2, sa);
                 if (!sp.inside) continue;
                 const float3 via = o.v - sp.v;
