@@ -11,9 +11,8 @@
 // Buffers keep fixed roles inside a step (fluid state in set [0] between
 // steps; set [1] holds the mid-step copy), except the solid contact list,
 // whose two parities alternate every build (the previous list is the spring
-// history).  A CUDA graph therefore captures one period of steps - a multiple
-// of 2 and of 5 gap - and is replayed; steps that do not fill a whole period
-// run uncaptured.
+// history).  CUDA graphs are captured by (kind of step, parity, length): a fluid
+// step each, a run of plain DEM steps up to 32 together.
 //
 // Overflow: list kernels record an overflow in a status word and every later
 // kernel returns at once, so a failed step leaves the state as it was after
@@ -1489,11 +1488,6 @@ int demsph_synchronize(demsph_engine* e)
     ENGINE_END(e)
 }
 
-// n_steps update() bodies without the driver hook.  With use_graph, steps run
-// uncaptured until i_step is a multiple of the period (and > 1: step 1 stores
-// the Shepard reference), whole periods replay one captured graph, the rest
-// runs uncaptured.  One synchronisation at the end; on a list overflow the
-// engine grows the list and resumes from the first incomplete step.
 // Kind of step i: bit 0 a fluid step (every gap steps), bit 1 a Shepard
 // re-initialisation (every 5 gap steps).  Steps of one kind launch the same
 // kernels with the same arguments, apart from the contact-list parity.
@@ -1585,7 +1579,10 @@ static int launchSteps(demsph_engine* e, double dt, int s, int end, int gap, std
     return len;
 }
 
-// The steps of demsph_update; `afterSteps` (when given) is enqueued after the
+// The steps of demsph_update: with use_graph, step 1 (it stores the Shepard
+// reference) runs uncaptured and the others replay graphs (launchSteps); on a
+// list overflow the engine grows the list and resumes from the first incomplete
+// step.  `afterSteps` (when given) is enqueued after the
 // steps of every attempt, before the one synchronisation that reads the
 // status, so a transfer it enqueues sees the state of the completed steps (an
 // attempt that overflowed is followed by one that enqueues it again).
