@@ -616,7 +616,7 @@ def run_many(args, world, rank, local):
             srv.close()
             return rank_total(w, "max", dist), out, clk
 
-        # the mix in one graph launch per round (demsph_batch_update), then the
+        # the mix in rounds over all scenes (demsph_batch_update), then the
         # same mix on per-scene streams with direct launches
         wall, st, clocks = mix(batch=True, batch_round_steps=args.round_steps)
         s_wall, s_st, _ = mix()
@@ -645,15 +645,15 @@ def run_many(args, world, rank, local):
                                       "breaks, fluid counts log-uniform in [2k, 60k], column heights uniform in "
                                       f"[0.2, 0.5] m, {steps} steps each, through the scene server",
                        "workers": args.workers, "hbm_budget_bytes": budget,
-                       "batched": "value: the faster of two forms of the server - one CUDA graph launch per "
-                                  "round advancing every active scene (each scene's round of about "
-                                  f"{args.round_steps} steps, whole Shepard periods, is a child graph; "
+                       "batched": "value: the faster of two forms of the server - rounds advancing every active "
+                                  "scene together (each scene's round is about "
+                                  f"{args.round_steps} steps, whole Shepard periods; "
                                   "demsph_batch_update; workers create engines and download results), and "
                                   "per-scene streams with 8 worker threads launching directly",
                        "autotune": "threads per fluid particle timed per size class (demsph_autotune)",
                        "timing": "host wall clock from the first submission to the last completion (engine "
                                  "creation and initialisation included)"},
-            "impl": "ours", "form": "one graph launch per round" if g_value >= s_value else "per-scene streams",
+            "impl": "ours", "form": "rounds over all scenes" if g_value >= s_value else "per-scene streams",
             "batched": {"value": g_value, "wall_s": wall, "p50_step_ms": st["p50_step_ms"],
                                         "p99_step_ms": st["p99_step_ms"], "peak_bytes": st["peak_bytes"],
                                         "scenes": st["completed"], "worker_create_s": st["create_s"],

@@ -604,7 +604,7 @@ class BatchInfo(C.Structure):
 
 
 class Batch:
-    """Many engines advanced in one CUDA graph launch (demsph_batch_*)."""
+    """Many engines advanced together (demsph_batch_*)."""
 
     def __init__(self, device=0):
         self.lib = load_library()
