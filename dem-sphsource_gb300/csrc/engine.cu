@@ -242,11 +242,14 @@ void allocContactLists(demsph_engine* e)
 void freePairs(demsph_engine* e)
 {
     DeviceState& d = e->d;
-    void* ptrs[] = {d.pfirst, d.plink, d.pflag, d.pforce, d.ptorqueA, d.ptorqueB, d.oldCount, d.oldId, d.oldFlag,
-                    d.pspring[0], d.pspring[1], d.pspring[2], d.oldSpring[0], d.oldSpring[1], d.oldSpring[2]};
-    for (void* p : ptrs) freeOne(e, p);
-    d.pflag = nullptr;
-    for (int k = 0; k < 3; ++k) d.pspring[k] = d.oldSpring[k] = nullptr;
+    const auto drop = [&](auto*& array) {
+        void* p = array;
+        freeOne(e, p);
+        array = nullptr;  // its address may come back as another array's
+    };
+    drop(d.pfirst), drop(d.plink), drop(d.pflag), drop(d.pforce), drop(d.ptorqueA), drop(d.ptorqueB);
+    drop(d.oldCount), drop(d.oldId), drop(d.oldFlag);
+    for (int k = 0; k < 3; ++k) drop(d.pspring[k]), drop(d.oldSpring[k]);
 }
 void allocPairs(demsph_engine* e)
 {
@@ -280,6 +283,27 @@ int contactSprings(const demsph_scene* sc)
             return 3;
     return 1;
 }
+
+}  // namespace
+
+namespace demsph {
+// A run that kept one spring a pair would start the others from zero at every
+// step once a model has rolling or torsion friction; the graphs hold the count
+// and the arrays.  Springs are never dropped again: a model without them leaves
+// zeros.
+void setContactSprings(demsph_engine* e, const demsph_scene* tables)
+{
+    DeviceState& d = e->d;
+    const int springs = contactSprings(tables);
+    if (springs <= d.pairSprings) return;
+    dropGraph(e);
+    freePairs(e);
+    d.pairSprings = springs;
+    allocPairs(e);
+}
+}  // namespace demsph
+
+namespace {
 
 // Tile mode of the fluid lists and pair loops (sph_tiles.cu) is used when
 // every fluid particle has the same parameters, the grid has at least three

@@ -249,6 +249,9 @@ inline int cudaFail(demsph_engine* e, const CudaError& c)
 
 void freeOne(demsph_engine* e, void*& p);
 void dropGraph(demsph_engine* e);
+// Contact tables of a running engine that now hold `tables`: the pair runs keep
+// the springs that these need.
+void setContactSprings(demsph_engine* e, const demsph_scene* tables);
 int readStatus(demsph_engine* e, int* stepsDone = nullptr);
 // Host transfers of the state enqueued on the engine's stream, without
 // synchronising (engine_io.cu).

@@ -519,6 +519,7 @@ int demsph_set_contact_models(demsph_engine* e, const demsph_scene* t)
     CK(cudaMemcpyAsync(const_cast<float*>(e->d.tab.hz), all.data(), sizeof(float) * all.size(), cudaMemcpyHostToDevice,
                        e->stream));
     CK(cudaStreamSynchronize(e->stream));
+    setContactSprings(e, t);
     return DEMSPH_OK;
     ENGINE_END(e)
 }
