@@ -143,7 +143,7 @@ void releaseStatusSlot(int2* slot)
 }
 
 // The status word and the steps completed since the last read that asked for
-// them: one copy of both (they are adjacent) into pinned memory.  Two copies
+// them (beginCount before they were launched): one copy of both (they are adjacent) into pinned memory.  Two copies
 // into pageable memory took 21 us, this 11.
 int readStatus(demsph_engine* e, int* stepsDone)
 {
@@ -155,8 +155,20 @@ int readStatus(demsph_engine* e, int* stepsDone)
     if (stepsDone) {
         *stepsDone = st.y - e->stepsSeen;
         e->stepsSeen = st.y;
+        e->countOpen = false;
     }
     return st.x;
+}
+
+// Before steps that are counted.  Steps of a call that failed before it read
+// their count are in the device's: it starts from zero again.
+void beginCount(demsph_engine* e)
+{
+    if (e->countOpen) {
+        CK(cudaMemsetAsync(e->d.stepsDone, 0, sizeof(int), e->stream));
+        e->stepsSeen = 0;
+    }
+    e->countOpen = true;
 }
 
 }  // namespace demsph
@@ -1618,6 +1630,7 @@ static int runUpdate(demsph_engine* e, double dt, int first_step, int n_steps, i
     int step = first_step;
     for (int attempt = 0; step < end; ++attempt) {
         if (attempt > 32) return fail(e, DEMSPH_ERR_CAPACITY, "list overflow persists after growing");
+        beginCount(e);
         const int startPar = e->par;
         const bool startOpened = e->resumeOpened;
         const bool graphs = use_graph && !e->profiling;
@@ -2126,7 +2139,14 @@ int demsph_batch_update(demsph_batch* b, demsph_engine* const* engines, int coun
     if (direct) {
         const auto tl = std::chrono::steady_clock::now();
         std::vector<int> next(members.size());
-        for (size_t k = 0; k < members.size(); ++k) next[k] = members[k].first;
+        for (size_t k = 0; k < members.size(); ++k) {
+            next[k] = members[k].first;
+            try {
+                beginCount(members[k].e);
+            } catch (const CudaError& c) {
+                engineFail(members[k].i, members[k].e, c);
+            }
+        }
         for (bool more = true; more;) {
             more = false;
             for (size_t k = 0; k < members.size(); ++k) {
@@ -2234,6 +2254,7 @@ int demsph_batch_update(demsph_batch* b, demsph_engine* const* engines, int coun
         b->exec = b->cache.front().exec;
         b->report = b->cache.front().report;
         const auto tl = std::chrono::steady_clock::now();
+        for (const auto& mb : members) mb.e->countOpen = true;  // until the report is read
         CK(cudaGraphLaunch(b->exec, b->stream));
         CK(cudaStreamSynchronize(b->stream));
         b->info.launch_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - tl).count();
@@ -2253,6 +2274,7 @@ int demsph_batch_update(demsph_batch* b, demsph_engine* const* engines, int coun
             mb.status = b->report[k].x;
             mb.done = b->report[k].y;
             e->stepsSeen = mb.done;  // the round's graph counts from zero
+            e->countOpen = false;
             e->replayedKernels += mb.r->kernels;
             for (const auto& fr : mb.r->fusedRuns) {
                 mb.fusedRuns.emplace_back(first + fr.first, fr.second);

@@ -146,10 +146,12 @@ struct demsph_engine {
     // demsph_update_io moves them on the second stream
     double* dscratch[2] = {nullptr, nullptr};
     size_t dscratchN[2] = {0, 0};
-    // Where the status and the step count are copied (pinned; statusSlot), and
-    // the step count as last read: the device's only grows.
+    // Where the status and the step count are copied (pinned; takeStatusSlot),
+    // the step count as last read (the device's only grows), and whether steps
+    // have been launched since (beginCount).
     int2* statusHost = nullptr;
     int stepsSeen = 0;
+    bool countOpen = false;
 
     // Exchanges everything two engines hold (device memory, stream, graphs,
     // state), field by field: demsph_append hands the caller's handle the
@@ -207,6 +209,7 @@ struct demsph_engine {
         swap(dscratchN[1], o.dscratchN[1]);
         swap(statusHost, o.statusHost);
         swap(stepsSeen, o.stepsSeen);
+        swap(countOpen, o.countOpen);
     }
 
     ~demsph_engine()
