@@ -1740,6 +1740,7 @@ __device__ __forceinline__ void clumpIntegrateLanes(const DeviceState& d, dfl ha
         addDF(vH, vL, a * hdt);
         if (im > 0.f) addDF(wH, wL, symTimes(I, T) * hdt);
         if (d.fixes & DEMSPH_FIX_CLUMP_ROTATION) {
+            __syncwarp();  // every lane has read the tensor that the first replaces
             if (live && lane == 0) clumpRotate(d, c, w0, xyz(wH), hdt);
             __syncwarp();
             for (int j = 0; j < 6; ++j) I[j] = ((volatile const float*)d.cIw)[6 * cc + j];
