@@ -1908,6 +1908,11 @@ void launchPairsOpen(const DeviceState& d, int par, cudaStream_t s)
 {
     launchStep(kPairsOpen, blocksFor(d.nrow, T), T, s, d, par);
 }
+int cooperativeRebuildBlocks()
+{
+    return std::min(cooperativeBlocks(kPairsRebuildCoop<true>, SORT_THREADS),
+                    cooperativeBlocks(kPairsRebuildCoop<false>, SORT_THREADS));
+}
 void launchPairsRebuild(const DeviceState& d, int par, cudaStream_t s)
 {
     // the cluster's threads are the lanes of 1024 rows: a step of 500 grains takes

@@ -1202,7 +1202,7 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
                 // at most two blocks per SM, and no more than two elements per
                 // thread need: small scenes leave the GPU to the others
                 const long long n = std::max<long long>(d.nf, ns);
-                d.wideBlocks = cooperativeSortBlocks();
+                d.wideBlocks = std::min(cooperativeSortBlocks(), cooperativeRebuildBlocks());
                 d.sortBlocks = (v && v[0] == '0') ? 0
                                                  : (int)std::min<long long>(d.wideBlocks,
                                                                             std::max<long long>(1, (n + 511) / 512));
@@ -1538,6 +1538,27 @@ static int stepKind(const DeviceState& d, int i, int gap)
 constexpr int MAX_GRAPH_STEPS = 32;
 constexpr size_t MAX_GRAPHS = 64;
 
+// What capturing steps changes of the engine as running them does.
+struct CaptureState {
+    int par;
+    bool walkOrder[2], keysAdvanced;
+    explicit CaptureState(const demsph_engine* e)
+        : par(e->par), walkOrder{e->walkOrder[0], e->walkOrder[1]}, keysAdvanced(e->keysAdvanced)
+    {
+    }
+};
+// Ends a capture that failed: nothing of it ran, or will.
+static void abandonCapture(demsph_engine* e, const CaptureState& before)
+{
+    cudaGraph_t junk = nullptr;
+    cudaStreamEndCapture(e->stream, &junk);
+    if (junk) cudaGraphDestroy(junk);
+    cudaGetLastError();
+    e->par = before.par;
+    for (int k = 0; k < 2; ++k) e->walkOrder[k] = before.walkOrder[k];
+    e->keysAdvanced = before.keysAdvanced;
+}
+
 // The graph of `length` steps of `kind` starting from the current parity,
 // captured on first use.
 static const demsph_engine::CachedGraph& graphFor(demsph_engine* e, int kind, int length, double dt, int step, int gap)
@@ -1550,16 +1571,22 @@ static const demsph_engine::CachedGraph& graphFor(demsph_engine* e, int kind, in
         e->graphs.erase(e->graphs.begin());
     }
     const int parity = e->par;
+    const CaptureState entry(e);
     cudaGraph_t g;
     const long long before = t_kernelLaunches;
     // runs of plain DEM steps fuse each step's closing integration with the
     // next one's opening (fluid steps are captured one at a time)
     const bool fused = e->fuseIntegration && kind == 0 && length >= 2;
     CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-    if (fused)
-        fusedSteps(e, dt, step, length, gap);
-    else
-        for (int k = 0; k < length; ++k) fullStep(e, dt, step + k, gap);
+    try {
+        if (fused)
+            fusedSteps(e, dt, step, length, gap);
+        else
+            for (int k = 0; k < length; ++k) fullStep(e, dt, step + k, gap);
+    } catch (...) {
+        abandonCapture(e, entry);
+        throw;
+    }
     CK(cudaStreamEndCapture(e->stream, &g));
     e->par = parity;  // nothing ran: the parity is where it was
     demsph_engine::CachedGraph c{kind, parity, length, nullptr, t_kernelLaunches - before, fused};
@@ -1953,6 +1980,7 @@ const demsph_engine::RoundGraph& roundFor(demsph_engine* e, double dt, int first
         r.id = ++g_roundIds;
     }
     const int parity = e->par;
+    const CaptureState entry(e);
     const long long before = t_kernelLaunches;
     CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     try {
@@ -1970,10 +1998,7 @@ const demsph_engine::RoundGraph& roundFor(demsph_engine* e, double dt, int first
             s += run;
         }
     } catch (...) {
-        cudaGraph_t junk = nullptr;
-        cudaStreamEndCapture(e->stream, &junk);
-        if (junk) cudaGraphDestroy(junk);
-        e->par = parity;
+        abandonCapture(e, entry);
         throw;
     }
     CK(cudaStreamEndCapture(e->stream, &r.graph));

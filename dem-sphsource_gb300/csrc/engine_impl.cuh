@@ -11,11 +11,6 @@
 
 namespace demsph {
 
-struct CudaError {
-    cudaError_t e;
-    const char* what;
-};
-
 #define CK(call)                                           \
     do {                                                   \
         cudaError_t _e = (call);                           \

@@ -245,11 +245,15 @@ int selftestBarrier(int missing, int* statusOut)
     if (cudaMalloc(&bar, 2 * sizeof(unsigned)) != cudaSuccess || cudaMalloc(&status, sizeof(int)) != cudaSuccess ||
         cudaMemset(bar, 0, 2 * sizeof(unsigned)) != cudaSuccess || cudaMemset(status, 0, sizeof(int)) != cudaSuccess) {
         rc = DEMSPH_ERR_CUDA;
-    } else if (!launchCooperative(kBarrierProbe, 2, 32, (cudaStream_t)0, bar, status, 2u + (unsigned)missing,
-                                  1 << 16) ||
-               cudaDeviceSynchronize() != cudaSuccess ||
-               cudaMemcpy(statusOut, status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) {
-        rc = DEMSPH_ERR_CUDA;
+    } else {
+        try {
+            launchCooperative(kBarrierProbe, 2, 32, (cudaStream_t)0, bar, status, 2u + (unsigned)missing, 1 << 16);
+        } catch (const CudaError&) {
+            rc = DEMSPH_ERR_CUDA;
+        }
+        if (rc == DEMSPH_OK && (cudaDeviceSynchronize() != cudaSuccess ||
+                                cudaMemcpy(statusOut, status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess))
+            rc = DEMSPH_ERR_CUDA;
     }
     cudaFree(bar);
     cudaFree(status);
@@ -258,12 +262,7 @@ int selftestBarrier(int missing, int* statusOut)
 
 int cooperativeSortBlocks()
 {
-    int dev = 0, sms = 0, perSm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kSolidSortCoop, SORT_THREADS, 0) != cudaSuccess)
-        return 0;
-    // two blocks per SM at most: room for other scenes' kernels beside it
-    return std::max(0, sms * std::min(perSm, 2));
+    return std::min(cooperativeBlocks(kSolidSortCoop, SORT_THREADS), cooperativeBlocks(kFluidReorderCoop, SORT_THREADS));
 }
 
 static RunIf fluidReorderWhen(const DeviceState& d, bool force)

@@ -3,6 +3,9 @@
 // files (grid.cu, lists.cu, sph.cu, dem.cu) only read this struct.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <algorithm>
+
 #include "engine.cuh"
 #include "../../include/demsph_gb300.h"
 
@@ -35,11 +38,18 @@ __device__ __forceinline__ void stepKernelBegin()
 // (default on; DEMSPH_OVERLAP_LAUNCHES=0 in the environment turns it off).
 bool overlapLaunches();
 
+// A CUDA call that failed.
+struct CudaError {
+    cudaError_t e;
+    const char* what;
+};
+
 // Launches a step kernel whose blocks wait on one another (grid barriers) as
 // a cooperative launch: all its blocks are resident at once, or the launch
-// fails.  Returns false when the launch was refused.
+// is refused, which throws (a step without its sort must not go on, and a graph
+// captured without it must not be kept).
 template <typename... KArgs, typename... Args>
-inline bool launchCooperative(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args)
+inline void launchCooperative(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args... args)
 {
     ++t_kernelLaunches;
     cudaLaunchConfig_t cfg = {};
@@ -52,7 +62,21 @@ inline bool launchCooperative(void (*kernel)(KArgs...), unsigned grid, unsigned 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess) throw CudaError{e, "a cooperative launch"};
+}
+
+// Blocks of a kernel of `threads` threads that a cooperative launch may have on
+// the current device: what is resident, two per SM at most (room for other
+// scenes' kernels beside it).
+template <typename... KArgs>
+inline int cooperativeBlocks(void (*kernel)(KArgs...), int threads)
+{
+    int dev = 0, sms = 0, perSm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, threads, 0) != cudaSuccess)
+        return 0;
+    return sms * std::min(perSm, 2);
 }
 
 // Barrier over all blocks of a cooperative launch.  bar[0] counts arrivals
@@ -491,6 +515,7 @@ void launchSolidSort(const DeviceState& d, bool force, bool fluidStep, int par, 
 // be used); DEMSPH_COOPERATIVE_SORT=0 in the environment keeps the four-launch
 // sort.
 int cooperativeSortBlocks();
+int cooperativeRebuildBlocks();  // of the contact pairs' rebuild (dem.cu)
 // Runs two blocks of a cooperative launch at a grid barrier that waits for
 // 2 + missing of them, with a short wait limit; stores the status bits.
 int selftestBarrier(int missing, int* statusOut);
