@@ -233,24 +233,29 @@ void allocFluidCandidates(demsph_engine* e)
 }
 
 // Per-slot arrays of the contact rows (scap slots per row).
+constexpr int LIST_WORK = 8;  // float4 a slot
 void allocContactLists(demsph_engine* e)
 {
     DeviceState& d = e->d;
     const size_t c = (size_t)d.scap * std::max(1, d.nrow);
     d.rev = dalloc<int>(c, e->owned, e->stream);
-    d.pF = dalloc<float4>(c, e->owned, e->stream);
-    d.pT = dalloc<float4>(c, e->owned, e->stream);
-    d.pTA = dalloc<float4>(c, e->owned, e->stream);
-    d.revF = dalloc<float4>(c, e->owned, e->stream);
-    d.revT = dalloc<float4>(c, e->owned, e->stream);
+    // what a contact list's step writes before it reads it, in one block: the
+    // pair runs use it between lists
+    d.listWork = dalloc<float4>(LIST_WORK * c, e->owned, e->stream);
+    float4** work[LIST_WORK] = {&d.pF, &d.pT, &d.pTA, &d.revF, &d.revT, &d.springIn[0], &d.springIn[1], &d.springIn[2]};
+    for (int k = 0; k < LIST_WORK; ++k) *work[k] = d.listWork + k * c;
     for (int p = 0; p < 2; ++p) d.fwd[p] = dalloc<int>(c, e->owned, e->stream);
-    for (int k = 0; k < 3; ++k) {
-        d.springIn[k] = dalloc<float4>(c, e->owned, e->stream);
+    for (int k = 0; k < 3; ++k)
         for (int p = 0; p < 2; ++p) d.springOut[p][k] = dalloc<float4>(c, e->owned, e->stream);
-    }
 }
 
-// The contact pairs of runs of plain DEM steps (a slot per forward candidate).
+// ---- the arrays of runs on contact pairs (a slot per forward candidate) ----
+// Made when a run first uses them, and given up whenever the lists grow: an
+// engine without such runs (a fluid step at least every third, staged calls,
+// direct launches) holds none.  The results of a step, and the history during a
+// rebuild of the candidates, take turns in the lists' block, which nothing else
+// uses between two lists; what is left is 26 bytes a candidate with one spring
+// (58 with three), 840 of the 4000 a contact row takes.
 void freePairs(demsph_engine* e)
 {
     DeviceState& d = e->d;
@@ -259,29 +264,76 @@ void freePairs(demsph_engine* e)
         freeOne(e, p);
         array = nullptr;  // its address may come back as another array's
     };
-    drop(d.pfirst), drop(d.plink), drop(d.pflag), drop(d.pforce), drop(d.ptorqueA), drop(d.ptorqueB);
-    drop(d.oldCount), drop(d.oldId), drop(d.oldFlag);
-    for (int k = 0; k < 3; ++k) drop(d.pspring[k]), drop(d.oldSpring[k]);
+    drop(d.pfirst), drop(d.plink), drop(d.pflag), drop(d.oldCount), drop(d.oldId), drop(d.oldFlag), drop(d.pairWork);
+    for (int k = 0; k < 3; ++k) {
+        drop(d.pspring[k]);
+        d.oldSpring[k] = nullptr;
+    }
+    d.pforce = d.ptorqueA = d.ptorqueB = nullptr;
+}
+size_t pairSlots(const DeviceState& d) { return (size_t)d.vcap * d.nrow; }
+// Whether the lists' block holds the three results (or springs) of the slots.
+bool pairsInListWork(const DeviceState& d) { return 3 * pairSlots(d) <= LIST_WORK * (size_t)d.scap * d.nrow; }
+size_t pairBytes(const DeviceState& d)
+{
+    return 8 * (size_t)d.nrow + pairSlots(d) * (10 + 16 * d.pairSprings + (pairsInListWork(d) ? 0 : 48));
+}
+// slot indices are ints; the rebuild is a cooperative launch
+bool pairsPossible(const demsph_engine* e)
+{
+    const DeviceState& d = e->d;
+    return e->pairRuns && e->pairsAllowed && d.nrow > 0 && d.sortBlocks > 0 && pairSlots(d) <= 2000000000ull;
+}
+// Whether there is room for the arrays: they are for speed, and leave three
+// quarters of the device's free memory to whoever needs it (not asked for less
+// than 64 MB).
+bool roomForPairs(const demsph_engine* e)
+{
+    const size_t bytes = pairBytes(e->d);
+    if (bytes < (64u << 20)) return true;
+    size_t unused = 0, total = 0;
+    uint64_t held = 0, used = 0;
+    cudaMemPool_t pool;
+    CK(cudaMemGetInfo(&unused, &total));
+    CK(cudaDeviceGetDefaultMemPool(&pool, e->device));
+    CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
+    CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    return bytes <= (unused + (size_t)(held - std::min(held, used))) / 4;
 }
 void allocPairs(demsph_engine* e)
 {
     DeviceState& d = e->d;
-    const size_t nr = (size_t)d.nrow, c = (size_t)d.vcap * nr;
-    // slot indices are ints; the rebuild is a cooperative launch
-    if (!e->pairRuns || d.nrow <= 0 || d.sortBlocks <= 0 || c > 2000000000ull) return;
+    const size_t nr = (size_t)d.nrow, c = pairSlots(d);
     d.pfirst = dalloc<int>(nr, e->owned, e->stream);
     d.plink = dalloc<int>(c, e->owned, e->stream, false);
     d.pflag = dalloc<unsigned char>(c, e->owned, e->stream);
-    d.pforce = dalloc<float4>(c, e->owned, e->stream, false);
-    d.ptorqueA = dalloc<float4>(c, e->owned, e->stream, false);
-    d.ptorqueB = dalloc<float4>(c, e->owned, e->stream, false);
     d.oldCount = dalloc<int>(nr, e->owned, e->stream);
     d.oldId = dalloc<int>(c, e->owned, e->stream, false);
     d.oldFlag = dalloc<unsigned char>(c, e->owned, e->stream);
-    for (int k = 0; k < d.pairSprings; ++k) {
-        d.pspring[k] = dalloc<float4>(c, e->owned, e->stream, false);
-        d.oldSpring[k] = dalloc<float4>(c, e->owned, e->stream, false);
+    for (int k = 0; k < d.pairSprings; ++k) d.pspring[k] = dalloc<float4>(c, e->owned, e->stream, false);
+    float4* work = d.listWork;
+    if (!pairsInListWork(d)) work = d.pairWork = dalloc<float4>(3 * c, e->owned, e->stream, false);
+    d.pforce = work;
+    d.ptorqueA = work + c;
+    d.ptorqueB = work + 2 * c;
+    for (int k = 0; k < d.pairSprings; ++k) d.oldSpring[k] = work + k * c;
+}
+// Before a run of `length` plain DEM steps is launched or captured (nothing is
+// allocated inside a capture).  Without room the runs keep their lists.
+void preparePairs(demsph_engine* e, int length)
+{
+    if (length < 3 || e->forceWalk || e->d.pflag || !pairsPossible(e)) return;
+    try {
+        if (roomForPairs(e)) {
+            allocPairs(e);
+            return;
+        }
+    } catch (const CudaError& c) {
+        freePairs(e);
+        cudaGetLastError();
+        if (c.e != cudaErrorMemoryAllocation) throw;
     }
+    e->pairRuns = false;
 }
 
 // Springs a contact keeps: one (sliding) unless some material pair has rolling
@@ -311,7 +363,6 @@ void setContactSprings(demsph_engine* e, const demsph_scene* tables)
     dropGraph(e);
     freePairs(e);
     d.pairSprings = springs;
-    allocPairs(e);
 }
 }  // namespace demsph
 
@@ -674,7 +725,7 @@ void fusedSteps(demsph_engine* e, double dt, int iStep, int length, int gap)
 
 // Grows whatever overflowed and clears the status.  e->par must be the parity
 // of the last successful solid list build (the history the retry reads).
-void grow(demsph_engine* e, int status)
+void growLists(demsph_engine* e, int status)
 {
     DeviceState& d = e->d;
     CK(cudaStreamSynchronize(e->stream));
@@ -708,8 +759,8 @@ void grow(demsph_engine* e, int status)
             float4* keepSpring[3] = {d.springOut[keep][0], d.springOut[keep][1], d.springOut[keep][2]};
             d.fwd[keep] = nullptr;
             for (int k = 0; k < 3; ++k) d.springOut[keep][k] = nullptr;
-            void* ptrs[] = {d.rev, d.pF, d.pT, d.pTA, d.revF, d.revT, d.fwd[keep ^ 1], d.springIn[0], d.springIn[1], d.springIn[2],
-                            d.springOut[keep ^ 1][0], d.springOut[keep ^ 1][1], d.springOut[keep ^ 1][2]};
+            void* ptrs[] = {d.rev, d.listWork, d.fwd[keep ^ 1], d.springOut[keep ^ 1][0], d.springOut[keep ^ 1][1],
+                            d.springOut[keep ^ 1][2]};
             for (void* p : ptrs) freeOne(e, p);
             d.scap = std::max(d.scap * 2, need[0] + need[0] / 2 + 1);
             allocContactLists(e);
@@ -725,8 +776,6 @@ void grow(demsph_engine* e, int status)
             freeOne(e, p);
             d.vcap = std::max(d.vcap * 2, need[1] + need[1] / 2 + 1);
             d.vcand = dalloc<int>((size_t)d.vcap * nr, e->owned, e->stream, false);
-            freePairs(e);  // the springs are in the lists again (closePairs)
-            allocPairs(e);
             CK(cudaMemsetAsync(d.rebuild, 0xff, 2 * sizeof(int), e->stream));  // rebuild on the retry
         }
     }
@@ -790,6 +839,12 @@ void grow(demsph_engine* e, int status)
     dropGraph(e);
 }
 
+void grow(demsph_engine* e, int status)
+{
+    freePairs(e);  // what lives between runs is in the lists (closePairs)
+    growLists(e, status);
+}
+
 // A step failed with status `st` after the steps before it completed (e->par is
 // their last list's parity).  Where the last of them ran on contact pairs, its
 // springs go back into the lists of that parity, which the retry reads.  runs:
@@ -805,8 +860,14 @@ void closePairs(demsph_engine* e, const std::vector<std::pair<int, int>>& runs, 
     launchPairsCount(d, old, e->stream);
     CK(cudaMemcpyAsync(&most, d.need, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
-    if (most > d.scap) grow(e, ST_SS_OVERFLOW);
+    void* work = nullptr;  // holds the history when it is closed from there
+    if (most > d.scap) {
+        work = d.listWork;
+        d.listWork = nullptr;
+        growLists(e, ST_SS_OVERFLOW);
+    }
     launchPairsClose(d, e->par, old, e->stream);
+    freeOne(e, work);
     e->walkOrder[e->par] = false;
 }
 
@@ -1215,7 +1276,6 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
                 const char* v = std::getenv("DEMSPH_PAIR_RUNS");
                 e->pairRuns = !(v && v[0] == '0') && e->fuseIntegration && o.solid_verlet_skin >= 0 && d.grid.gx >= 3 &&
                               d.grid.gy >= 3 && d.grid.gz >= 3 && (e->nMassive > 0 || e->movingDummies > 0);
-                allocPairs(e);
             }
             d.forceRows = o.contact_rows_per_warp > 0 ? o.contact_rows_per_warp : 32;
             e->adaptRows = o.contact_rows_per_warp == 0;
@@ -1570,13 +1630,14 @@ static const demsph_engine::CachedGraph& graphFor(demsph_engine* e, int kind, in
         cudaGraphExecDestroy(e->graphs.front().exec);
         e->graphs.erase(e->graphs.begin());
     }
+    // runs of plain DEM steps fuse each step's closing integration with the
+    // next one's opening (fluid steps are captured one at a time)
+    const bool fused = e->fuseIntegration && kind == 0 && length >= 2;
+    if (fused) preparePairs(e, length);
     const int parity = e->par;
     const CaptureState entry(e);
     cudaGraph_t g;
     const long long before = t_kernelLaunches;
-    // runs of plain DEM steps fuse each step's closing integration with the
-    // next one's opening (fluid steps are captured one at a time)
-    const bool fused = e->fuseIntegration && kind == 0 && length >= 2;
     CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
     try {
         if (fused)
@@ -1689,6 +1750,7 @@ static int runUpdate(demsph_engine* e, double dt, int first_step, int n_steps, i
             if (kind == 0)
                 while (len < MAX_GRAPH_STEPS && s + len < end && stepKind(d, s + len, gap) == 0) ++len;
             if (e->fuseIntegration && kind == 0 && len >= 2) {
+                preparePairs(e, len);
                 fusedSteps(e, dt, s, len, gap);
                 fusedRuns.emplace_back(s, len);
                 e->runStats.fused_passes += len - 1;
@@ -1860,6 +1922,25 @@ long long demsph_device_bytes(const demsph_engine* e)
     return b;
 }
 
+long long demsph_pair_run_bytes(const demsph_engine* e)
+{
+    if (!e) return -1;
+    const DeviceState& d = e->d;
+    return e->pairRuns && d.nrow > 0 && d.sortBlocks > 0 ? (long long)pairBytes(d) : 0;
+}
+
+int demsph_set_pair_runs(demsph_engine* e, int enable)
+{
+    ENGINE_GUARD(e)
+    if (e->pairsAllowed == (enable != 0)) return DEMSPH_OK;
+    CK(cudaStreamSynchronize(e->stream));
+    dropGraph(e);  // they hold the arrays, or run without
+    e->pairsAllowed = enable != 0;
+    if (!enable) freePairs(e);
+    return DEMSPH_OK;
+    ENGINE_END(e)
+}
+
 long long demsph_estimate_bytes(const demsph_scene* sc, const demsph_options* opt)
 {
     if (!sc || sc->n_fluid < 0 || sc->n_solid < 0) return -1;
@@ -1881,8 +1962,8 @@ long long demsph_estimate_bytes(const demsph_scene* sc, const demsph_options* op
     // solid: state, sort and wall springs; per contact row: its slots, two
     // list parities, springs in and out, candidates; per cell: counts and starts
     const long long kvf = kff + kff / 2, kvs = kfs + kfs / 2;
-    return nf * (444 + 4 * (kff + kfs) + 4 * (kvf + kvs) + 64) + ns * (248 + 48LL * sc->n_wall) +
-           rows * (80 + slots * 184 + 2 * slots * 4 + 2 * slots * (58 + 32 * contactSprings(sc))) + (cells + 1) * 16 + (long long)sc->n_clump * 160 +
+    return nf * (380 + 4 * (kff + kfs) + 4 * (kvf + kvs)) + ns * (248 + 48LL * sc->n_wall) +
+           rows * (72 + slots * 184 + 2 * slots * 4) + (cells + 1) * 16 + (long long)sc->n_clump * 160 +
            std::min(64 * rows + 1024, std::max(1LL, kfs * nf)) * 4 + (1 << 20);
 }
 
@@ -1966,6 +2047,15 @@ __global__ void kBatchReport(int* const* where, int n, int2* out)
     if (i < n) out[i] = make_int2(*where[2 * i], *where[2 * i + 1]);
 }
 
+// Steps of one graph from step s on: a run of plain DEM steps, or one step.
+int runLength(const DeviceState& d, int s, int end, int gap)
+{
+    int run = 1;
+    if (stepKind(d, s, gap) == 0)
+        while (s + run < end && stepKind(d, s + run, gap) == 0) ++run;
+    return run;
+}
+
 // The round of `n` steps of engine e from step `first` (captured on first use).
 const demsph_engine::RoundGraph& roundFor(demsph_engine* e, double dt, int first, int n, int gap)
 {
@@ -1979,6 +2069,8 @@ const demsph_engine::RoundGraph& roundFor(demsph_engine* e, double dt, int first
         std::lock_guard<std::mutex> g(g_roundMutex);
         r.id = ++g_roundIds;
     }
+    if (e->fuseIntegration)
+        for (int s = first, run; s < first + n; s += run) preparePairs(e, run = runLength(d, s, first + n, gap));
     const int parity = e->par;
     const CaptureState entry(e);
     const long long before = t_kernelLaunches;
@@ -1986,9 +2078,7 @@ const demsph_engine::RoundGraph& roundFor(demsph_engine* e, double dt, int first
     try {
         CK(cudaMemsetAsync(d.stepsDone, 0, sizeof(int), e->stream));
         for (int s = first, end = first + n; s < end;) {
-            int run = 1;
-            if (stepKind(d, s, gap) == 0)
-                while (s + run < end && stepKind(d, s + run, gap) == 0) ++run;
+            const int run = runLength(d, s, end, gap);
             if (run >= 2 && e->fuseIntegration) {
                 fusedSteps(e, dt, s, run, gap);
                 r.fusedRuns.emplace_back(s - first, run);

@@ -89,8 +89,9 @@ struct demsph_engine {
     // Runs of three or more plain DEM steps evaluate the contact candidates as
     // pairs between their first and last step, without contact lists
     // (DEMSPH_PAIR_RUNS=0 keeps the lists; off for good once the lists come from
-    // the walk).
+    // the walk, or where there was no room for the pairs).
     bool pairRuns = true;
+    bool pairsAllowed = true;  // demsph_set_pair_runs
     // The per-solid sums run the solids' integration pass in the same launch
     // when the integrated solids are exactly the contact rows
     // (DEMSPH_FOLD_INTEGRATION=0 keeps the separate pass).
@@ -181,6 +182,7 @@ struct demsph_engine {
         swap(fuseIntegration, o.fuseIntegration);
         swap(mergeContacts, o.mergeContacts);
         swap(pairRuns, o.pairRuns);
+        swap(pairsAllowed, o.pairsAllowed);
         swap(foldIntegration, o.foldIntegration);
         swap(resumeOpened, o.resumeOpened);
         swap(keysAdvanced, o.keysAdvanced);

@@ -116,7 +116,9 @@ struct Request {
     int steps = 0, next = 1, gap = 1;
     double dt = 0;
     long long mobile = 0;          // solids with mass: updated every step
-    long long reserved = 0;        // bytes held against the budget
+    long long reserved = 0;        // bytes held against the budget for its lists
+    long long pairBytes = 0;       // what its contact pairs take, held where pairs is set
+    bool pairs = false;
     State state = State::Pending;
     bool busy = false;             // a worker is advancing it
     demsph_engine* eng = nullptr;
@@ -168,6 +170,22 @@ struct demsph_server {
                 anyAdmitted = true;
                 firstAdmit = r.admitted;
             }
+        }
+    }
+
+    // Contact pairs of a scene about to replay graphs (lock held, nobody else
+    // uses its engine): out of what the budget leaves while nothing waits to be
+    // admitted, and given back when something does.
+    void sharePairs(Request& r, bool useful)
+    {
+        const bool on = pending.empty() && (r.pairs || (useful && used + r.pairBytes <= cfg.hbm_budget_bytes));
+        if (on == r.pairs || r.pairBytes <= 0 || demsph_set_pair_runs(r.eng, on) != DEMSPH_OK) return;
+        r.pairs = on;
+        used += on ? r.pairBytes : -r.pairBytes;
+        peak = std::max(peak, used);
+        if (!on) {
+            admit();
+            cv.notify_all();
         }
     }
 
@@ -268,6 +286,7 @@ struct demsph_server {
             for (size_t q = 0; q < k; ++q) {
                 Request& r = *mem[q];
                 r.busy = true;
+                sharePairs(r, true);
                 eng[q] = r.eng;
                 first[q] = r.next;
                 n[q] = roundSteps(r);
@@ -316,7 +335,8 @@ struct demsph_server {
         r.state = s;
         r.finished = Clock::now();
         lastFinish = r.finished;
-        used -= r.reserved;
+        used -= r.reserved + (r.pairs ? r.pairBytes : 0);
+        r.pairs = false;
         --activeN;
         if (s == State::Done) ++completed;
         else ++failed;
@@ -333,6 +353,7 @@ struct demsph_server {
             if (stop) return;
             r->busy = true;
             const int useGraph = cfg.graphs > 0 || (cfg.graphs == 0 && activeN == 1) ? 1 : 0;
+            if (r->eng) sharePairs(*r, useGraph && !cfg.batch);
             lock.unlock();
             int rc = DEMSPH_OK;
             std::string err;
@@ -350,6 +371,12 @@ struct demsph_server {
                 if (known) r->opt.fluid_lanes = known;
                 rc = demsph_create(&r->scene->s, &r->opt, &r->eng);
                 if (rc == DEMSPH_OK) rc = demsph_initialize(r->eng);
+                if (rc == DEMSPH_OK) {
+                    rc = demsph_set_pair_runs(r->eng, 0);
+                    std::lock_guard<std::mutex> g(m);
+                    r->pairBytes = demsph_pair_run_bytes(r->eng);
+                    if (rc == DEMSPH_OK) sharePairs(*r, useGraph && !cfg.batch);
+                }
                 if (rc == DEMSPH_OK && cls >= 0 && !known) {
                     int lanes = 0;
                     rc = demsph_autotune(r->eng, &lanes);
@@ -563,7 +590,7 @@ int demsph_server_request_info(demsph_server* s, long long id, demsph_request_in
     *info = demsph_request_info{};
     info->state = (int)r.state;
     info->steps_done = r.next - 1;
-    info->reserved_bytes = r.reserved;
+    info->reserved_bytes = r.reserved + (r.pairs ? r.pairBytes : 0);
     const auto now = Clock::now();
     const bool admitted = r.state != State::Pending;
     const bool ended = r.state == State::Done || r.state == State::Failed;

@@ -297,6 +297,17 @@ DEMSPH_API void* demsph_stream(demsph_engine* e);
    sized by dataBase on the host. */
 DEMSPH_API long long demsph_device_bytes(const demsph_engine* e);
 DEMSPH_API long long demsph_estimate_bytes(const demsph_scene* scene, const demsph_options* opts);
+/* Runs of three or more plain DEM steps keep their contacts as pairs, in device
+   memory (26 or 58 bytes a contact candidate) that an engine takes when such a
+   run first needs it, where that leaves three quarters of the free memory, and
+   that neither demsph_estimate_bytes nor a first demsph_device_bytes counts.
+   Without it the runs build contact lists, with the same bits.
+   demsph_pair_run_bytes: what the engine would take (0: no such runs).
+   demsph_set_pair_runs: enable = 0 gives the memory back and takes none from
+   then on (a caller with a budget); enable != 0, the start, allows it.  No
+   counterpart in the reference. */
+DEMSPH_API long long demsph_pair_run_bytes(const demsph_engine* e);
+DEMSPH_API int demsph_set_pair_runs(demsph_engine* e, int enable);
 /* Kernels this engine has executed so far (graph replays counted by their
    kernels), as issued from the calling thread. */
 DEMSPH_API long long demsph_kernel_launches(demsph_engine* e);

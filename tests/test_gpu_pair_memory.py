@@ -1,0 +1,77 @@
+"""Memory of the contact pairs: none until a run uses them, little beside the
+contact lists then, and a run goes on with contact lists where there is no room
+for them."""
+import os
+
+import numpy as np
+import pytest
+
+import cudart_fake
+from test_gpu_parity import _dry_granular, _same_state_and_lists
+
+pytestmark = pytest.mark.gpu
+
+CANDIDATES = 32  # a row's, at the default of 16 contacts
+
+
+def _device_bytes(e):
+    import ctypes as C
+    e.lib.demsph_device_bytes.restype = C.c_longlong
+    return e.lib.demsph_device_bytes(e.h)
+
+
+def _rolling(scenes):
+    r = _dry_granular(scenes)
+    r.calls[:] = [(fn, a[:5] + (0.2, 0.2, a[7], 0.05, 0.05)) if fn == "setHertzianContactModel" else (fn, a)
+                  for fn, a in r.calls]
+    return r
+
+
+@pytest.mark.parametrize("rolling", [False, True])
+def test_pairs_take_memory_once_a_run_uses_them(ds, scenes, rolling, monkeypatch):
+    b, sc = ds.build_scene(_rolling(scenes) if rolling else _dry_granular(scenes))
+    monkeypatch.setenv("DEMSPH_PAIR_RUNS", "0")
+    lists = ds.Engine(sc)
+    monkeypatch.setenv("DEMSPH_PAIR_RUNS", "1")
+    pairs = ds.Engine(sc)
+    dt = sc.time_step
+    for e in (lists, pairs):
+        e.initialize()
+        e.step(dt, 1, 1)
+        e.update(dt, 2, 9, 1, use_graph=False)
+        for s in range(11, 19, 2):
+            e.update(dt, s, 2, 1, use_graph=True)
+    assert _device_bytes(pairs) == _device_bytes(lists)
+    for e in (lists, pairs):
+        e.update(dt, 19, 40, 1, use_graph=True)
+    more = _device_bytes(pairs) - _device_bytes(lists)
+    # per candidate: its solid's slot 4, flag 1, the same before a rebuild 5, 16 a spring kept
+    assert 0 < more <= sc.n_solid * (8 + CANDIDATES * (10 + (48 if rolling else 16)))
+    _same_state_and_lists(lists, pairs)
+
+
+def _no_room(ds, scenes, fakes):
+    b, sc = ds.build_scene(_dry_granular(scenes))
+    os.environ["DEMSPH_PAIR_RUNS"] = "0"
+    lists = ds.Engine(sc)
+    os.environ["DEMSPH_PAIR_RUNS"] = "1"
+    fakes.fake_arm(cudart_fake.ALLOCATION, 1, 16 * CANDIDATES * sc.n_solid)  # the springs of the pairs
+    short = ds.Engine(sc)
+    dt = sc.time_step
+    for e in (lists, short):
+        e.initialize()
+        for first, n in ((1, 9), (10, 40), (50, 40)):
+            e.update(dt, first, n, 1, use_graph=True)
+    assert fakes.fake_count(cudart_fake.ALLOCATION) == 1
+    assert _device_bytes(short) == _device_bytes(lists)
+    s0, s1 = lists.download_solids(), short.download_solids()
+    for k in s0:
+        assert np.array_equal(s0[k], s1[k]), k
+
+
+def test_a_run_without_room_for_pairs(tmp_path):
+    cudart_fake.run(os.path.abspath(__file__), "no_room", tmp_path)
+
+
+if __name__ == "__main__":
+    cudart_fake.main({"no_room": _no_room})
