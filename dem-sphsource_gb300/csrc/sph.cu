@@ -543,13 +543,15 @@ __device__ __forceinline__ void fillWalkTableDF(WalkTableDF& tab, const GridDev&
     }
     __syncthreads();
 }
-// One axis of x_i - x_j: the differences of the leading parts are error-free,
-// the trailing parts (2^-24 of them) plain sums: 2^-46 of the cell size.
+// One axis of x_i - x_j: the differences of the leading parts and of the trailing
+// ones with their rounding errors (34 operations to the 44 of two double-float
+// additions).
 __device__ __forceinline__ dfl relTable(float hi, float lo, float hj, float lj, float oh, float ol)
 {
-    const dfl a = df_two_sum(hi, -hj);
-    const dfl b = df_two_sum(a.hi, -oh);
-    return df_fast_two_sum(b.hi, __fadd_rn(__fadd_rn(a.lo, b.lo), __fsub_rn(__fsub_rn(lo, lj), ol)));
+    const dfl a = df_two_sum(hi, -hj), b = df_two_sum(a.hi, -oh);
+    const dfl l = df_two_sum(lo, -lj), m = df_two_sum(l.hi, -ol);
+    const dfl r = df_fast_two_sum(b.hi, __fadd_rn(m.hi, __fadd_rn(a.lo, b.lo)));
+    return df_fast_two_sum(r.hi, __fadd_rn(r.lo, __fadd_rn(l.lo, m.lo)));
 }
 // A sum of double-floats: leading parts error-free into two words, what those
 // leave and the trailing parts into a third (14 operations a term to df_add's
@@ -570,41 +572,43 @@ struct DFSum {
     }
 };
 // S += f(|x| / h), f(q) = (1 - q/2)^4 (1 + 2q) (shepardTerm): every product and
-// sum of leading parts with its rounding error, the trailing parts in plain
-// float, about 130 operations where double-float arithmetic throughout takes
-// 300, and no branch.  Beyond the support (f is 1e-28 within the rounding of q
-// at its edge) and for entries past the list (ok false) nothing is added.
-// Bound by these operations: the re-initialisation of 48k particles (30
-// partners) 62 to 41 us.  Sums of 64 partners, h from 1e-4 to 250, against 64
-// bits: 5.4e-15 rms, 3.2e-14 at most; double-float throughout 6.9e-15, 4.5e-14.
+// sum of leading parts with its rounding error, the trailing products fused and
+// each result normalised; no branch.  With t = 1 - q/2 the second factor is
+// 5 - 4t, and both leading terms are known to be the larger ones.  Beyond the
+// support (f is 1e-28 within the rounding of q at its edge) and for entries past
+// the list (ok false) nothing is added.
+// Bound by these operations: the re-initialisation of 48k particles (30 partners)
+// takes 47.6 us, with double-float arithmetic throughout 62, of 410k 255.  Against
+// 64 bits (a host emulation, distances and cells at random, h from 1e-4 to 150,
+// root and reciprocal off by up to one unit): a term 1.24e-15 rms and 1.8e-14 at
+// most, with double-float throughout 1.25e-15 and 1.9e-14 (42 us, but 1.64e-15 and
+// 2.6e-14, with the trailing parts summed in plain float); sums of 64 terms
+// 1.4e-14 and 3.2e-14 rms.
 __device__ __forceinline__ void addShepardTerm(DFSum& S, dfl x, dfl y, dfl z, dfl invh, bool ok)
 {
     const dfl xx = df_two_prod(x.hi, x.hi), yy = df_two_prod(y.hi, y.hi), zz = df_two_prod(z.hi, z.hi);
     const dfl s1 = df_two_sum(xx.hi, yy.hi), s2 = df_two_sum(s1.hi, zz.hi);
-    const float low = (xx.lo + yy.lo + zz.lo) + 2.f * (x.hi * x.lo + y.hi * y.lo + z.hi * z.lo) + (s1.lo + s2.lo);
+    const float lx = __fmaf_rn(2.f * x.hi, x.lo, xx.lo), ly = __fmaf_rn(2.f * y.hi, y.lo, yy.lo),
+                lz = __fmaf_rn(2.f * z.hi, z.lo, zz.lo);
+    const dfl s = df_fast_two_sum(s2.hi, ((lx + ly) + s1.lo) + (lz + s2.lo));
     // the root: one correction of the approximate float root and of the
     // reciprocal, then the residual's share
-    const float r0 = fastSqrt(s2.hi), w0 = 0.5f * fastRcp(r0);
-    const float r = r0 > 0.f ? __fmaf_rn(__fmaf_rn(-r0, r0, s2.hi), w0, r0) : r0;
+    const float r0 = fastSqrt(s.hi), w0 = 0.5f * fastRcp(r0);
+    const float r = r0 > 0.f ? __fmaf_rn(__fmaf_rn(-r0, r0, s.hi), w0, r0) : r0;
     const float w1 = __fmaf_rn(w0, __fmaf_rn(-2.f * r, w0, 1.f), w0);
-    const float rl = r0 > 0.f ? (__fmaf_rn(-r, r, s2.hi) + low) * w1 : 0.f;
-    dfl q = df_two_prod(r, invh.hi);
-    q.lo += r * invh.lo + rl * invh.hi;
-    q = df_fast_two_sum(q.hi, q.lo);
-    const float half = 0.5f * q.hi;
-    const float t = __fsub_rn(1.f, half);
-    const float tl = __fsub_rn(__fsub_rn(1.f, t), half) - 0.5f * q.lo;
-    dfl t2 = df_two_prod(t, t);
-    t2.lo += tl * (2.f * t + tl);
-    t2 = df_fast_two_sum(t2.hi, t2.lo);
-    dfl t4 = df_two_prod(t2.hi, t2.hi);
-    t4.lo += t2.lo * (2.f * t2.hi + t2.lo);
-    t4 = df_fast_two_sum(t4.hi, t4.lo);
-    dfl w = df_two_sum(1.f, 2.f * q.hi);
-    w.lo += 2.f * q.lo;
+    const float rl = r0 > 0.f ? (__fmaf_rn(-r, r, s.hi) + s.lo) * w1 : 0.f;
+    const dfl q = df_two_prod(r, invh.hi);
+    const float ql = __fmaf_rn(rl, invh.hi, __fmaf_rn(r, invh.lo, q.lo));
+    const dfl u = df_fast_two_sum(1.f, -0.5f * q.hi), t = df_fast_two_sum(u.hi, __fmaf_rn(-0.5f, ql, u.lo));  // 1 - q/2
+    const auto square = [](dfl v) {
+        const dfl p = df_two_prod(v.hi, v.hi);
+        return df_fast_two_sum(p.hi, __fmaf_rn(2.f * v.hi, v.lo, p.lo));
+    };
+    const dfl t4 = square(square(t)), v = df_fast_two_sum(5.f, -4.f * t.hi),
+              w = df_fast_two_sum(v.hi, __fmaf_rn(-4.f, t.lo, v.lo));  // 1 + 2q = 5 - 4 (1 - q/2)
     dfl f = df_two_prod(t4.hi, w.hi);
-    f.lo += t4.hi * w.lo + t4.lo * (w.hi + w.lo);
-    const bool in = ok && !(q.hi >= 2.f);
+    f.lo = __fmaf_rn(t4.lo, w.hi, __fmaf_rn(t4.hi, w.lo, f.lo));
+    const bool in = ok && !(t.hi <= 0.f);
     S.add(in ? f.hi : 0.f, in ? f.lo : 0.f);
 }
 
