@@ -1111,7 +1111,10 @@ int demsph_create(const demsph_scene* sc, const demsph_options* opt, demsph_engi
                 CK(cudaMemcpyAsync(d.fdrho[0], drho.data(), sizeof(float) * nf, cudaMemcpyHostToDevice, e->stream));
                 CK(cudaMemcpyAsync(d.facc, acc.data(), sizeof(float4) * nf, cudaMemcpyHostToDevice, e->stream));
                 CK(cudaMemcpyAsync(d.fpar, par.data(), sizeof(float4) * nf, cudaMemcpyHostToDevice, e->stream));
-                d.uniformFluid = 1;
+                // the pair terms of uniform fluids take reciprocals of products of
+                // two densities in one operation that flushes subnormals: not for
+                // densities whose products come near them
+                d.uniformFluid = par[0].x >= 1.e-16f && par[0].x <= 1.e16f ? 1 : 0;
                 for (int i = 1; i < nf && d.uniformFluid; ++i)
                     d.uniformFluid = par[i].x == par[0].x && par[i].y == par[0].y && par[i].z == par[0].z &&
                                      par[i].w == par[0].w && ph[i].w == ph[0].w && pl[i].w == pl[0].w;
