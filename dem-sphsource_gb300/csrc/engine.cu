@@ -55,6 +55,7 @@ void dropGraph(demsph_engine* e)
 {
     for (const auto& g : e->graphs) cudaGraphExecDestroy(g.exec);
     e->graphs.clear();
+    std::memset(e->runSeen, 0, sizeof(e->runSeen));
     for (const auto& r : e->rounds) cudaGraphDestroy(r.graph);
     e->rounds.clear();
 }
@@ -1596,10 +1597,10 @@ static int stepKind(const DeviceState& d, int i, int gap)
     return (i % gap == 0 ? 1 : 0) | (i % (5 * gap) == 0 ? 2 : 0);
 }
 
-// Steps of a graph, and graphs kept: a graph's first and last step cost about
-// twice the others, and instantiating one about 5 us per launch.
-constexpr int MAX_GRAPH_STEPS = 32;
-constexpr size_t MAX_GRAPHS = 64;
+// Most steps of a graph: a run's first and last step cost about twice the others.
+// An engine holds a graph for each length and parity at most, and two kinds of
+// fluid step: 68.
+constexpr int MAX_GRAPH_STEPS = demsph_engine::MAX_RUN;
 
 // What capturing steps changes of the engine as running them does.
 struct CaptureState {
@@ -1628,11 +1629,6 @@ static const demsph_engine::CachedGraph& graphFor(demsph_engine* e, int kind, in
 {
     for (const auto& g : e->graphs)
         if (g.kind == kind && g.parity == e->par && g.length == length) return g;
-    if (e->graphs.size() >= MAX_GRAPHS) {  // runs of ever new lengths: the oldest goes
-        CK(cudaStreamSynchronize(e->stream));
-        cudaGraphExecDestroy(e->graphs.front().exec);
-        e->graphs.erase(e->graphs.begin());
-    }
     // runs of plain DEM steps fuse each step's closing integration with the
     // next one's opening (fluid steps are captured one at a time)
     const bool fused = e->fuseIntegration && kind == 0 && length >= 2;
@@ -1685,16 +1681,35 @@ static void adaptRowsPerWarp(demsph_engine* e, const int* stats)
     dropGraph(e);  // the launch shape and the state are baked into the graphs
 }
 
-// Launches the next graph of the steps from s to end: a run of plain DEM steps
+// Launches a fused run of plain DEM steps without a graph.
+static void launchRun(demsph_engine* e, double dt, int s, int len, int gap, std::vector<std::pair<int, int>>& fusedRuns)
+{
+    preparePairs(e, len);
+    fusedSteps(e, dt, s, len, gap);
+    fusedRuns.emplace_back(s, len);
+    e->runStats.fused_passes += len - 1;
+}
+
+// Launches the next part of the steps from s to end: a run of plain DEM steps
 // replays one graph of its length, longer ones in parts (the first and last step
-// of a part build contact lists), a fluid step a 1-step graph.  Returns its steps
-// and records it in fusedRuns when it is fused.
+// of a part build contact lists), a fluid step a 1-step graph.  A run of a length
+// (and parity) that is new goes without, and has its graph made when it comes
+// back: a step of a 13k coupled scene, calls of 5 to 32 plain steps, takes 21.3
+// us in the first, 31.7 in the second and 17.2 from the third on, where a graph
+// made at once took 32.4 in the first; a program whose calls are of ever new
+// lengths pays for none.  Returns its steps and records it in fusedRuns when it
+// is fused.
 static int launchSteps(demsph_engine* e, double dt, int s, int end, int gap, std::vector<std::pair<int, int>>& fusedRuns)
 {
     const int kind = stepKind(e->d, s, gap);
     int len = 1;
     if (kind == 0)
         while (len < MAX_GRAPH_STEPS && s + len < end && stepKind(e->d, s + len, gap) == 0) ++len;
+    if (kind == 0 && len >= 2 && e->fuseIntegration && !e->runSeen[e->par][len]) {
+        e->runSeen[e->par][len] = true;
+        launchRun(e, dt, s, len, gap, fusedRuns);
+        return len;
+    }
     const auto& g = graphFor(e, kind, len, dt, s, gap);
     CK(cudaGraphLaunch(g.exec, e->stream));
     e->replayedKernels += g.kernels;
@@ -1753,10 +1768,7 @@ static int runUpdate(demsph_engine* e, double dt, int first_step, int n_steps, i
             if (kind == 0)
                 while (len < MAX_GRAPH_STEPS && s + len < end && stepKind(d, s + len, gap) == 0) ++len;
             if (e->fuseIntegration && kind == 0 && len >= 2) {
-                preparePairs(e, len);
-                fusedSteps(e, dt, s, len, gap);
-                fusedRuns.emplace_back(s, len);
-                e->runStats.fused_passes += len - 1;
+                launchRun(e, dt, s, len, gap, fusedRuns);
             } else {
                 for (int k = 0; k < len; ++k) fullStep(e, dt, s + k, gap);  // the steps flip the parity
             }

@@ -72,6 +72,8 @@ struct demsph_engine {
     int movingDummies = 0;  // dummy particles given a velocity (in the move list)
     // CUDA graphs of step runs, keyed by the kind of step, the contact-list
     // parity they start from and their length (all for one dt and gap)
+    static constexpr int MAX_RUN = 32;         // plain DEM steps of one graph
+    bool runSeen[2][MAX_RUN + 1] = {};         // lengths launched so far, by the parity they start from
     struct CachedGraph {
         int kind, parity, length;
         cudaGraphExec_t exec;
@@ -188,6 +190,7 @@ struct demsph_engine {
         swap(keysAdvanced, o.keysAdvanced);
         swap(runStats, o.runStats);
         swap(graphs, o.graphs);
+        swap(runSeen, o.runSeen);
         swap(rounds, o.rounds);
         swap(graphGap, o.graphGap);
         swap(graphDt, o.graphDt);
