@@ -56,6 +56,7 @@ void dropGraph(demsph_engine* e)
     for (const auto& g : e->graphs) cudaGraphExecDestroy(g.exec);
     e->graphs.clear();
     std::memset(e->runSeen, 0, sizeof(e->runSeen));
+    ++e->graphsDropped;
     for (const auto& r : e->rounds) cudaGraphDestroy(r.graph);
     e->rounds.clear();
 }
@@ -2043,11 +2044,14 @@ int demsph_profile_report(demsph_engine* e, char* buf, int cap)
 // memory.  It serves rounds that repeat: rounds that are whole multiples of the
 // Shepard period (5 gap steps) and of even length keep their phase and parity,
 // so a steady batch launches the same executable graph round after round.
-// Building it costs about 5 us a kernel, as much as the round takes, so a set
-// of rounds that has not come before (another length, phase or parity, a member
-// whose graphs were dropped by list growth) is launched as the members' own
-// graphs on their own streams, in turn, which each engine keeps: 40 steps of
-// eight scenes of 2k to 48k whose phases never repeat 15.7 ms with a graph built
+// Building it costs about 5 us a kernel, as much as the round takes, so it is
+// made for a set of rounds that comes back while it is one of the last GRAPHS
+// sets, as many as have their graph kept: rounds that cycle through more sets
+// would build one in every call.  The others, and a set with a member whose
+// graphs were dropped (list growth, another dt or gap, a setter), are launched as
+// the members' own graphs on their own streams, in turn, which each engine keeps:
+// 40 steps of eight scenes of 2k to 48k whose phases never repeat 15.7 ms with a
+// graph built
 // for each call, 9.7 ms without.  A member whose round overflowed a list
 // resumes alone after its lists grow (demsph_update's path), before the call
 // returns.
@@ -2134,9 +2138,10 @@ struct demsph_batch {
         int2* report;   // the mapped status array the graph writes
         int** where;    // the status addresses it reads
     };
+    static constexpr size_t GRAPHS = 4;
     std::vector<Cached> cache;
-    // the member sets of recent rounds (their engines, phases, lengths and
-    // parities): one that comes back gets its graph
+    // the member sets of the last rounds (their engines with the times their
+    // graphs were dropped, phases, lengths and parities)
     std::vector<std::vector<long long>> seen;
     demsph_batch_info info{};
     std::string err;
@@ -2254,14 +2259,14 @@ int demsph_batch_update(demsph_batch* b, demsph_engine* const* engines, int coun
     std::vector<long long> set;
     for (const auto& mb : members) {
         const int period = mb.e->d.nf > 0 ? 5 * gap[mb.i] : 1;
-        for (const long long v : {mb.e->serial, (long long)(mb.first % period), (long long)mb.length, (long long)mb.startPar})
+        for (const long long v : {mb.e->serial, mb.e->graphsDropped, (long long)(mb.first % period), (long long)mb.length,
+                                  (long long)mb.startPar})
             set.push_back(v);
     }
     const auto known = std::find(b->seen.begin(), b->seen.end(), set);
     const bool direct = known == b->seen.end();
     if (direct) {
-        constexpr size_t KEEP = 16;
-        if (b->seen.size() >= KEEP) b->seen.pop_back();
+        if (b->seen.size() >= demsph_batch::GRAPHS) b->seen.pop_back();
         b->seen.insert(b->seen.begin(), set);
     } else {
         std::rotate(b->seen.begin(), known, known + 1);
@@ -2328,8 +2333,7 @@ int demsph_batch_update(demsph_batch* b, demsph_engine* const* engines, int coun
             std::rotate(b->cache.begin(), b->cache.begin() + hit, b->cache.begin() + hit + 1);
         } else {
             const auto ti = std::chrono::steady_clock::now();
-            constexpr size_t KEEP = 4;
-            while (b->cache.size() >= KEEP) {  // the least recently used goes
+            while (b->cache.size() >= demsph_batch::GRAPHS) {  // the least recently used goes
                 auto& c = b->cache.back();
                 CK(cudaGraphExecDestroy(c.exec));
                 CK(cudaFreeHost(c.report));

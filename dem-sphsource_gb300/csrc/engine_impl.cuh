@@ -73,6 +73,7 @@ struct demsph_engine {
     // CUDA graphs of step runs, keyed by the kind of step, the contact-list
     // parity they start from and their length (all for one dt and gap)
     static constexpr int MAX_RUN = 32;         // plain DEM steps of one graph
+    long long graphsDropped = 0;               // times dropGraph ran
     bool runSeen[2][MAX_RUN + 1] = {};         // lengths launched so far, by the parity they start from
     struct CachedGraph {
         int kind, parity, length;
@@ -191,6 +192,7 @@ struct demsph_engine {
         swap(runStats, o.runStats);
         swap(graphs, o.graphs);
         swap(runSeen, o.runSeen);
+        ++graphsDropped, ++o.graphsDropped;  // the graphs changed hands
         swap(rounds, o.rounds);
         swap(graphGap, o.graphGap);
         swap(graphDt, o.graphDt);

@@ -437,14 +437,16 @@ DEMSPH_API int demsph_export_fluid_sumw0(demsph_engine* e, double* sumw0);
    No counterpart in the reference (one scene per process).  One call advances
    engines[0..count) by n_steps[k] steps from first_step[k] each (time step
    dt[k], fluid gap gap[k]), the scenes' kernels overlapping on the device.  A
-   set of rounds that has come before goes in one CUDA graph launch: each
-   engine's round of steps is a child graph, captured once per (phase in the
-   fluid and Shepard schedule, length, contact-list parity, dt, gap), the
-   children run as independent branches, and the executable graph is reused
-   while every member's round repeats (rounds of even length that are multiples
-   of 5 gap steps repeat).  A set that has not is launched as each engine's own
-   step graphs on its own stream.  Every scene's state afterwards is bit for bit its state
-   after demsph_update over the same steps.  Step 1 and profiled runs go
+   set of rounds that comes back while it is one of the last four goes in one
+   CUDA graph launch: each engine's round of steps is a child graph, captured
+   once per (phase in the fluid and Shepard schedule, length, contact-list
+   parity, dt, gap), the children run as independent branches, and the
+   executable graph is reused while every member's round repeats (rounds of even
+   length that are multiples of 5 gap steps repeat).  Another set, and one with a
+   member whose graphs were dropped since (list growth, another dt or gap, a
+   setter), is launched as each engine's own step graphs on its own stream.
+   Every scene's state afterwards is bit for bit its state after demsph_update
+   over the same steps.  Step 1 and profiled runs go
    through demsph_update first; a member whose lists overflowed grows them and
    finishes its steps alone before the call returns.  status_out[k] receives
    each engine's status (its message in demsph_last_error); the return value
