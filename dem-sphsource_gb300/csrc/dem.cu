@@ -314,7 +314,6 @@ __device__ __forceinline__ void bondUpdate(const DeviceState& d, float dt, int b
     d.bTB[b] = f4(Tq + nxF * g.sB);
 }
 
-// Wall overlap r - ((x - p) . n) in double-float.
 // A wall and a solid's springs with it (zeros unless they are held).
 struct WallIn {
     float4 nh, nl, s[3];
@@ -334,6 +333,7 @@ __device__ __forceinline__ void loadWallSprings(const DeviceState& d, int prev, 
 #pragma unroll
     for (int j = 0; j < 3; ++j) w.s[j] = held ? d.wspring[prev][j][h] : make_float4(0.f, 0.f, 0.f, 0.f);
 }
+// Wall overlap r - ((x - p) . n) in double-float.
 __device__ __forceinline__ float wallOverlap(const DeviceState& d, int4 c, float4 h, float4 l, const WallIn& w, float r,
                                              float rlo)
 {
@@ -1230,10 +1230,11 @@ __device__ __forceinline__ int pairSumsRow(const DeviceState& d, int par, float 
 // 19.3 to 12.1 us with cold caches, a DEM step 20.9 to 18.1.
 constexpr int SUM_LANES = 8, SUM_ITEMS = 2 * SUM_LANES;
 constexpr int SUM_BLOCKS = 4;  // blocks per SM: all of them resident under the rule of launchPairSums
-struct SumItems {
+struct alignas(16) SumItems {  // stored as float4
     // force xyz -, torque xyz -; the rows of a warp eight banks apart
     float v[T / SUM_LANES][SUM_ITEMS * 8 + 8];
 };
+static_assert(alignof(SumItems) == 16 && sizeof(SumItems::v[0]) % 16 == 0, "float4 stores to every row");
 // This lane's component (force xyz in lanes 0 to 2, torque xyz in 3 to 5).
 // Called by whole warps.
 __device__ __forceinline__ KahanF pairSumsGroup(const DeviceState& d, SumItems& items, int row, int a, bool live)
