@@ -185,7 +185,6 @@ struct demsph_engine {
         swap(fuseIntegration, o.fuseIntegration);
         swap(mergeContacts, o.mergeContacts);
         swap(pairRuns, o.pairRuns);
-        swap(pairsAllowed, o.pairsAllowed);
         swap(foldIntegration, o.foldIntegration);
         swap(resumeOpened, o.resumeOpened);
         swap(keysAdvanced, o.keysAdvanced);

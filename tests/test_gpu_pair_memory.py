@@ -69,6 +69,27 @@ def _no_room(ds, scenes, fakes):
         assert np.array_equal(s0[k], s1[k]), k
 
 
+def test_an_append_keeps_the_setting(ds, scenes):
+    """demsph_set_pair_runs(e, 0) holds for the engine that an append puts in its place."""
+    b, sc = ds.build_scene(_dry_granular(scenes))
+    e = ds.Engine(sc)
+    e._chk(e.lib.demsph_set_pair_runs(e.h, 0), "demsph_set_pair_runs")
+    e.initialize()
+    e.update(sc.time_step, 1, 9, 1)
+    add = ds.Builder(10)
+    o, s = [sc.domain_origin[a] for a in range(3)], [sc.domain_size[a] for a in range(3)]
+    add.setDomain(o, s)
+    add.addSolid(np.array([[o[0] + 0.5 * s[0], o[1] + 0.5 * s[1], o[2] + s[2] - 2.0e-3]]), (0, 0, 0), 1.0e-3, 2500.0, 0)
+    more = add.scene()
+    e.append(sc, more)
+    before = _device_bytes(e)
+    e.update(sc.time_step, 10, 40, 1)
+    assert _device_bytes(e) == before
+    e._chk(e.lib.demsph_set_pair_runs(e.h, 1), "demsph_set_pair_runs")
+    e.update(sc.time_step, 50, 40, 1)
+    assert _device_bytes(e) > before
+
+
 def test_a_run_without_room_for_pairs(tmp_path):
     cudart_fake.run(os.path.abspath(__file__), "no_room", tmp_path)
 
