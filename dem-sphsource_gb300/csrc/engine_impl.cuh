@@ -49,9 +49,10 @@ struct demsph_engine {
     demsph_options opt{};         // the options the engine was created with
     int device = 0;
     cudaStream_t stream = nullptr;
-    // a second stream and two events: inside runs of plain DEM steps the
-    // coupling force of a step runs beside its contact detection (a branch of
-    // the captured graph, joined before the contact forces)
+    // a second stream and two events: the coupling force of a step on contact
+    // lists inside a run of plain DEM steps runs beside its contact detection (a
+    // branch of the captured graph, joined before the per-solid sums; a step on
+    // contact pairs computes it in their launch)
     cudaStream_t side = nullptr;
     cudaEvent_t forkEv = nullptr, joinEv = nullptr;
     std::vector<demsph::Allocation> owned;  // every device buffer of the engine
@@ -84,10 +85,11 @@ struct demsph_engine {
     // Graphs of two or more plain DEM steps integrate the end of one step and
     // the start of the next in one pass (DEMSPH_FUSE_INTEGRATION=0 keeps two).
     bool fuseIntegration = true;
-    // In those graphs the steps a fused pass opens build their contact list
-    // and contact forces in one launch when the scene has no bonds and the
-    // lists come from candidates (DEMSPH_MERGE_CONTACTS=0 keeps two launches;
-    // off for good once the lists come from the walk).
+    // In those graphs the steps a fused pass opens, where they are not on contact
+    // pairs (runs of two steps, or without pairs), build their contact list and
+    // contact forces in one launch when the scene has no bonds and the lists come
+    // from candidates (DEMSPH_MERGE_CONTACTS=0 keeps two launches; off for good
+    // once the lists come from the walk).
     bool mergeContacts = true;
     // Runs of three or more plain DEM steps evaluate the contact candidates as
     // pairs between their first and last step, without contact lists

@@ -1,5 +1,5 @@
-// WCSPH pair loops: Riemann continuity, Riemann momentum, Shepard density
-// re-initialisation and the SPH->DEM coupling force.
+// WCSPH pair loops: Riemann continuity, Riemann momentum and Shepard density
+// re-initialisation (the SPH->DEM coupling force, a sum per solid, is in dem.cu).
 //
 // Physics restated from core/integrate.cu:3-330 (reference) with the Wendland
 // C2 kernel of core/SPHKernelDEMContactModel.h:5-32.  Algebraic forms used

@@ -256,8 +256,9 @@ struct demsph_server {
             }
             // members: last round's members still running, plus newcomers -
             // newcomers join when no engine is being created, or 1 s after the
-            // membership last grew (each change instantiates a new graph; the
-            // first round waits the same way for the engines being created)
+            // membership last grew (each change makes a set of rounds that is
+            // launched member by member at first and gets its graph when it comes
+            // back; the first round waits the same way for the engines being created)
             if (ids.empty() && lastJoin == Clock::time_point{}) lastJoin = Clock::now();
             const bool admitNew = !creating() || seconds(lastJoin, Clock::now()) > 1.0;
             mem.clear();
