@@ -1,6 +1,7 @@
 /* Fakes of the CUDA runtime's calls for tests of failing calls, preloaded into a
    child process: each passes on to the runtime, counts, and on request returns an
-   error in the place of one call, which then does not happen. */
+   error in the place of one call, which then does not happen (or, of free memory,
+   another number). */
 #include <cuda_runtime_api.h>
 #include <dlfcn.h>
 
@@ -17,6 +18,9 @@ void fake_arm(int kind, long long nth, size_t bytes)
     if (kind == ALLOCATION) failBytes = bytes;
 }
 long long fake_count(int kind) { return calls[kind]; }
+
+static size_t freeBytes;  /* what cudaMemGetInfo reports as free; 0: the truth */
+void fake_free(size_t bytes) { freeBytes = bytes; }
 
 static int fails(int kind) { return ++calls[kind] == failAt[kind]; }
 static void* real(const char* name) { return dlsym(dlopen("libcudart.so.13", RTLD_LAZY), name); }
@@ -35,6 +39,12 @@ cudaError_t cudaMallocAsync(void** p, size_t bytes, cudaStream_t s)
 {
     if (bytes == failBytes && fails(ALLOCATION)) return cudaErrorMemoryAllocation;
     return ((cudaError_t(*)(void**, size_t, cudaStream_t))real("cudaMallocAsync"))(p, bytes, s);
+}
+cudaError_t cudaMemGetInfo(size_t* unused, size_t* total)
+{
+    const cudaError_t e = ((cudaError_t(*)(size_t*, size_t*))real("cudaMemGetInfo"))(unused, total);
+    if (e == cudaSuccess && freeBytes) *unused = freeBytes;
+    return e;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* cfg, const void* kernel, void** args)
 {

@@ -94,5 +94,30 @@ def test_a_run_without_room_for_pairs(tmp_path):
     cudart_fake.run(os.path.abspath(__file__), "no_room", tmp_path)
 
 
+def _crowded(ds, scenes, fakes, free, used):
+    """80k grains, whose pairs take 67 MB, on a device that reports `free` bytes."""
+    import ctypes as C
+    fakes.fake_free.argtypes = [C.c_size_t]
+    b, sc = ds.build_scene(scenes.granular_settle(n_spheres=80_000, n_clumps=0, box=(0.1, 0.1), spacing=2.1e-3, steps=20,
+                                                  z0=1.0e-3, name="bed"))
+    os.environ["DEMSPH_PAIR_RUNS"] = "0"
+    lists = ds.Engine(sc)
+    os.environ["DEMSPH_PAIR_RUNS"] = "1"
+    fakes.fake_free(int(free))
+    e = ds.Engine(sc)
+    for x in (lists, e):
+        x.initialize()
+        x.update(sc.time_step, 1, 9, 1)
+    assert (_device_bytes(e) > _device_bytes(lists)) == bool(int(used))
+    s0, s1 = lists.download_solids(), e.download_solids()
+    for k in s0:
+        assert np.array_equal(s0[k], s1[k]), k
+
+
+@pytest.mark.parametrize("free,used", [(100 << 20, 0), (2 << 30, 1)])
+def test_large_pairs_leave_most_of_the_free_memory(tmp_path, free, used):
+    cudart_fake.run(os.path.abspath(__file__), "crowded", tmp_path, free, used)
+
+
 if __name__ == "__main__":
-    cudart_fake.main({"no_room": _no_room})
+    cudart_fake.main({"no_room": _no_room, "crowded": _crowded})
