@@ -243,9 +243,9 @@ void allocContactLists(demsph_engine* e)
     d.rev = dalloc<int>(c, e->owned, e->stream);
     // what a contact list's step writes before it reads it, in one block: the
     // pair runs use it between lists
-    d.listWork = dalloc<float4>(LIST_WORK * c, e->owned, e->stream);
+    e->listWork = dalloc<float4>(LIST_WORK * c, e->owned, e->stream);
     float4** work[LIST_WORK] = {&d.pF, &d.pT, &d.pTA, &d.revF, &d.revT, &d.springIn[0], &d.springIn[1], &d.springIn[2]};
-    for (int k = 0; k < LIST_WORK; ++k) *work[k] = d.listWork + k * c;
+    for (int k = 0; k < LIST_WORK; ++k) *work[k] = e->listWork + k * c;
     for (int p = 0; p < 2; ++p) d.fwd[p] = dalloc<int>(c, e->owned, e->stream);
     for (int k = 0; k < 3; ++k)
         for (int p = 0; p < 2; ++p) d.springOut[p][k] = dalloc<float4>(c, e->owned, e->stream);
@@ -266,7 +266,7 @@ void freePairs(demsph_engine* e)
         freeOne(e, p);
         array = nullptr;  // its address may come back as another array's
     };
-    drop(d.pfirst), drop(d.plink), drop(d.pflag), drop(d.oldCount), drop(d.oldId), drop(d.oldFlag), drop(d.pairWork);
+    drop(d.pfirst), drop(d.plink), drop(d.pflag), drop(d.oldCount), drop(d.oldId), drop(d.oldFlag), drop(e->pairWork);
     for (int k = 0; k < 3; ++k) {
         drop(d.pspring[k]);
         d.oldSpring[k] = nullptr;
@@ -313,8 +313,8 @@ void allocPairs(demsph_engine* e)
     d.oldId = dalloc<int>(c, e->owned, e->stream, false);
     d.oldFlag = dalloc<unsigned char>(c, e->owned, e->stream);
     for (int k = 0; k < d.pairSprings; ++k) d.pspring[k] = dalloc<float4>(c, e->owned, e->stream, false);
-    float4* work = d.listWork;
-    if (!pairsInListWork(d)) work = d.pairWork = dalloc<float4>(3 * c, e->owned, e->stream, false);
+    float4* work = e->listWork;
+    if (!pairsInListWork(d)) work = e->pairWork = dalloc<float4>(3 * c, e->owned, e->stream, false);
     d.pforce = work;
     d.ptorqueA = work + c;
     d.ptorqueB = work + 2 * c;
@@ -761,7 +761,7 @@ void growLists(demsph_engine* e, int status)
             float4* keepSpring[3] = {d.springOut[keep][0], d.springOut[keep][1], d.springOut[keep][2]};
             d.fwd[keep] = nullptr;
             for (int k = 0; k < 3; ++k) d.springOut[keep][k] = nullptr;
-            void* ptrs[] = {d.rev, d.listWork, d.fwd[keep ^ 1], d.springOut[keep ^ 1][0], d.springOut[keep ^ 1][1],
+            void* ptrs[] = {d.rev, e->listWork, d.fwd[keep ^ 1], d.springOut[keep ^ 1][0], d.springOut[keep ^ 1][1],
                             d.springOut[keep ^ 1][2]};
             for (void* p : ptrs) freeOne(e, p);
             d.scap = std::max(d.scap * 2, need[0] + need[0] / 2 + 1);
@@ -864,8 +864,8 @@ void closePairs(demsph_engine* e, const std::vector<std::pair<int, int>>& runs, 
     CK(cudaStreamSynchronize(e->stream));
     void* work = nullptr;  // holds the history when it is closed from there
     if (most > d.scap) {
-        work = d.listWork;
-        d.listWork = nullptr;
+        work = e->listWork;
+        e->listWork = nullptr;
         growLists(e, ST_SS_OVERFLOW);
     }
     launchPairsClose(d, e->par, old, e->stream);

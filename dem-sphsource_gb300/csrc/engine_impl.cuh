@@ -97,6 +97,9 @@ struct demsph_engine {
     // the walk, or where there was no room for the pairs).
     bool pairRuns = true;
     bool pairsAllowed = true;  // demsph_set_pair_runs
+    // the block of pF, pT, pTA, revF, revT and springIn, and the pairs' results
+    // and old springs where that does not hold them
+    float4 *listWork = nullptr, *pairWork = nullptr;
     // The per-solid sums run the solids' integration pass in the same launch
     // when the integrated solids are exactly the contact rows
     // (DEMSPH_FOLD_INTEGRATION=0 keeps the separate pass).
@@ -187,6 +190,8 @@ struct demsph_engine {
         swap(fuseIntegration, o.fuseIntegration);
         swap(mergeContacts, o.mergeContacts);
         swap(pairRuns, o.pairRuns);
+        swap(listWork, o.listWork);
+        swap(pairWork, o.pairWork);
         swap(foldIntegration, o.foldIntegration);
         swap(resumeOpened, o.resumeOpened);
         swap(keysAdvanced, o.keysAdvanced);

@@ -335,7 +335,6 @@ struct DeviceState {
     // previous list (In) and after the contact forces of the step whose list
     // has parity p (Out[p]); a step reads only the other parity's Out, so a
     // step abandoned after an overflow leaves the history it started from
-    float4* listWork;        // the block of pF, pT, pTA, revF, revT and springIn
     float4* springIn[3];
     float4* springOut[2][3];
     float4* pF;              // pair contact force on A, as the reference stores it (exports)
@@ -381,7 +380,6 @@ struct DeviceState {
     int* oldId;              // their solids, flags and springs, by slot
     unsigned char* oldFlag;
     float4* oldSpring[3];
-    float4* pairWork;        // results and old springs where the lists' block does not hold them
     int* need;               // [0] most contacts of a row, [1] most candidates of a row,
                              // [2] / [3] most fluid / solid candidates of a fluid particle,
                              // [4] most walk candidates of a fluid particle in tile mode (for growing)
